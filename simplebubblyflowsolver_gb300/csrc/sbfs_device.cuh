@@ -166,6 +166,40 @@ __device__ __forceinline__ int wrap(int J, int ny) {
   return r;
 }
 
+// FP64 forms.  Measured on GB300 (1995 MHz, any occupancy from one warp a
+// scheduler up): a DFMA whose three operands are vector registers issues at
+// 596 G/s (64.7 cycles a warp and scheduler), a DADD, a DMUL or a DFMA with
+// a constant-bank, uniform-register or immediate operand at 502 G/s (76.8
+// cycles).  So sums and products are written as fused operations with a 1 or
+// a -0 that the compiler cannot see through: a + b = fma(a, 1, b) and
+// a b = fma(a, b, -0) are the same values bit for bit (one rounding, the
+// same signed zeros, infinities and NaNs), and reg() moves a kernel argument
+// into vector registers.  `index` is any thread-dependent value below 2^24:
+// its upper bits are a zero the compiler does not know.
+struct Fp64 {
+  unsigned z;
+  double one, nzero;
+  __device__ __forceinline__ explicit Fp64(unsigned index) : z(index >> 24) {
+    one = __hiloint2double(0x3ff00000 ^ z, z);
+    nzero = __hiloint2double(0x80000000 ^ z, z);
+  }
+  __device__ __forceinline__ double reg(double x) const {
+    return __hiloint2double(__double2hiint(x) ^ z, __double2loint(x) ^ z);
+  }
+  __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
+  __device__ __forceinline__ double sub(double a, double b) const { return fma(-b, one, a); }
+  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, nzero); }
+  __device__ __forceinline__ double2 cadd(double2 a, double2 b) const {
+    return make_double2(add(a.x, b.x), add(a.y, b.y));
+  }
+  __device__ __forceinline__ double2 csub(double2 a, double2 b) const {
+    return make_double2(sub(a.x, b.x), sub(a.y, b.y));
+  }
+  __device__ __forceinline__ double2 cmul(double2 a, double2 b) const {
+    return make_double2(fma(a.x, b.x, mul(-a.y, b.y)), fma(a.x, b.y, mul(a.y, b.x)));
+  }
+};
+
 // bit-level helpers: sign and threshold tests on the integer pattern of a
 // double keep these comparisons off the FP64 pipe
 __device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
@@ -206,6 +240,14 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return fma(r, fma(e, e, e), r);
 }
 
+// the same with the 1 of e in registers (see Fp64)
+__device__ __forceinline__ double rcp_nr(double x, const Fp64 &f) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, f.one);
+  return fma(r, fma(e, e, e), r);
+}
+
 // 1 / sqrt(s) for finite normal s > 0: rsqrt.approx.ftz.f64 seed and one
 // third-order step y <- y (1 + e/2 + 3e^2/8), e = 1 - s y^2 (the series of
 // (1 - e)^(-1/2) truncated after e^2): five FP64 operations
@@ -216,11 +258,22 @@ __device__ __forceinline__ double rsqrt_nr(double s) {
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
+__device__ __forceinline__ double rsqrt_nr(double s, const Fp64 &f) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+  const double e = fma(-f.mul(s, y), y, f.one);
+  return fma(f.mul(y, e), fma(e, f.reg(0.375), f.reg(0.5)), y);
+}
+
 // 1 / max(sqrt(s), eps) with eps = DBL_EPSILON (the reference normalises a
 // gradient by 1 / fmax(|g|, DBL_EPSILON), curvature_tensor.c:43, 87)
 __device__ __forceinline__ double inv_norm(double s) {
   constexpr double eps = 2.220446049250313080847e-16;
   return lt_pos(s, eps * eps) ? 1. / eps : rsqrt_nr(s);
+}
+__device__ __forceinline__ double inv_norm(double s, const Fp64 &f) {
+  constexpr double eps = 2.220446049250313080847e-16;
+  return lt_pos(s, eps * eps) ? 1. / eps : rsqrt_nr(s, f);
 }
 
 }  // namespace sbfs

@@ -39,11 +39,6 @@ constexpr int BX = 32, BY = 8;
 
 __device__ __forceinline__ size_t ix(const Grid &g, int row, int col) { return (size_t)row * g.p1 + col; }
 __device__ __forceinline__ bool same(double a, double b) { return dbits(a) == dbits(b); }
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 
 // Interface-branch compaction.  An FP64 instruction costs its warp an issue
 // slot however few of its lanes run it (measured: eight FMA chains on 1 to
@@ -95,10 +90,11 @@ __device__ __forceinline__ void corner_normal(const Grid &g, const Metrics &m, c
   // four values differ by ~1e-16 and the reference's sum is rounding noise
   // that the normalisation below (by max(|g|, eps)) scales up to O(1);
   // another order gives O(1) different corner normals
-  const double gx = m.ihxxf[I] * (((-a + b) - c) + d);
-  const double gy = g.ihy * (((-a - b) + c) + d);
-  const double inv = inv_norm(fma(gx, gx, gy * gy));
-  reinterpret_cast<double2 *>(dvof)[(size_t)r * (g.p2 / 2) + (I - 1)] = make_double2(gx * inv, gy * inv);
+  const Fp64 f(I);
+  const double gx = f.mul(m.ihxxf[I], f.add(f.sub(f.sub(b, a), c), d));
+  const double gy = f.mul(f.reg(g.ihy), f.add(f.add(f.sub(-a, b), c), d));
+  const double inv = inv_norm(fma(gx, gx, f.mul(gy, gy)), f);
+  reinterpret_cast<double2 *>(dvof)[(size_t)r * (g.p2 / 2) + (I - 1)] = make_double2(f.mul(gx, inv), f.mul(gy, inv));
 }
 
 // compact: the corners with a gradient are handed to the block's first
@@ -121,21 +117,23 @@ __global__ void __launch_bounds__(BX *BY) k_props(Grid g, Metrics m, Phys ph0, c
   if (!cmp && !in) return;  // when compacting, every thread meets the barriers below
   const int zr = blockIdx.z * g.ny;  // first row of this case
   const int r = J - 1 + zr, rm = wrap(J - 1, g.ny) + zr;
+  const Fp64 f(I);
   bool need = false;  // the corner gradient is not identically zero
   if (in) {
     const double v = vof[ix(g, r, I)];
-    if (DEN) den[ix(g, r, I)] = clip_pos(fma(ph.dm1, v, 1.), ph.den_lo, ph.den_hi);
+    if (DEN) den[ix(g, r, I)] = clip_pos(fma(f.reg(ph.dm1), v, f.one), ph.den_lo, ph.den_hi);
     if (VIS) {
       // 1 + (visr - 1) 0.5 (a + b) = 1 + c2 (a + b), c2 = (visr - 1) / 2
-      const double c = SCALED ? ph.vsx_c : ph.vm1, c2 = SCALED ? ph.vsx_c2 : ph.hvm1, one = SCALED ? ph.vsx_1 : 1.;
+      const double c = SCALED ? ph.vsx_c : ph.vm1, c2 = f.reg(SCALED ? ph.vsx_c2 : ph.hvm1);
+      const double one = SCALED ? f.reg(ph.vsx_1) : f.one;
       if (I >= 1) {
         double vis;
         if (I == 1) vis = fma(c, vof[ix(g, r, 0)], one);
         else if (I == g.nx + 1) vis = fma(c, v, one);
-        else vis = fma(c2, vof[ix(g, r, I - 1)] + v, one);
+        else vis = fma(c2, f.add(vof[ix(g, r, I - 1)], v), one);
         visux[ix(g, r, I - 1)] = SCALED ? clip_pos(vis, ph.vsx_lo, ph.vsx_hi) : clip_pos(vis, ph.vis_lo, ph.vis_hi);
       }
-      const double vy = SCALED ? fma(ph.vsy_c2, vof[ix(g, rm, I)] + v, ph.vsy_1) : fma(c2, vof[ix(g, rm, I)] + v, 1.);
+      const double vy = fma(SCALED ? f.reg(ph.vsy_c2) : c2, f.add(vof[ix(g, rm, I)], v), SCALED ? f.reg(ph.vsy_1) : f.one);
       visuy[ix(g, r, I)] = SCALED ? clip_pos(vy, ph.vsy_lo, ph.vsy_hi) : clip_pos(vy, ph.vis_lo, ph.vis_hi);
     }
     if (GRAD && I >= 1) {
@@ -295,23 +293,24 @@ __device__ __forceinline__ void flux_force_body(const Grid &g, const Metrics &m,
     }
   }
   if (FORCE) {
+    const Fp64 w(I);
     // f = 0.5 (rho_l + rho_r) 2 / (1 + denr) / We 0.5 (k_l + k_r) (phi_r - phi_l) / h
     if (I >= 2) {
       double f = 0.;
       if (!same(vxm, v0)) {
-        const double rho = den0[ix(g, r, I - 1)] + den0[ix(g, r, I)];
+        const double rho = w.add(den0[ix(g, r, I - 1)], den0[ix(g, r, I)]);
         const double kap = ITF_KAPPA ? face_kappa_sum(vxm, v0, curv[ix(g, r, I - 1)], curv[ix(g, r, I)])
-                                     : curv[ix(g, r, I - 1)] + curv[ix(g, r, I)];
-        f = (rho * kap) * ((ph.qf * m.ihxxf[I]) * (v0 - vxm));
+                                     : w.add(curv[ix(g, r, I - 1)], curv[ix(g, r, I)]);
+        f = w.mul(w.mul(rho, kap), w.mul(w.mul(w.reg(ph.qf), m.ihxxf[I]), w.sub(v0, vxm)));
       }
       ifrcx[ix(g, r, I - 2)] = f;
     }
     double f = 0.;
     if (!same(vym, v0)) {
-      const double rho = den0[ix(g, rm, I)] + den0[ix(g, r, I)];
+      const double rho = w.add(den0[ix(g, rm, I)], den0[ix(g, r, I)]);
       const double kap = ITF_KAPPA ? face_kappa_sum(vym, v0, curv[ix(g, rm, I)], curv[ix(g, r, I)])
-                                   : curv[ix(g, rm, I)] + curv[ix(g, r, I)];
-      f = (rho * kap) * (ph.qfy * (v0 - vym));
+                                   : w.add(curv[ix(g, rm, I)], curv[ix(g, r, I)]);
+      f = w.mul(w.mul(rho, kap), w.mul(w.reg(ph.qfy), w.sub(v0, vym)));
     }
     ifrcy[ix(g, r, I - 1)] = f;
   }
@@ -387,9 +386,10 @@ __device__ __forceinline__ void cell_curv(const Grid &g, const Metrics &m, const
   const int r = J - 1 + zr, rp = wrap(J + 1, g.ny) + zr;
   const double2 d00 = dv[(size_t)r * q + (I - 1)], d10 = dv[(size_t)r * q + I];
   const double2 d01 = dv[(size_t)rp * q + (I - 1)], d11 = dv[(size_t)rp * q + I];
-  const double ddx = (d10.x + d11.x) - (d00.x + d01.x);
-  const double ddy = (d01.y + d11.y) - (d00.y + d10.y);
-  curv[ix(g, r, I)] = -fma(m.hihxxc[I], ddx, g.hihy * ddy);
+  const Fp64 f(I);
+  const double ddx = f.sub(f.add(d10.x, d11.x), f.add(d00.x, d01.x));
+  const double ddy = f.sub(f.add(d01.y, d11.y), f.add(d00.y, d10.y));
+  curv[ix(g, r, I)] = -fma(m.hihxxc[I], ddx, f.mul(f.reg(g.hihy), ddy));
 }
 
 // unit normal (n0, n1) and K = 1/phi - 1 of interface cell (I, J) of a case
@@ -607,7 +607,8 @@ __global__ void __launch_bounds__(BX *BY)
   const int r = J - 1 + zr, rp = wrap(J + 1, g.ny) + zr;
   const double fxm = fluxx[ix(g, r, I - 1)], fxp = fluxx[ix(g, r, I)];
   const double fym = fluxy[ix(g, r, I)], fyp = fluxy[ix(g, rp, I)];
-  const double s = fma(m.ihxxc[I], fxm - fxp, g.ihy * (fym - fyp));
+  const Fp64 f(I);
+  const double s = fma(m.ihxxc[I], f.sub(fxm, fxp), f.mul(f.reg(g.ihy), f.sub(fym, fyp)));
   src_a[ix(g, r, I - 1)] = s;
   double v = vof[ix(g, r, I)];
   v = fma(sc[sc_adt(k)], s, v);
@@ -617,8 +618,8 @@ __global__ void __launch_bounds__(BX *BY)
   if (I == 1) vo[ix(g, r, 0)] = 0.;
   if (I == g.nx) vo[ix(g, r, g.nx + 1)] = 0.;
   if (FUSED) {
-    const double c = ph.dm1;
-    den1[ix(g, r, I)] = clip_pos(fma(c, v, 1.), ph.den_lo, ph.den_hi);
+    const double c = f.reg(ph.dm1);
+    den1[ix(g, r, I)] = clip_pos(fma(c, v, f.one), ph.den_lo, ph.den_hi);
     mfx[ix(g, r, I - 1)] = fma(c, fxm, ux[ix(g, r, I - 1)]);
     mfy[ix(g, r, I)] = fma(c, fym, uy[ix(g, r, I)]);
     if (I == 1) {
@@ -858,6 +859,7 @@ __global__ void __launch_bounds__(BX *BY)
   const int I = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int J = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (I > g.nx + 1 || J > g.ny) return;
+  const Fp64 f(I);
   const int zr = blockIdx.z * g.ny;  // first row of this case
   const int r = J - 1 + zr, rm = wrap(J - 1, g.ny) + zr, rp = wrap(J + 1, g.ny) + zr;
   const double u0 = ux[ix(g, r, I - 1)];    // ux at face I, row J
@@ -867,14 +869,14 @@ __global__ void __launch_bounds__(BX *BY)
   {
     // corner (I, J - 1/2): txy = 0.5 (mu_s + mu_n) du/dy + 0.5 (mu_w + mu_e) dv/dx
     const double us = ux[ix(g, rm, I - 1)], ww = uy[ix(g, r, I - 1)];
-    const double sx = visux[ix(g, rm, I - 1)] + vx0;
-    const double sy = visuy[ix(g, r, I - 1)] + vy0;
-    const double du = u0 - us, dw = w0 - ww;
-    const double t4 = SCALED ? fma(sx, du, sy * (dw * c2nuf[I])) : fma(sx, du * ph.nuy2, sy * (dw * c2nuf[I]));  // 4 nu txy
-    const double fy = mfy[ix(g, r, I - 1)] + mfy[ix(g, r, I)];
-    const double fx = mfx[ix(g, rm, I - 1)] + mfx[ix(g, r, I - 1)];
-    pxy[ix(g, r, I - 1)] = fma(-(m.rq[I] * fy), us + u0, t4);
-    pyx[ix(g, r, I - 1)] = fma(-fx, ww + w0, t4);
+    const double sx = f.add(visux[ix(g, rm, I - 1)], vx0);
+    const double sy = f.add(visuy[ix(g, r, I - 1)], vy0);
+    const double du = f.sub(u0, us), dw = f.sub(w0, ww);
+    const double t4 = fma(sx, SCALED ? du : du * ph.nuy2, f.mul(sy, f.mul(dw, c2nuf[I])));  // 4 nu txy
+    const double fy = f.add(mfy[ix(g, r, I - 1)], mfy[ix(g, r, I)]);
+    const double fx = f.add(mfx[ix(g, rm, I - 1)], mfx[ix(g, r, I - 1)]);
+    pxy[ix(g, r, I - 1)] = fma(-f.mul(m.rq[I], fy), f.add(us, u0), t4);
+    pyx[ix(g, r, I - 1)] = fma(-fx, f.add(ww, w0), t4);
     if (STRESS == 2 || (STRESS == 1 && (I == 1 || I == g.nx + 1)))
       txy[ix(g, r, I - 1)] = SCALED ? fma(sx, du * (g.hihy * ph.inuy2), sy * (dw * (m.hihxxf[I] * ph.inuy4)))
                                     : fma(sx, du * g.hihy, sy * (dw * m.hihxxf[I]));
@@ -882,10 +884,10 @@ __global__ void __launch_bounds__(BX *BY)
   if (I <= g.nx) {
     // centre (I, J): txx = (mu_l + mu_r) du/dx, tyy = (mu_s + mu_n) dv/dy
     const double u1 = ux[ix(g, r, I)], w1 = uy[ix(g, rp, I)];
-    const double sx = vx0 + visux[ix(g, r, I)], sy = vy0 + visuy[ix(g, rp, I)];
-    const double du = u1 - u0, dw = w1 - w0;
-    pxx[ix(g, r, I - 1)] = fma(-(mfx[ix(g, r, I - 1)] + mfx[ix(g, r, I)]), u0 + u1, sx * (du * c4nuc[I]));
-    pyy[ix(g, r, I - 1)] = fma(-(mfy[ix(g, r, I)] + mfy[ix(g, rp, I)]), w0 + w1, SCALED ? sy * dw : sy * (dw * ph.nuy4));
+    const double sx = f.add(vx0, visux[ix(g, r, I)]), sy = f.add(vy0, visuy[ix(g, rp, I)]);
+    const double du = f.sub(u1, u0), dw = f.sub(w1, w0);
+    pxx[ix(g, r, I - 1)] = fma(-f.add(mfx[ix(g, r, I - 1)], mfx[ix(g, r, I)]), f.add(u0, u1), f.mul(sx, f.mul(du, c4nuc[I])));
+    pyy[ix(g, r, I - 1)] = fma(-f.add(mfy[ix(g, r, I)], mfy[ix(g, rp, I)]), f.add(w0, w1), f.mul(sy, SCALED ? dw : dw * ph.nuy4));
     if (STRESS == 2) {
       txx[ix(g, r, I - 1)] = sx * (du * m.ihxxc[I]);
       tyy[ix(g, r, I - 1)] = sy * (dw * g.ihy);
@@ -931,6 +933,7 @@ __global__ void __launch_bounds__(BX *BY)
   const int I = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int J = blockIdx.y * blockDim.y + threadIdx.y + 1;
   if (I > g.nx || J > g.ny) return;
+  const Fp64 f(I);
   const int zr = blockIdx.z * g.ny;  // first row of this case
   const int r = J - 1 + zr, rm = wrap(J - 1, g.ny) + zr, rp = wrap(J + 1, g.ny) + zr;
   // the update is carried as 2u with 2 alpha dt, ... and 1 / (2 rho_face):
@@ -941,25 +944,26 @@ __global__ void __launch_bounds__(BX *BY)
   // e grad psi_old is stored times the Poisson factor pax (x faces) or pay
   // (y faces): e pa = (2 rho_ref pa) / (2 rho) - pa
   const double rpx = sc[sc_rpx(k)], pax = sc[sc_pax(k)];
+  const double q4y = f.reg(g.q4y), hgrav = f.reg(ph.hgrav);
   const double ps0 = CACHED && I != 1 && I != g.nx ? 0. : psio[ix(g, r, I)];
   // ---- ux at face I
   if (I >= 2) {
     const double u0 = ux[ix(g, r, I - 1)];
     double a = ifrcx[ix(g, r, I - 2)];
-    const double rho0 = CACHED ? srx[ix(g, r, I - 1)] : den0[ix(g, r, I - 1)] + den0[ix(g, r, I)];  // 2 rho^k
-    a = fma(ph.hgrav, rho0, a);
-    a = fma(m.q4f[I], pxx[ix(g, r, I - 1)] - pxx[ix(g, r, I - 2)], a);
-    a = fma(g.q4y, pxy[ix(g, rp, I - 1)] - pxy[ix(g, r, I - 1)], a);
-    const double rho1 = den1[ix(g, r, I - 1)] + den1[ix(g, r, I)];  // 2 rho^{k+1}
+    const double rho0 = CACHED ? srx[ix(g, r, I - 1)] : f.add(den0[ix(g, r, I - 1)], den0[ix(g, r, I)]);  // 2 rho^k
+    a = fma(hgrav, rho0, a);
+    a = fma(m.q4f[I], f.sub(pxx[ix(g, r, I - 1)], pxx[ix(g, r, I - 2)]), a);
+    a = fma(q4y, f.sub(pxy[ix(g, rp, I - 1)], pxy[ix(g, r, I - 1)]), a);
+    const double rho1 = f.add(den1[ix(g, r, I - 1)], den1[ix(g, r, I)]);  // 2 rho^{k+1}
     srx[ix(g, r, I - 1)] = rho1;
-    const double ir2 = rcp_nr(rho1);
-    double u = fma(adt2, a, rho0 * u0);
+    const double ir2 = rcp_nr(rho1, f);
+    double u = fma(adt2, a, f.mul(rho0, u0));
     if (k != 0) u = fma(bdt2, sxb[ix(g, r, I - 2)], u);
-    u = fma(gx[I], p[ix(g, r, I - 1)] - p[ix(g, r, I)], u);
-    const double us = u * ir2;
+    u = fma(gx[I], f.sub(p[ix(g, r, I - 1)], p[ix(g, r, I)]), u);
+    const double us = f.mul(u, ir2);
     ux_out[ix(g, r, I - 1)] = us;
     sxa[ix(g, r, I - 2)] = a;
-    const double e = fma(rpx, ir2, -pax) * (CACHED ? dpx[ix(g, r, I - 1)] : ps0 - psio[ix(g, r, I - 1)]);
+    const double e = f.mul(fma(rpx, ir2, -pax), CACHED ? dpx[ix(g, r, I - 1)] : f.sub(ps0, psio[ix(g, r, I - 1)]));
     egx[ix(g, r, I - 1)] = e;
     qx[ix(g, r, I - 1)] = fma(sc[sc_pdx(k)], us, e);
   }
@@ -967,20 +971,20 @@ __global__ void __launch_bounds__(BX *BY)
   {
     const double w0 = uy[ix(g, r, I)];
     double a = ifrcy[ix(g, r, I - 1)];
-    a = fma(m.q4c[I], pyx[ix(g, r, I)] - pyx[ix(g, r, I - 1)], a);
-    a = fma(g.q4y, pyy[ix(g, r, I - 1)] - pyy[ix(g, rm, I - 1)], a);
-    const double rho0 = CACHED ? sry[ix(g, r, I)] : den0[ix(g, rm, I)] + den0[ix(g, r, I)];  // 2 rho^k
-    const double rho1 = den1[ix(g, rm, I)] + den1[ix(g, r, I)];
+    a = fma(m.q4c[I], f.sub(pyx[ix(g, r, I)], pyx[ix(g, r, I - 1)]), a);
+    a = fma(q4y, f.sub(pyy[ix(g, r, I - 1)], pyy[ix(g, rm, I - 1)]), a);
+    const double rho0 = CACHED ? sry[ix(g, r, I)] : f.add(den0[ix(g, rm, I)], den0[ix(g, r, I)]);  // 2 rho^k
+    const double rho1 = f.add(den1[ix(g, rm, I)], den1[ix(g, r, I)]);
     sry[ix(g, r, I)] = rho1;
-    const double ir2 = rcp_nr(rho1);
-    double u = fma(adt2, a, rho0 * w0);
+    const double ir2 = rcp_nr(rho1, f);
+    double u = fma(adt2, a, f.mul(rho0, w0));
     if (k != 0) u = fma(bdt2, syb[ix(g, r, I - 1)], u);
-    u = fma(sc[sc_gdt2y(k)], p[ix(g, rm, I)] - p[ix(g, r, I)], u);
-    const double ws = u * ir2;
+    u = fma(sc[sc_gdt2y(k)], f.sub(p[ix(g, rm, I)], p[ix(g, r, I)]), u);
+    const double ws = f.mul(u, ir2);
     uy_out[ix(g, r, I)] = ws;
     sya[ix(g, r, I - 1)] = a;
     const double e =
-        fma(sc[sc_rpy(k)], ir2, -sc[sc_pay(k)]) * (CACHED ? dpy[ix(g, r, I)] : ps0 - psio[ix(g, rm, I)]);
+        f.mul(fma(sc[sc_rpy(k)], ir2, -sc[sc_pay(k)]), CACHED ? dpy[ix(g, r, I)] : f.sub(ps0, psio[ix(g, rm, I)]));
     egy[ix(g, r, I)] = e;
     qy[ix(g, r, I)] = fma(sc[sc_pdy(k)], ws, e);
   }
@@ -1032,7 +1036,8 @@ __global__ void __launch_bounds__(BX *BY)
 // tw: the twiddle buffer, exp(-2 pi i m / 2M) for m = 0..M, then W_M^e for
 // e < M, then their conjugates (the inverse's): one load per twiddle.
 template <int W>
-__device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__restrict__ tw, bool inverse) {
+__device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__restrict__ tw, bool inverse, const Fp64 &f) {
+  const double two = f.reg(2.);
   const double2 *__restrict__ wm = tw + (M + 1) + (inverse ? M : 0);
   int Ns = 1;
   if ((__ffs(M) - 1) & 1) {  // log2 M odd (M >= 8): an untwiddled radix-8 stage
@@ -1040,7 +1045,7 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
     // 1/sqrt(2) of W8 and W8^3 rides in the odd half's last FMAs: 52 FP64
     // operations for 8 points, where a radix-2 stage and a twiddled radix-4
     // stage take 64 for the same three levels
-    const double c8 = 0.70710678118654752440;
+    const double c8 = f.reg(0.70710678118654752440);
     const int q8 = M >> 3;
     for (int t = threadIdx.x; t < W * q8; t += blockDim.x) {
       const int c = t / q8, j = t - c * q8;
@@ -1050,24 +1055,24 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const double2 u = xr[j + q * q8], w = xr[j + (q + 4) * q8];
-        a[q] = cadd(u, w);
-        b[q] = csub(u, w);
+        a[q] = f.cadd(u, w);
+        b[q] = f.csub(u, w);
       }
       // even outputs: DFT4 of a; -i (forward) or +i (inverse) rotations are sign flips
-      const double2 e0 = cadd(a[0], a[2]), e1 = csub(a[0], a[2]), e2 = cadd(a[1], a[3]), e3 = csub(a[1], a[3]);
+      const double2 e0 = f.cadd(a[0], a[2]), e1 = f.csub(a[0], a[2]), e2 = f.cadd(a[1], a[3]), e3 = f.csub(a[1], a[3]);
       const double2 re3 = inverse ? make_double2(-e3.y, e3.x) : make_double2(e3.y, -e3.x);
-      yr[0] = cadd(e0, e2);
-      yr[2] = cadd(e1, re3);
-      yr[4] = csub(e0, e2);
-      yr[6] = csub(e1, re3);
+      yr[0] = f.cadd(e0, e2);
+      yr[2] = f.cadd(e1, re3);
+      yr[4] = f.csub(e0, e2);
+      yr[6] = f.csub(e1, re3);
       // odd outputs: t1 = b1 W8 = c8 P1, t2 = b2 W8^2 (a rotation), t3 = b3 W8^3 = c8 P3
-      const double2 P1 = inverse ? make_double2(b[1].x - b[1].y, b[1].x + b[1].y)
-                                 : make_double2(b[1].x + b[1].y, b[1].y - b[1].x);
-      const double2 P3 = inverse ? make_double2(-(b[3].x + b[3].y), b[3].x - b[3].y)
-                                 : make_double2(b[3].y - b[3].x, -(b[3].x + b[3].y));
+      const double2 P1 = inverse ? make_double2(f.sub(b[1].x, b[1].y), f.add(b[1].x, b[1].y))
+                                 : make_double2(f.add(b[1].x, b[1].y), f.sub(b[1].y, b[1].x));
+      const double2 P3 = inverse ? make_double2(-f.add(b[3].x, b[3].y), f.sub(b[3].x, b[3].y))
+                                 : make_double2(f.sub(b[3].y, b[3].x), -f.add(b[3].x, b[3].y));
       const double2 t2 = inverse ? make_double2(-b[2].y, b[2].x) : make_double2(b[2].y, -b[2].x);
-      const double2 A0 = cadd(b[0], t2), A1 = csub(b[0], t2);
-      const double2 E = cadd(P1, P3), D = csub(P1, P3);  // t1 + t3 = c8 E, t1 - t3 = c8 D
+      const double2 A0 = f.cadd(b[0], t2), A1 = f.csub(b[0], t2);
+      const double2 E = f.cadd(P1, P3), D = f.csub(P1, P3);  // t1 + t3 = c8 E, t1 - t3 = c8 D
       const double2 rD = inverse ? make_double2(-D.y, D.x) : make_double2(D.y, -D.x);
       yr[1] = make_double2(fma(c8, E.x, A0.x), fma(c8, E.y, A0.y));
       yr[3] = make_double2(fma(c8, rD.x, A1.x), fma(c8, rD.y, A1.y));
@@ -1097,23 +1102,23 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
         const int e = kk * step;
         const double2 w1 = wm[e], w2 = wm[2 * e], w3 = wm[3 * e];
         a0 = make_double2(fma(w2.x, v2.x, fma(-w2.y, v2.y, v0.x)), fma(w2.x, v2.y, fma(w2.y, v2.x, v0.y)));
-        a1 = make_double2(fma(2., v0.x, -a0.x), fma(2., v0.y, -a0.y));
-        const double2 t1 = cmul(v1, w1);
+        a1 = make_double2(fma(two, v0.x, -a0.x), fma(two, v0.y, -a0.y));
+        const double2 t1 = f.cmul(v1, w1);
         a2 = make_double2(fma(w3.x, v3.x, fma(-w3.y, v3.y, t1.x)), fma(w3.x, v3.y, fma(w3.y, v3.x, t1.y)));
-        a3 = make_double2(fma(2., t1.x, -a2.x), fma(2., t1.y, -a2.y));
+        a3 = make_double2(fma(two, t1.x, -a2.x), fma(two, t1.y, -a2.y));
       } else {
-        a0 = cadd(v0, v2);
-        a1 = csub(v0, v2);
-        a2 = cadd(v1, v3);
-        a3 = csub(v1, v3);
+        a0 = f.cadd(v0, v2);
+        a1 = f.csub(v0, v2);
+        a2 = f.cadd(v1, v3);
+        a3 = f.csub(v1, v3);
       }
       // -i a3 (forward) or +i a3 (inverse)
       const double2 r3 = inverse ? make_double2(-a3.y, a3.x) : make_double2(a3.y, -a3.x);
       const int d = ((j - kk) << 2) + kk;
-      yr[d] = cadd(a0, a2);
-      yr[d + Ns] = cadd(a1, r3);
-      yr[d + 2 * Ns] = csub(a0, a2);
-      yr[d + 3 * Ns] = csub(a1, r3);
+      yr[d] = f.cadd(a0, a2);
+      yr[d + Ns] = f.cadd(a1, r3);
+      yr[d + 2 * Ns] = f.csub(a0, a2);
+      yr[d + 3 * Ns] = f.csub(a1, r3);
     }
     __syncthreads();
     double2 *tmp = x;
@@ -1139,6 +1144,7 @@ __global__ void __launch_bounds__(256)
   double2 *A = smem, *B = smem + W * M;
   double *Ad = reinterpret_cast<double *>(A);
   const int I0 = blockIdx.x * W + 1;
+  const Fp64 f(blockIdx.x + threadIdx.x);
   const double pdx = sc[sc_pdx(k)], pdy = sc[sc_pdy(k)];
   for (int t = threadIdx.x; t < W * ny; t += blockDim.x) {
     const int c = t % W, r = t / W;
@@ -1151,7 +1157,7 @@ __global__ void __launch_bounds__(256)
       // differences of pax e grad psi_old and pay e grad psi_old across the
       // cell (its faces' values written by k_predict_mf or k_face_factor)
       if (Q) {
-        val = (ux[ix(g, rg, I)] - ux[ix(g, rg, I - 1)]) + (uy[ix(g, rp, I)] - uy[ix(g, rg, I)]);
+        val = f.add(f.sub(ux[ix(g, rg, I)], ux[ix(g, rg, I - 1)]), f.sub(uy[ix(g, rp, I)], uy[ix(g, rg, I)]));
       } else {
         const double X = egx[ix(g, rg, I)] - egx[ix(g, rg, I - 1)];
         const double Y = egy[ix(g, rp, I)] - egy[ix(g, rg, I)];
@@ -1163,7 +1169,7 @@ __global__ void __launch_bounds__(256)
     Ad[c * ny + r] = val;
   }
   __syncthreads();
-  double2 *Z = fft_rows<W>(A, B, M, tw, false);
+  double2 *Z = fft_rows<W>(A, B, M, tw, false, f);
   // the packed transform z_m, m < M; k_poisson_tdm does the real-to-complex
   // split (there the FP64 pipe has room)
   const int M1 = M + 1;
@@ -1184,6 +1190,7 @@ __global__ void __launch_bounds__(256)
   const int ny = g.ny, M = ny >> 1, M1 = M + 1;
   double2 *A = smem, *B = smem + W * M;
   const int I0 = blockIdx.x * W + 1;
+  const Fp64 f(blockIdx.x + threadIdx.x);
   for (int t = threadIdx.x; t < W * M; t += blockDim.x) {
     const int c = t / M, mm = t - c * M;
     const int I = I0 + c;
@@ -1192,7 +1199,7 @@ __global__ void __launch_bounds__(256)
     A[c * M + mm] = I <= g.nx ? spec[(size_t)(I - 1) * M1 + mm] : make_double2(0., 0.);
   }
   __syncthreads();
-  const double2 *zr = fft_rows<W>(A, B, M, tw, true);
+  const double2 *zr = fft_rows<W>(A, B, M, tw, true, f);
   const double *xd = reinterpret_cast<const double *>(zr);
   for (int t = threadIdx.x; t < W * ny; t += blockDim.x) {
     const int c = t % W, r = t / W;
@@ -1229,6 +1236,7 @@ __global__ void __launch_bounds__(512)
   pdl_entry();
   extern __shared__ double2 smem_d2[];
   __shared__ double xch[16][4][2];  // per system of the block, per warp of the system: a chunk-map total
+  const Fp64 f64(blockIdx.x + threadIdx.x);
   const int nx = g.nx, M = g.ny / 2, M1 = M + 1;
   const int p0 = blockIdx.x * PB;
   const int np = min(PB, M / 2 + 1 - p0);  // pairs (p, M - p), p = 0 .. M/2
@@ -1248,8 +1256,8 @@ __global__ void __launch_bounds__(512)
     if (i < nx) {
       const double2 zm = sp[(size_t)i * M1 + p];
       const double2 zr = sp[(size_t)i * M1 + (p == 0 ? 0 : M - p)];
-      const double2 E = make_double2(zm.x + zr.x, zm.y - zr.y);
-      const double2 O = make_double2(zm.y + zr.y, zr.x - zm.x);  // -i (zm - conj zr)
+      const double2 E = make_double2(f64.add(zm.x, zr.x), f64.sub(zm.y, zr.y));
+      const double2 O = make_double2(f64.add(zm.y, zr.y), f64.sub(zr.x, zm.x));  // -i (zm - conj zr)
       // X_p = E + w^p O; X_{M-p} = conj E + w^{M-p} conj O (the pair's E and O
       // with the signs of their imaginary parts flipped), products in FMAs
       const double2 wa = tw[p], wb = tw[M - p];
@@ -1278,7 +1286,7 @@ __global__ void __launch_bounds__(512)
 #pragma unroll 8
     for (int k = 0; k < L; ++k) {
       const double4_32a c = f[(size_t)k * lanes];
-      t = fma(-c.y, t, c.x * x[k]);
+      t = fma(-c.y, t, f64.mul(c.x, x[k]));
       x[k] = t;
     }
     T = t;
@@ -1288,7 +1296,7 @@ __global__ void __launch_bounds__(512)
       const double Tp = __shfl_up_sync(0xffffffffu, T, d), Bp = __shfl_up_sync(0xffffffffu, B, d);
       if (lane >= d) {
         T = fma(B, Tp, T);
-        B *= Bp;
+        B = f64.mul(B, Bp);
       }
     }
   }
@@ -1324,7 +1332,7 @@ __global__ void __launch_bounds__(512)
       const double Sp = __shfl_down_sync(0xffffffffu, Sx, d), Cp = __shfl_down_sync(0xffffffffu, Cc, d);
       if (lane + d < 32) {
         Sx = fma(Cc, Sp, Sx);
-        Cc *= Cp;
+        Cc = f64.mul(Cc, Cp);
       }
     }
   }
@@ -1378,8 +1386,8 @@ __global__ void __launch_bounds__(512)
     const double2 Xb = make_double2(sm[(4 * q + 2) * sys_len + at], sm[(4 * q + 3) * sys_len + at]);
     // z_p = E + i D conj w^p and z_{M-p} = conj E - i conj D conj w^{M-p}, with
     // E = X_p + conj X_{M-p}, D = X_p - conj X_{M-p}; products in FMAs
-    const double2 E = make_double2(Xa.x + Xb.x, Xa.y - Xb.y);
-    const double2 D = make_double2(Xa.x - Xb.x, Xa.y + Xb.y);
+    const double2 E = make_double2(f64.add(Xa.x, Xb.x), f64.sub(Xa.y, Xb.y));
+    const double2 D = make_double2(f64.sub(Xa.x, Xb.x), f64.add(Xa.y, Xb.y));
     const double2 wa = tw[p];
     sp[(size_t)i * M1 + p] =
         make_double2(fma(D.x, wa.y, fma(-D.y, wa.x, E.x)), fma(D.y, wa.y, fma(D.x, wa.x, E.y)));
@@ -1411,6 +1419,7 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
   extern __shared__ double smem_cl[];
   // per system: forward (T, B) and backward (S, C) totals of this CTA's warp, the gauge sum
   __shared__ double xf[4][2], xb[4][2], xg[4];
+  const Fp64 f64(blockIdx.x + threadIdx.x);
   const int nx = g.nx, M = g.ny / 2, M1 = M + 1;
   const int rank = (int)cl.block_rank();
   const int p = (int)blockIdx.x / kTdmCluster;  // the pair (p, M - p), p = 0 .. M/2
@@ -1425,8 +1434,8 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
     if (i < nx) {
       const double2 zm = sp[(size_t)i * M1 + p];
       const double2 zr = sp[(size_t)i * M1 + (p == 0 ? 0 : M - p)];
-      const double2 E = make_double2(zm.x + zr.x, zm.y - zr.y);
-      const double2 O = make_double2(zm.y + zr.y, zr.x - zm.x);
+      const double2 E = make_double2(f64.add(zm.x, zr.x), f64.sub(zm.y, zr.y));
+      const double2 O = make_double2(f64.add(zm.y, zr.y), f64.sub(zr.x, zm.x));
       const double2 wa = tw[p], wb = tw[M - p];
       xa = make_double2(fma(wa.x, O.x, fma(-wa.y, O.y, E.x)), fma(wa.x, O.y, fma(wa.y, O.x, E.y)));
       xbv = make_double2(fma(wb.x, O.x, fma(wb.y, O.y, E.x)), fma(wb.y, O.x, fma(-wb.x, O.y, -E.y)));
@@ -1448,7 +1457,7 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
 #pragma unroll 8
     for (int k = 0; k < L; ++k) {
       const double4_32a c = f[(size_t)k * lanes];
-      t = fma(-c.y, t, c.x * x[k]);
+      t = fma(-c.y, t, f64.mul(c.x, x[k]));
       x[k] = t;
     }
     T = t;
@@ -1458,7 +1467,7 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
       const double Tp = __shfl_up_sync(0xffffffffu, T, d), Bp = __shfl_up_sync(0xffffffffu, B, d);
       if (lane >= d) {
         T = fma(B, Tp, T);
-        B *= Bp;
+        B = f64.mul(B, Bp);
       }
     }
   }
@@ -1491,7 +1500,7 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
       const double Sp = __shfl_down_sync(0xffffffffu, Sx, d), Cp = __shfl_down_sync(0xffffffffu, Cc, d);
       if (lane + d < 32) {
         Sx = fma(Cc, Sp, Sx);
-        Cc *= Cp;
+        Cc = f64.mul(Cc, Cp);
       }
     }
   }
@@ -1539,8 +1548,8 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
     const int at = (t / L) * S + (t % L);
     const double2 Xa = make_double2(smem_cl[0 * sys_len + at], smem_cl[1 * sys_len + at]);
     const double2 Xb = make_double2(smem_cl[2 * sys_len + at], smem_cl[3 * sys_len + at]);
-    const double2 E = make_double2(Xa.x + Xb.x, Xa.y - Xb.y);
-    const double2 D = make_double2(Xa.x - Xb.x, Xa.y + Xb.y);
+    const double2 E = make_double2(f64.add(Xa.x, Xb.x), f64.sub(Xa.y, Xb.y));
+    const double2 D = make_double2(f64.sub(Xa.x, Xb.x), f64.add(Xa.y, Xb.y));
     const double2 wa = tw[p];
     sp[(size_t)i * M1 + p] =
         make_double2(fma(D.x, wa.y, fma(-D.y, wa.x, E.x)), fma(D.y, wa.y, fma(D.x, wa.x, E.y)));
@@ -1580,10 +1589,11 @@ __global__ void __launch_bounds__(BX *BY)
   const int zr = blockIdx.z * g.ny;  // first row of this case
   const int r = J - 1 + zr, rm = wrap(J - 1, g.ny) + zr;
   const double cnewy = sc[sc_cnewy(k)], coldyp = sc[sc_coldyp(k)];
+  const Fp64 f(I);
   const double pn0 = psin[ix(g, r, I)];
   if (I >= 2) {
     double u = ux[ix(g, r, I - 1)];
-    const double d = pn0 - psin[ix(g, r, I - 1)];
+    const double d = f.sub(pn0, psin[ix(g, r, I - 1)]);
     if (DP) dpx[ix(g, r, I - 1)] = d;
     u = fma(-cn[I], d, u);
     u = fma(co[I], egx[ix(g, r, I - 1)], u);
@@ -1591,7 +1601,7 @@ __global__ void __launch_bounds__(BX *BY)
   }
   {
     double u = uy[ix(g, r, I)];
-    const double d = pn0 - psin[ix(g, rm, I)];
+    const double d = f.sub(pn0, psin[ix(g, rm, I)]);
     if (DP) dpy[ix(g, r, I)] = d;
     u = fma(-cnewy, d, u);
     u = fma(coldyp, egy[ix(g, r, I)], u);
@@ -1606,7 +1616,7 @@ __global__ void __launch_bounds__(BX *BY)
     uy[ix(g, r, g.nx + 1)] = 0.;
   }
   if (PRES) {
-    const double pv = p[ix(g, r, I)] + pn0;
+    const double pv = f.add(p[ix(g, r, I)], pn0);
     p[ix(g, r, I)] = pv;
     if (I == 1) p[ix(g, r, 0)] = pv;
     if (I == g.nx) p[ix(g, r, g.nx + 1)] = pv;
