@@ -21,6 +21,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "sbfs_intfp.cuh"
+
 namespace sbfs {
 
 // per-column coefficients, index = I (0..nx+2), built on the host
@@ -199,6 +201,52 @@ struct Fp64 {
     return make_double2(fma(a.x, b.x, mul(-a.y, b.y)), fma(a.x, b.y, mul(a.y, b.x)));
   }
 };
+
+// The operations a kernel hands to the integer pipes (sbfs_intfp.cuh): INT
+// takes the integer forms and collects their `bad`, otherwise they run on the
+// FP64 unit like the rest.  A cell is computed with Fp64Int<true> and, where
+// bad is set, once more with Fp64Int<false>; the values are the same.
+template <bool INT>
+struct Fp64Int {
+  const Fp64 &f;
+  unsigned bad = 0;
+  __device__ __forceinline__ explicit Fp64Int(const Fp64 &f64) : f(f64) {}
+  __device__ __forceinline__ double add(double a, double b) { return INT ? intfp::add<false>(a, b, bad) : f.add(a, b); }
+  __device__ __forceinline__ double sub(double a, double b) { return INT ? intfp::sub<false>(a, b, bad) : f.sub(a, b); }
+  // a, b > 0
+  __device__ __forceinline__ double addp(double a, double b) { return INT ? intfp::addp(a, b, bad) : f.add(a, b); }
+  template <bool ZERO = false>
+  __device__ __forceinline__ void addsub(double a, double b, double &s, double &d) {
+    if (INT) {
+      intfp::addsub<ZERO>(a, b, s, d, bad);
+    } else {
+      s = f.add(a, b);
+      d = f.sub(a, b);
+    }
+  }
+  __device__ __forceinline__ double mul(double a, double b) {
+    return INT ? intfp::mul<false>(a, b, bad) : f.mul(a, b);
+  }
+  // addsub<true> and mulz: where both operands, or one, are often exactly zero
+  __device__ __forceinline__ double mulz(double a, double b) {
+    return INT ? intfp::mul<true>(a, b, bad) : f.mul(a, b);
+  }
+};
+
+// the same row index, opaque: the FP64 repeat of a cell reads its inputs again
+// instead of keeping them in registers across the integer forms (k_predict_mf
+// 84 registers with them, two blocks an SM)
+__device__ __forceinline__ int reread(int r) {
+  asm volatile("" : "+r"(r));
+  return r;
+}
+
+// one double from global to shared memory without a register in between; a
+// thread's own copies have arrived after async_wait
+__device__ __forceinline__ void async_copy(double *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // bit-level helpers: sign and threshold tests on the integer pattern of a
 // double keep these comparisons off the FP64 pipe

@@ -844,8 +844,48 @@ __global__ void __launch_bounds__(BX *BY)
 // thread (I, J): I = 1..nx+1 handles the corner (I, J - 1/2) and, for I <= nx,
 // the centre (I, J)
 // ---------------------------------------------------------------------------
+struct MomIn {
+  double u0, us, u1, w0, ww, w1;        // ux at face I: row J, row J-1; at face I+1.  uy: cell I, I-1; row J+1/2
+  double vx0, vxs, vx1, vy0, vyw, vyn;  // viscosities, likewise
+  double mx0, mxs, mx1, my0, myw, my1;  // mass fluxes, likewise
+  double rq, c2, c4;
+};
+struct MomOut {
+  double xx, yy, xy, yx;
+};
+
+// the four fluxes of one thread; returns whether an integer form gave up.
+// Of the 27 FP64 operations (SCALED) the four sum-and-difference pairs of the
+// velocities and four of the products run on the integer pipes.  2048 x 1024
+// swarm, one launch: 110.6 us all in FP64 (FP64 unit 85% busy); 69.1 us with
+// a fifth product on the integer side (integer pipes 90%, FP64 73%), 73.6 us
+// with one sum more; 65.9 us as it stands (89%, 82%).
+template <bool INT, bool SCALED>
+__device__ __forceinline__ bool momflux_cell(const Fp64 &f, const MomIn &in, const Phys &ph, MomOut &o) {
+  Fp64Int<INT> q(f);
+  {
+    double su, du, sw, dw;
+    q.template addsub<true>(in.u0, in.us, su, du);  // zero along the walls
+    q.addsub(in.w0, in.ww, sw, dw);
+    const double sx = f.add(in.vxs, in.vx0), sy = f.add(in.vyw, in.vy0);
+    const double t4 = fma(sx, SCALED ? du : f.mul(du, f.reg(ph.nuy2)), q.mul(sy, q.mul(dw, in.c2)));  // 4 nu txy
+    const double fy = f.add(in.myw, in.my0), fx = f.add(in.mxs, in.mx0);
+    o.xy = fma(-q.mul(in.rq, fy), su, t4);
+    o.yx = fma(-fx, sw, t4);
+  }
+  {
+    double su, du, sw, dw;
+    q.addsub(in.u1, in.u0, su, du);
+    q.addsub(in.w1, in.w0, sw, dw);
+    const double sx = f.add(in.vx0, in.vx1), sy = f.add(in.vy0, in.vyn);
+    o.xx = fma(-f.add(in.mx0, in.mx1), su, f.mul(sx, q.mul(du, in.c4)));
+    o.yy = fma(-f.add(in.my0, in.my1), sw, f.mul(sy, SCALED ? dw : f.mul(dw, f.reg(ph.nuy4))));
+  }
+  return INT && q.bad != 0;
+}
+
 template <int STRESS, bool SCALED>
-__global__ void __launch_bounds__(BX *BY)
+__global__ void __launch_bounds__(BX *BY, 5)
     k_momflux(Grid g, Metrics m, Phys ph0, const double *__restrict__ ux, const double *__restrict__ uy,
               const double *__restrict__ visux, const double *__restrict__ visuy, const double *__restrict__ mfx,
               const double *__restrict__ mfy, double *__restrict__ pxx, double *__restrict__ pyy,
@@ -862,35 +902,57 @@ __global__ void __launch_bounds__(BX *BY)
   const Fp64 f(I);
   const int zr = blockIdx.z * g.ny;  // first row of this case
   const int r = J - 1 + zr, rm = wrap(J - 1, g.ny) + zr, rp = wrap(J + 1, g.ny) + zr;
-  const double u0 = ux[ix(g, r, I - 1)];    // ux at face I, row J
-  const double vx0 = visux[ix(g, r, I - 1)];
-  const double w0 = uy[ix(g, r, I)];        // uy of cell I at J - 1/2
-  const double vy0 = visuy[ix(g, r, I)];
-  {
-    // corner (I, J - 1/2): txy = 0.5 (mu_s + mu_n) du/dy + 0.5 (mu_w + mu_e) dv/dx
-    const double us = ux[ix(g, rm, I - 1)], ww = uy[ix(g, r, I - 1)];
-    const double sx = f.add(visux[ix(g, rm, I - 1)], vx0);
-    const double sy = f.add(visuy[ix(g, r, I - 1)], vy0);
-    const double du = f.sub(u0, us), dw = f.sub(w0, ww);
-    const double t4 = fma(sx, SCALED ? du : du * ph.nuy2, f.mul(sy, f.mul(dw, c2nuf[I])));  // 4 nu txy
-    const double fy = f.add(mfy[ix(g, r, I - 1)], mfy[ix(g, r, I)]);
-    const double fx = f.add(mfx[ix(g, rm, I - 1)], mfx[ix(g, r, I - 1)]);
-    pxy[ix(g, r, I - 1)] = fma(-f.mul(m.rq[I], fy), f.add(us, u0), t4);
-    pyx[ix(g, r, I - 1)] = fma(-fx, f.add(ww, w0), t4);
-    if (STRESS == 2 || (STRESS == 1 && (I == 1 || I == g.nx + 1)))
-      txy[ix(g, r, I - 1)] = SCALED ? fma(sx, du * (g.hihy * ph.inuy2), sy * (dw * (m.hihxxf[I] * ph.inuy4)))
-                                    : fma(sx, du * g.hihy, sy * (dw * m.hihxxf[I]));
+  const bool centre = I <= g.nx;
+  // centre (I, J); the threads of the last face have none and take the column before
+  const int Ic = centre ? I : I - 2;
+  auto load = [&](int r, int rm, int rp) {
+    MomIn in;
+    in.u0 = ux[ix(g, r, I - 1)];  // ux at face I, row J
+    in.vx0 = visux[ix(g, r, I - 1)];
+    in.w0 = uy[ix(g, r, I)];  // uy of cell I at J - 1/2
+    in.vy0 = visuy[ix(g, r, I)];
+    in.mx0 = mfx[ix(g, r, I - 1)];
+    in.my0 = mfy[ix(g, r, I)];
+    // corner (I, J - 1/2)
+    in.us = ux[ix(g, rm, I - 1)];
+    in.ww = uy[ix(g, r, I - 1)];
+    in.vxs = visux[ix(g, rm, I - 1)];
+    in.vyw = visuy[ix(g, r, I - 1)];
+    in.mxs = mfx[ix(g, rm, I - 1)];
+    in.myw = mfy[ix(g, r, I - 1)];
+    in.rq = m.rq[I];
+    in.c2 = c2nuf[I];
+    // centre
+    in.u1 = ux[ix(g, r, Ic)];
+    in.w1 = uy[ix(g, rp, centre ? I : Ic)];
+    in.vx1 = visux[ix(g, r, Ic)];
+    in.vyn = visuy[ix(g, rp, I)];
+    in.mx1 = mfx[ix(g, r, Ic)];
+    in.my1 = mfy[ix(g, rp, I)];
+    in.c4 = c4nuc[Ic];
+    return in;
+  };
+  MomIn in = load(r, rm, rp);
+  MomOut o;
+  if (momflux_cell<true, SCALED>(f, in, ph, o)) {
+    in = load(reread(r), reread(rm), reread(rp));
+    momflux_cell<false, SCALED>(f, in, ph, o);
   }
-  if (I <= g.nx) {
-    // centre (I, J): txx = (mu_l + mu_r) du/dx, tyy = (mu_s + mu_n) dv/dy
-    const double u1 = ux[ix(g, r, I)], w1 = uy[ix(g, rp, I)];
-    const double sx = f.add(vx0, visux[ix(g, r, I)]), sy = f.add(vy0, visuy[ix(g, rp, I)]);
-    const double du = f.sub(u1, u0), dw = f.sub(w1, w0);
-    pxx[ix(g, r, I - 1)] = fma(-f.add(mfx[ix(g, r, I - 1)], mfx[ix(g, r, I)]), f.add(u0, u1), f.mul(sx, f.mul(du, c4nuc[I])));
-    pyy[ix(g, r, I - 1)] = fma(-f.add(mfy[ix(g, r, I)], mfy[ix(g, rp, I)]), f.add(w0, w1), f.mul(sy, SCALED ? dw : dw * ph.nuy4));
+  pxy[ix(g, r, I - 1)] = o.xy;
+  pyx[ix(g, r, I - 1)] = o.yx;
+  if (STRESS == 2 || (STRESS == 1 && (I == 1 || I == g.nx + 1))) {
+    // txy = 0.5 (mu_s + mu_n) du/dy + 0.5 (mu_w + mu_e) dv/dx
+    const MomIn in = load(reread(r), reread(rm), reread(rp));
+    const double sx = in.vxs + in.vx0, sy = in.vyw + in.vy0, du = in.u0 - in.us, dw = in.w0 - in.ww;
+    txy[ix(g, r, I - 1)] = SCALED ? fma(sx, du * (g.hihy * ph.inuy2), sy * (dw * (m.hihxxf[I] * ph.inuy4)))
+                                  : fma(sx, du * g.hihy, sy * (dw * m.hihxxf[I]));
+  }
+  if (centre) {
+    pxx[ix(g, r, I - 1)] = o.xx;
+    pyy[ix(g, r, I - 1)] = o.yy;
     if (STRESS == 2) {
-      txx[ix(g, r, I - 1)] = sx * (du * m.ihxxc[I]);
-      tyy[ix(g, r, I - 1)] = sy * (dw * g.ihy);
+      txx[ix(g, r, I - 1)] = (in.vx0 + in.vx1) * ((in.u1 - in.u0) * m.ihxxc[I]);
+      tyy[ix(g, r, I - 1)] = (in.vy0 + in.vyn) * ((in.w1 - in.w0) * g.ihy);
     }
   }
 }
@@ -913,8 +975,45 @@ __global__ void __launch_bounds__(BX *BY)
 // thread (I, J): I = 1..nx handles the ux face I (I >= 2) and the uy face
 // (I, J - 1/2)
 // ---------------------------------------------------------------------------
+struct PredIn {
+  double u0, frc, rho0, dps;  // velocity, surface tension, 2 rho^k, psi_old's difference across the face
+  double pd1, pd0, po1, po0;  // fluxes either side of the face, along it and across
+  double r1a, r1b, p0, p1, sb;  // rho^{k+1} and p of the two cells, the last substage's right-hand side
+  double cd, co, gp, rp, pa, pd;
+};
+struct PredOut {
+  double rho1, u, a, e, q;
+};
+
+// one face; returns whether an integer form gave up.  The FP64 unit keeps the
+// fused multiply-adds and the pressure difference (zero everywhere in a first
+// step, which the integer form would leave to it).  2048 x 1024 swarm, one
+// launch: 137.4 us all in FP64; with the integer forms 119.8 us, the loads of
+// the second face then exposed (warps waiting on global memory 6.5 of 9.6
+// cycles an issue); 106 us with those loads in flight during the first face
+// (yb); 99.7 us at five blocks an SM and the pressure difference in FP64.
+template <bool INT, bool GRAV>
+__device__ __forceinline__ bool predict_face(const Fp64 &f, const PredIn &in, double hgrav, double adt2, double bdt2,
+                                             int k, PredOut &o) {
+  Fp64Int<INT> n(f);
+  double a = in.frc;
+  if (GRAV) a = fma(hgrav, in.rho0, a);
+  a = fma(in.cd, n.sub(in.pd1, in.pd0), a);
+  a = fma(in.co, n.sub(in.po1, in.po0), a);
+  o.rho1 = n.addp(in.r1a, in.r1b);  // 2 rho^{k+1}
+  const double ir2 = rcp_nr(o.rho1, f);
+  double u = fma(adt2, a, n.mul(in.rho0, in.u0));
+  if (k != 0) u = fma(bdt2, in.sb, u);
+  u = fma(in.gp, f.sub(in.p0, in.p1), u);
+  o.u = n.mul(u, ir2);
+  o.a = a;
+  o.e = n.mulz(fma(in.rp, ir2, -in.pa), in.dps);
+  o.q = fma(in.pd, o.u, o.e);
+  return INT && n.bad != 0;
+}
+
 template <bool CACHED>
-__global__ void __launch_bounds__(BX *BY)
+__global__ void __launch_bounds__(BX *BY, 5)
     k_predict_mf(Grid g, Metrics m, Phys ph0, const double *__restrict__ sc, int k, const double *__restrict__ ux,
                  const double *__restrict__ uy, double *__restrict__ ux_out, double *__restrict__ uy_out,
                  const double *__restrict__ pxx, const double *__restrict__ pyy, const double *__restrict__ pxy,
@@ -945,48 +1044,84 @@ __global__ void __launch_bounds__(BX *BY)
   // (y faces): e pa = (2 rho_ref pa) / (2 rho) - pa
   const double rpx = sc[sc_rpx(k)], pax = sc[sc_pax(k)];
   const double q4y = f.reg(g.q4y), hgrav = f.reg(ph.hgrav);
+  __shared__ double yb[11][BX * BY];
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  async_copy(&yb[0][tid], uy + ix(g, r, I));
+  async_copy(&yb[1][tid], ifrcy + ix(g, r, I - 1));
+  async_copy(&yb[2][tid], pyx + ix(g, r, I));
+  async_copy(&yb[3][tid], pyx + ix(g, r, I - 1));
+  async_copy(&yb[4][tid], pyy + ix(g, r, I - 1));
+  async_copy(&yb[5][tid], pyy + ix(g, rm, I - 1));
+  async_copy(&yb[6][tid], den1 + ix(g, rm, I));
+  async_copy(&yb[7][tid], p + ix(g, rm, I));
+  if (k != 0) async_copy(&yb[8][tid], syb + ix(g, r, I - 1));
+  if (CACHED) {
+    async_copy(&yb[9][tid], sry + ix(g, r, I));
+    async_copy(&yb[10][tid], dpy + ix(g, r, I));
+  }
   const double ps0 = CACHED && I != 1 && I != g.nx ? 0. : psio[ix(g, r, I)];
   // ---- ux at face I
   if (I >= 2) {
-    const double u0 = ux[ix(g, r, I - 1)];
-    double a = ifrcx[ix(g, r, I - 2)];
-    const double rho0 = CACHED ? srx[ix(g, r, I - 1)] : f.add(den0[ix(g, r, I - 1)], den0[ix(g, r, I)]);  // 2 rho^k
-    a = fma(hgrav, rho0, a);
-    a = fma(m.q4f[I], f.sub(pxx[ix(g, r, I - 1)], pxx[ix(g, r, I - 2)]), a);
-    a = fma(q4y, f.sub(pxy[ix(g, rp, I - 1)], pxy[ix(g, r, I - 1)]), a);
-    const double rho1 = f.add(den1[ix(g, r, I - 1)], den1[ix(g, r, I)]);  // 2 rho^{k+1}
-    srx[ix(g, r, I - 1)] = rho1;
-    const double ir2 = rcp_nr(rho1, f);
-    double u = fma(adt2, a, f.mul(rho0, u0));
-    if (k != 0) u = fma(bdt2, sxb[ix(g, r, I - 2)], u);
-    u = fma(gx[I], f.sub(p[ix(g, r, I - 1)], p[ix(g, r, I)]), u);
-    const double us = f.mul(u, ir2);
-    ux_out[ix(g, r, I - 1)] = us;
-    sxa[ix(g, r, I - 2)] = a;
-    const double e = f.mul(fma(rpx, ir2, -pax), CACHED ? dpx[ix(g, r, I - 1)] : f.sub(ps0, psio[ix(g, r, I - 1)]));
-    egx[ix(g, r, I - 1)] = e;
-    qx[ix(g, r, I - 1)] = fma(sc[sc_pdx(k)], us, e);
+    auto load = [&](int r, int rm, int rp) {
+      PredIn in;
+      in.u0 = ux[ix(g, r, I - 1)];
+      in.frc = ifrcx[ix(g, r, I - 2)];
+      in.pd1 = pxx[ix(g, r, I - 1)], in.pd0 = pxx[ix(g, r, I - 2)];
+      in.po1 = pxy[ix(g, rp, I - 1)], in.po0 = pxy[ix(g, r, I - 1)];
+      in.r1a = den1[ix(g, r, I - 1)], in.r1b = den1[ix(g, r, I)];
+      in.p0 = p[ix(g, r, I - 1)], in.p1 = p[ix(g, r, I)];
+      in.sb = k != 0 ? sxb[ix(g, r, I - 2)] : 0.;
+      in.rho0 = CACHED ? srx[ix(g, r, I - 1)] : f.add(den0[ix(g, r, I - 1)], den0[ix(g, r, I)]);  // 2 rho^k
+      in.dps = CACHED ? dpx[ix(g, r, I - 1)] : f.sub(ps0, psio[ix(g, r, I - 1)]);
+      in.cd = m.q4f[I], in.co = q4y, in.gp = gx[I], in.rp = rpx, in.pa = pax, in.pd = sc[sc_pdx(k)];
+      return in;
+    };
+    PredOut o;
+    if (predict_face<true, true>(f, load(r, rm, rp), hgrav, adt2, bdt2, k, o))
+      predict_face<false, true>(f, load(reread(r), reread(rm), reread(rp)), hgrav, adt2, bdt2, k, o);
+    srx[ix(g, r, I - 1)] = o.rho1;
+    ux_out[ix(g, r, I - 1)] = o.u;
+    sxa[ix(g, r, I - 2)] = o.a;
+    egx[ix(g, r, I - 1)] = o.e;
+    qx[ix(g, r, I - 1)] = o.q;
   }
   // ---- uy at face (I, J - 1/2)
   {
-    const double w0 = uy[ix(g, r, I)];
-    double a = ifrcy[ix(g, r, I - 1)];
-    a = fma(m.q4c[I], f.sub(pyx[ix(g, r, I)], pyx[ix(g, r, I - 1)]), a);
-    a = fma(q4y, f.sub(pyy[ix(g, r, I - 1)], pyy[ix(g, rm, I - 1)]), a);
-    const double rho0 = CACHED ? sry[ix(g, r, I)] : f.add(den0[ix(g, rm, I)], den0[ix(g, r, I)]);  // 2 rho^k
-    const double rho1 = f.add(den1[ix(g, rm, I)], den1[ix(g, r, I)]);
-    sry[ix(g, r, I)] = rho1;
-    const double ir2 = rcp_nr(rho1, f);
-    double u = fma(adt2, a, f.mul(rho0, w0));
-    if (k != 0) u = fma(bdt2, syb[ix(g, r, I - 1)], u);
-    u = fma(sc[sc_gdt2y(k)], f.sub(p[ix(g, rm, I)], p[ix(g, r, I)]), u);
-    const double ws = f.mul(u, ir2);
-    uy_out[ix(g, r, I)] = ws;
-    sya[ix(g, r, I - 1)] = a;
-    const double e =
-        f.mul(fma(sc[sc_rpy(k)], ir2, -sc[sc_pay(k)]), CACHED ? dpy[ix(g, r, I)] : f.sub(ps0, psio[ix(g, rm, I)]));
-    egy[ix(g, r, I)] = e;
-    qy[ix(g, r, I)] = fma(sc[sc_pdy(k)], ws, e);
+    auto coefs = [&](PredIn &in) {
+      in.cd = m.q4c[I], in.co = q4y, in.gp = sc[sc_gdt2y(k)], in.rp = sc[sc_rpy(k)], in.pa = sc[sc_pay(k)],
+      in.pd = sc[sc_pdy(k)];
+    };
+    async_wait();
+    PredIn in;
+    in.u0 = yb[0][tid], in.frc = yb[1][tid];
+    in.pd1 = yb[2][tid], in.pd0 = yb[3][tid];
+    in.po1 = yb[4][tid], in.po0 = yb[5][tid];
+    in.r1a = yb[6][tid], in.r1b = den1[ix(g, r, I)];
+    in.p0 = yb[7][tid], in.p1 = p[ix(g, r, I)];
+    in.sb = k != 0 ? yb[8][tid] : 0.;
+    in.rho0 = CACHED ? yb[9][tid] : f.add(den0[ix(g, rm, I)], den0[ix(g, r, I)]);  // 2 rho^k
+    in.dps = CACHED ? yb[10][tid] : f.sub(ps0, psio[ix(g, rm, I)]);
+    coefs(in);
+    PredOut o;
+    if (predict_face<true, false>(f, in, hgrav, adt2, bdt2, k, o)) {
+      const int r_ = reread(r), rm_ = reread(rm);
+      in.u0 = uy[ix(g, r_, I)];
+      in.frc = ifrcy[ix(g, r_, I - 1)];
+      in.pd1 = pyx[ix(g, r_, I)], in.pd0 = pyx[ix(g, r_, I - 1)];
+      in.po1 = pyy[ix(g, r_, I - 1)], in.po0 = pyy[ix(g, rm_, I - 1)];
+      in.r1a = den1[ix(g, rm_, I)], in.r1b = den1[ix(g, r_, I)];
+      in.p0 = p[ix(g, rm_, I)], in.p1 = p[ix(g, r_, I)];
+      in.sb = k != 0 ? syb[ix(g, r_, I - 1)] : 0.;
+      in.rho0 = CACHED ? sry[ix(g, r_, I)] : f.add(den0[ix(g, rm_, I)], den0[ix(g, r_, I)]);
+      in.dps = CACHED ? dpy[ix(g, r_, I)] : f.sub(psio[ix(g, r_, I)], psio[ix(g, rm_, I)]);
+      coefs(in);
+      predict_face<false, false>(f, in, hgrav, adt2, bdt2, k, o);
+    }
+    sry[ix(g, r, I)] = o.rho1;
+    uy_out[ix(g, r, I)] = o.u;
+    sya[ix(g, r, I - 1)] = o.a;
+    egy[ix(g, r, I)] = o.e;
+    qy[ix(g, r, I)] = o.q;
   }
   // walls: impermeable, no-slip; the wall faces' e grad psi_old (zero for a
   // Neumann psi_old, computed as the reference does)
