@@ -224,6 +224,16 @@ struct Fp64Int {
       d = f.sub(a, b);
     }
   }
+  // the same for operands far apart, both parts of a complex pair
+  __device__ __forceinline__ void caddsub(double2 a, double2 b, double2 &s, double2 &d) {
+    if (INT) {
+      intfp::addsub<false, true>(a.x, b.x, s.x, d.x, bad);
+      intfp::addsub<false, true>(a.y, b.y, s.y, d.y, bad);
+    } else {
+      s = f.cadd(a, b);
+      d = f.csub(a, b);
+    }
+  }
   __device__ __forceinline__ double mul(double a, double b) {
     return INT ? intfp::mul<false>(a, b, bad) : f.mul(a, b);
   }

@@ -884,8 +884,8 @@ __device__ __forceinline__ bool momflux_cell(const Fp64 &f, const MomIn &in, con
   return INT && q.bad != 0;
 }
 
-template <int STRESS, bool SCALED>
-__global__ void __launch_bounds__(BX *BY, 5)
+template <int STRESS, bool SCALED, bool INT>
+__global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
     k_momflux(Grid g, Metrics m, Phys ph0, const double *__restrict__ ux, const double *__restrict__ uy,
               const double *__restrict__ visux, const double *__restrict__ visuy, const double *__restrict__ mfx,
               const double *__restrict__ mfy, double *__restrict__ pxx, double *__restrict__ pyy,
@@ -934,7 +934,7 @@ __global__ void __launch_bounds__(BX *BY, 5)
   };
   MomIn in = load(r, rm, rp);
   MomOut o;
-  if (momflux_cell<true, SCALED>(f, in, ph, o)) {
+  if (momflux_cell<INT, SCALED>(f, in, ph, o)) {
     in = load(reread(r), reread(rm), reread(rp));
     momflux_cell<false, SCALED>(f, in, ph, o);
   }
@@ -1012,8 +1012,8 @@ __device__ __forceinline__ bool predict_face(const Fp64 &f, const PredIn &in, do
   return INT && n.bad != 0;
 }
 
-template <bool CACHED>
-__global__ void __launch_bounds__(BX *BY, 5)
+template <bool CACHED, bool INT>
+__global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
     k_predict_mf(Grid g, Metrics m, Phys ph0, const double *__restrict__ sc, int k, const double *__restrict__ ux,
                  const double *__restrict__ uy, double *__restrict__ ux_out, double *__restrict__ uy_out,
                  const double *__restrict__ pxx, const double *__restrict__ pyy, const double *__restrict__ pxy,
@@ -1044,20 +1044,22 @@ __global__ void __launch_bounds__(BX *BY, 5)
   // (y faces): e pa = (2 rho_ref pa) / (2 rho) - pa
   const double rpx = sc[sc_rpx(k)], pax = sc[sc_pax(k)];
   const double q4y = f.reg(g.q4y), hgrav = f.reg(ph.hgrav);
-  __shared__ double yb[11][BX * BY];
+  __shared__ double yb[INT ? 11 : 1][BX * BY];
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  async_copy(&yb[0][tid], uy + ix(g, r, I));
-  async_copy(&yb[1][tid], ifrcy + ix(g, r, I - 1));
-  async_copy(&yb[2][tid], pyx + ix(g, r, I));
-  async_copy(&yb[3][tid], pyx + ix(g, r, I - 1));
-  async_copy(&yb[4][tid], pyy + ix(g, r, I - 1));
-  async_copy(&yb[5][tid], pyy + ix(g, rm, I - 1));
-  async_copy(&yb[6][tid], den1 + ix(g, rm, I));
-  async_copy(&yb[7][tid], p + ix(g, rm, I));
-  if (k != 0) async_copy(&yb[8][tid], syb + ix(g, r, I - 1));
-  if (CACHED) {
-    async_copy(&yb[9][tid], sry + ix(g, r, I));
-    async_copy(&yb[10][tid], dpy + ix(g, r, I));
+  if (INT) {
+    async_copy(&yb[0][tid], uy + ix(g, r, I));
+    async_copy(&yb[1][tid], ifrcy + ix(g, r, I - 1));
+    async_copy(&yb[2][tid], pyx + ix(g, r, I));
+    async_copy(&yb[3][tid], pyx + ix(g, r, I - 1));
+    async_copy(&yb[4][tid], pyy + ix(g, r, I - 1));
+    async_copy(&yb[5][tid], pyy + ix(g, rm, I - 1));
+    async_copy(&yb[6][tid], den1 + ix(g, rm, I));
+    async_copy(&yb[7][tid], p + ix(g, rm, I));
+    if (k != 0) async_copy(&yb[8][tid], syb + ix(g, r, I - 1));
+    if (CACHED) {
+      async_copy(&yb[9][tid], sry + ix(g, r, I));
+      async_copy(&yb[10][tid], dpy + ix(g, r, I));
+    }
   }
   const double ps0 = CACHED && I != 1 && I != g.nx ? 0. : psio[ix(g, r, I)];
   // ---- ux at face I
@@ -1077,7 +1079,7 @@ __global__ void __launch_bounds__(BX *BY, 5)
       return in;
     };
     PredOut o;
-    if (predict_face<true, true>(f, load(r, rm, rp), hgrav, adt2, bdt2, k, o))
+    if (predict_face<INT, true>(f, load(r, rm, rp), hgrav, adt2, bdt2, k, o))
       predict_face<false, true>(f, load(reread(r), reread(rm), reread(rp)), hgrav, adt2, bdt2, k, o);
     srx[ix(g, r, I - 1)] = o.rho1;
     ux_out[ix(g, r, I - 1)] = o.u;
@@ -1091,31 +1093,36 @@ __global__ void __launch_bounds__(BX *BY, 5)
       in.cd = m.q4c[I], in.co = q4y, in.gp = sc[sc_gdt2y(k)], in.rp = sc[sc_rpy(k)], in.pa = sc[sc_pay(k)],
       in.pd = sc[sc_pdy(k)];
     };
-    async_wait();
-    PredIn in;
-    in.u0 = yb[0][tid], in.frc = yb[1][tid];
-    in.pd1 = yb[2][tid], in.pd0 = yb[3][tid];
-    in.po1 = yb[4][tid], in.po0 = yb[5][tid];
-    in.r1a = yb[6][tid], in.r1b = den1[ix(g, r, I)];
-    in.p0 = yb[7][tid], in.p1 = p[ix(g, r, I)];
-    in.sb = k != 0 ? yb[8][tid] : 0.;
-    in.rho0 = CACHED ? yb[9][tid] : f.add(den0[ix(g, rm, I)], den0[ix(g, r, I)]);  // 2 rho^k
-    in.dps = CACHED ? yb[10][tid] : f.sub(ps0, psio[ix(g, rm, I)]);
-    coefs(in);
-    PredOut o;
-    if (predict_face<true, false>(f, in, hgrav, adt2, bdt2, k, o)) {
-      const int r_ = reread(r), rm_ = reread(rm);
-      in.u0 = uy[ix(g, r_, I)];
-      in.frc = ifrcy[ix(g, r_, I - 1)];
-      in.pd1 = pyx[ix(g, r_, I)], in.pd0 = pyx[ix(g, r_, I - 1)];
-      in.po1 = pyy[ix(g, r_, I - 1)], in.po0 = pyy[ix(g, rm_, I - 1)];
-      in.r1a = den1[ix(g, rm_, I)], in.r1b = den1[ix(g, r_, I)];
-      in.p0 = p[ix(g, rm_, I)], in.p1 = p[ix(g, r_, I)];
-      in.sb = k != 0 ? syb[ix(g, r_, I - 1)] : 0.;
-      in.rho0 = CACHED ? sry[ix(g, r_, I)] : f.add(den0[ix(g, rm_, I)], den0[ix(g, r_, I)]);
-      in.dps = CACHED ? dpy[ix(g, r_, I)] : f.sub(psio[ix(g, r_, I)], psio[ix(g, rm_, I)]);
+    auto load = [&](int r, int rm) {
+      PredIn in;
+      in.u0 = uy[ix(g, r, I)], in.frc = ifrcy[ix(g, r, I - 1)];
+      in.pd1 = pyx[ix(g, r, I)], in.pd0 = pyx[ix(g, r, I - 1)];
+      in.po1 = pyy[ix(g, r, I - 1)], in.po0 = pyy[ix(g, rm, I - 1)];
+      in.r1a = den1[ix(g, rm, I)], in.r1b = den1[ix(g, r, I)];
+      in.p0 = p[ix(g, rm, I)], in.p1 = p[ix(g, r, I)];
+      in.sb = k != 0 ? syb[ix(g, r, I - 1)] : 0.;
+      in.rho0 = CACHED ? sry[ix(g, r, I)] : f.add(den0[ix(g, rm, I)], den0[ix(g, r, I)]);  // 2 rho^k
+      in.dps = CACHED ? dpy[ix(g, r, I)] : f.sub(psio[ix(g, r, I)], psio[ix(g, rm, I)]);
       coefs(in);
-      predict_face<false, false>(f, in, hgrav, adt2, bdt2, k, o);
+      return in;
+    };
+    PredOut o;
+    if (INT) {
+      async_wait();
+      PredIn in;
+      in.u0 = yb[0][tid], in.frc = yb[1][tid];
+      in.pd1 = yb[2][tid], in.pd0 = yb[3][tid];
+      in.po1 = yb[4][tid], in.po0 = yb[5][tid];
+      in.r1a = yb[6][tid], in.r1b = den1[ix(g, r, I)];
+      in.p0 = yb[7][tid], in.p1 = p[ix(g, r, I)];
+      in.sb = k != 0 ? yb[8][tid] : 0.;
+      in.rho0 = CACHED ? yb[9][tid] : f.add(den0[ix(g, rm, I)], den0[ix(g, r, I)]);  // 2 rho^k
+      in.dps = CACHED ? yb[10][tid] : f.sub(ps0, psio[ix(g, rm, I)]);
+      coefs(in);
+      if (predict_face<true, false>(f, in, hgrav, adt2, bdt2, k, o))
+        predict_face<false, false>(f, load(reread(r), reread(rm)), hgrav, adt2, bdt2, k, o);
+    } else {
+      predict_face<false, false>(f, load(r, rm), hgrav, adt2, bdt2, k, o);
     }
     sry[ix(g, r, I)] = o.rho1;
     uy_out[ix(g, r, I)] = o.u;
@@ -1166,53 +1173,108 @@ __global__ void __launch_bounds__(BX *BY, 5)
 // into the right-hand-side coefficients.
 // ---------------------------------------------------------------------------
 
-// Stockham FFT (radix 4, one radix-8 stage first when log2 M is odd) of W
-// rows of length M in shared memory.  Returns the buffer holding the result.
+// -i z (forward) or +i z (inverse)
+__device__ __forceinline__ double2 rot(double2 z, bool inverse) {
+  return inverse ? make_double2(-z.y, z.x) : make_double2(z.y, -z.x);
+}
+
+// One untwiddled radix-8 butterfly, xr[0], xr[q], .. xr[7 q] into yr[0..7];
+// returns whether an integer form gave up.
+//   X_2m = DFT4(v_q + v_q+4)_m, X_2m+1 = DFT4((v_q - v_q+4) W8^q)_m; the
+//   1/sqrt(2) of W8 and W8^3 rides in the odd half's last FMAs: 52 FP64
+//   operations for 8 points, where a radix-2 stage and a twiddled radix-4
+//   stage take 64 for the same three levels
+// INT: 24 of the 52, the sums and differences of the first level and of the
+// even half's second, run on the integer pipes.
+template <bool INT>
+__device__ __forceinline__ bool radix8(const Fp64 &f, const double2 *xr, double2 *yr, int q, double c8, bool inverse) {
+  Fp64Int<INT> n(f);
+  double2 a[4], b[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) n.caddsub(xr[i * q], xr[(i + 4) * q], a[i], b[i]);
+  // even outputs: DFT4 of a
+  double2 e0, e1, e2, e3;
+  n.caddsub(a[0], a[2], e0, e1);
+  n.caddsub(a[1], a[3], e2, e3);
+  const double2 re3 = rot(e3, inverse);
+  yr[0] = f.cadd(e0, e2);
+  yr[2] = f.cadd(e1, re3);
+  yr[4] = f.csub(e0, e2);
+  yr[6] = f.csub(e1, re3);
+  // odd outputs: t1 = b1 W8 = c8 P1, t2 = b2 W8^2 (a rotation), t3 = b3 W8^3 = c8 P3
+  const double2 P1 = inverse ? make_double2(f.sub(b[1].x, b[1].y), f.add(b[1].x, b[1].y))
+                             : make_double2(f.add(b[1].x, b[1].y), f.sub(b[1].y, b[1].x));
+  const double2 P3 = inverse ? make_double2(-f.add(b[3].x, b[3].y), f.sub(b[3].x, b[3].y))
+                             : make_double2(f.sub(b[3].y, b[3].x), -f.add(b[3].x, b[3].y));
+  const double2 t2 = rot(b[2], inverse);
+  const double2 A0 = f.cadd(b[0], t2), A1 = f.csub(b[0], t2);
+  const double2 E = f.cadd(P1, P3), D = f.csub(P1, P3);  // t1 + t3 = c8 E, t1 - t3 = c8 D
+  const double2 rD = rot(D, inverse);
+  yr[1] = make_double2(fma(c8, E.x, A0.x), fma(c8, E.y, A0.y));
+  yr[3] = make_double2(fma(c8, rD.x, A1.x), fma(c8, rD.y, A1.y));
+  yr[5] = make_double2(fma(-c8, E.x, A0.x), fma(-c8, E.y, A0.y));
+  yr[7] = make_double2(fma(-c8, rD.x, A1.x), fma(-c8, rD.y, A1.y));
+  return INT && n.bad != 0;
+}
+
+// One radix-4 butterfly, xr[0], xr[q], xr[2 q], xr[3 q] into yr[0], yr[s],
+// yr[2 s], yr[3 s], the inputs times 1, wm[e], wm[2 e], wm[3 e] (TWIDDLE);
+// returns whether an integer form gave up.
+//   a0 = v0 + w2 v2 and a2 = w1 v1 + w3 v3 with the products folded into
+//   FMAs, a1 = 2 v0 - a0 and a3 = 2 (w1 v1) - a2: 24 FP64 operations per
+//   butterfly instead of 28 (cmul, then add and subtract)
+// INT: the eight closing sums and differences and two products run on the
+// integer pipes (without twiddles, the eight opening ones).  2048 x 1024, one
+// launch, FP64 alone -> shared: k_poisson_fwd 70.5 -> 55.3 us, k_poisson_inv
+// 58.0 -> 46.3 us (56.9 and 46.6 with the two products left in FP64; 60.8 and
+// 51.5 at three blocks an SM, 60.8 and 46.4 at five).
+template <bool INT, bool TWIDDLE>
+__device__ __forceinline__ bool radix4(const Fp64 &f, const double2 *xr, double2 *yr, int q, int s,
+                                       const double2 *__restrict__ wm, int e, double two, bool inverse) {
+  Fp64Int<INT> n(f);
+  const double2 v0 = xr[0], v1 = xr[q], v2 = xr[2 * q], v3 = xr[3 * q];
+  if (TWIDDLE) {
+    const double2 w1 = wm[e], w2 = wm[2 * e], w3 = wm[3 * e];
+    const double2 a0 = make_double2(fma(w2.x, v2.x, fma(-w2.y, v2.y, v0.x)), fma(w2.x, v2.y, fma(w2.y, v2.x, v0.y)));
+    const double2 a1 = make_double2(fma(two, v0.x, -a0.x), fma(two, v0.y, -a0.y));
+    const double2 t1 = make_double2(fma(v1.x, w1.x, (1 ? n.mulz(-v1.y, w1.y) : f.mul(-v1.y, w1.y))), fma(v1.x, w1.y, (1 ? n.mulz(v1.y, w1.x) : f.mul(v1.y, w1.x))));
+    const double2 a2 = make_double2(fma(w3.x, v3.x, fma(-w3.y, v3.y, t1.x)), fma(w3.x, v3.y, fma(w3.y, v3.x, t1.y)));
+    const double2 a3 = make_double2(fma(two, t1.x, -a2.x), fma(two, t1.y, -a2.y));
+    const double2 r3 = rot(a3, inverse);
+    n.caddsub(a0, a2, yr[0], yr[2 * s]);
+    n.caddsub(a1, r3, yr[s], yr[3 * s]);
+  } else {
+    double2 a0, a1, a2, a3;
+    n.caddsub(v0, v2, a0, a1);
+    n.caddsub(v1, v3, a2, a3);
+    const double2 r3 = rot(a3, inverse);
+    yr[0] = f.cadd(a0, a2);
+    yr[s] = f.cadd(a1, r3);
+    yr[2 * s] = f.csub(a0, a2);
+    yr[3 * s] = f.csub(a1, r3);
+  }
+  return INT && n.bad != 0;
+}
+
+// Stockham FFT (radix 4, one radix-8 stage first when log2 M is odd) of the
+// first `cols` of W rows of length M in shared memory.  Returns the buffer
+// holding the result.
 // tw: the twiddle buffer, exp(-2 pi i m / 2M) for m = 0..M, then W_M^e for
 // e < M, then their conjugates (the inverse's): one load per twiddle.
-template <int W>
-__device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__restrict__ tw, bool inverse, const Fp64 &f) {
+template <int W, bool INT>
+__device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__restrict__ tw, bool inverse, const Fp64 &f,
+                             int cols) {
   const double two = f.reg(2.);
   const double2 *__restrict__ wm = tw + (M + 1) + (inverse ? M : 0);
   int Ns = 1;
-  if ((__ffs(M) - 1) & 1) {  // log2 M odd (M >= 8): an untwiddled radix-8 stage
-    // X_2m = DFT4(v_q + v_q+4)_m, X_2m+1 = DFT4((v_q - v_q+4) W8^q)_m; the
-    // 1/sqrt(2) of W8 and W8^3 rides in the odd half's last FMAs: 52 FP64
-    // operations for 8 points, where a radix-2 stage and a twiddled radix-4
-    // stage take 64 for the same three levels
+  if ((__ffs(M) - 1) & 1) {  // log2 M odd (M >= 8)
     const double c8 = f.reg(0.70710678118654752440);
     const int q8 = M >> 3;
-    for (int t = threadIdx.x; t < W * q8; t += blockDim.x) {
+    for (int t = threadIdx.x; t < cols * q8; t += blockDim.x) {
       const int c = t / q8, j = t - c * q8;
-      const double2 *xr = x + c * M;
+      const double2 *xr = x + c * M + j;
       double2 *yr = y + c * M + 8 * j;
-      double2 a[4], b[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double2 u = xr[j + q * q8], w = xr[j + (q + 4) * q8];
-        a[q] = f.cadd(u, w);
-        b[q] = f.csub(u, w);
-      }
-      // even outputs: DFT4 of a; -i (forward) or +i (inverse) rotations are sign flips
-      const double2 e0 = f.cadd(a[0], a[2]), e1 = f.csub(a[0], a[2]), e2 = f.cadd(a[1], a[3]), e3 = f.csub(a[1], a[3]);
-      const double2 re3 = inverse ? make_double2(-e3.y, e3.x) : make_double2(e3.y, -e3.x);
-      yr[0] = f.cadd(e0, e2);
-      yr[2] = f.cadd(e1, re3);
-      yr[4] = f.csub(e0, e2);
-      yr[6] = f.csub(e1, re3);
-      // odd outputs: t1 = b1 W8 = c8 P1, t2 = b2 W8^2 (a rotation), t3 = b3 W8^3 = c8 P3
-      const double2 P1 = inverse ? make_double2(f.sub(b[1].x, b[1].y), f.add(b[1].x, b[1].y))
-                                 : make_double2(f.add(b[1].x, b[1].y), f.sub(b[1].y, b[1].x));
-      const double2 P3 = inverse ? make_double2(-f.add(b[3].x, b[3].y), f.sub(b[3].x, b[3].y))
-                                 : make_double2(f.sub(b[3].y, b[3].x), -f.add(b[3].x, b[3].y));
-      const double2 t2 = inverse ? make_double2(-b[2].y, b[2].x) : make_double2(b[2].y, -b[2].x);
-      const double2 A0 = f.cadd(b[0], t2), A1 = f.csub(b[0], t2);
-      const double2 E = f.cadd(P1, P3), D = f.csub(P1, P3);  // t1 + t3 = c8 E, t1 - t3 = c8 D
-      const double2 rD = inverse ? make_double2(-D.y, D.x) : make_double2(D.y, -D.x);
-      yr[1] = make_double2(fma(c8, E.x, A0.x), fma(c8, E.y, A0.y));
-      yr[3] = make_double2(fma(c8, rD.x, A1.x), fma(c8, rD.y, A1.y));
-      yr[5] = make_double2(fma(-c8, E.x, A0.x), fma(-c8, E.y, A0.y));
-      yr[7] = make_double2(fma(-c8, rD.x, A1.x), fma(-c8, rD.y, A1.y));
+      if (radix8<INT>(f, xr, yr, q8, c8, inverse)) radix8<false>(f, xr, yr, q8, c8, inverse);
     }
     __syncthreads();
     double2 *tmp = x;
@@ -1223,37 +1285,18 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
   const int q4 = M >> 2;
   for (; Ns < M; Ns <<= 2) {
     const int step = M / (4 * Ns);
-    for (int t = threadIdx.x; t < W * q4; t += blockDim.x) {
+    for (int t = threadIdx.x; t < cols * q4; t += blockDim.x) {
       const int c = t / q4, j = t - c * q4;
-      const double2 *xr = x + c * M;
-      double2 *yr = y + c * M;
       const int kk = j & (Ns - 1);
-      const double2 v0 = xr[j], v1 = xr[j + q4], v2 = xr[j + 2 * q4], v3 = xr[j + 3 * q4];
-      double2 a0, a1, a2, a3;
+      const double2 *xr = x + c * M + j;
+      double2 *yr = y + c * M + ((j - kk) << 2) + kk;
       if (Ns > 1) {
-        // a0 = v0 + w2 v2 and a2 = w1 v1 + w3 v3 with the products folded into
-        // FMAs, a1 = 2 v0 - a0 and a3 = 2 (w1 v1) - a2: 24 FP64 operations per
-        // butterfly instead of 28 (cmul, then add and subtract)
-        const int e = kk * step;
-        const double2 w1 = wm[e], w2 = wm[2 * e], w3 = wm[3 * e];
-        a0 = make_double2(fma(w2.x, v2.x, fma(-w2.y, v2.y, v0.x)), fma(w2.x, v2.y, fma(w2.y, v2.x, v0.y)));
-        a1 = make_double2(fma(two, v0.x, -a0.x), fma(two, v0.y, -a0.y));
-        const double2 t1 = f.cmul(v1, w1);
-        a2 = make_double2(fma(w3.x, v3.x, fma(-w3.y, v3.y, t1.x)), fma(w3.x, v3.y, fma(w3.y, v3.x, t1.y)));
-        a3 = make_double2(fma(two, t1.x, -a2.x), fma(two, t1.y, -a2.y));
+        if (radix4<INT, true>(f, xr, yr, q4, Ns, wm, kk * step, two, inverse))
+          radix4<false, true>(f, xr, yr, q4, Ns, wm, kk * step, two, inverse);
       } else {
-        a0 = f.cadd(v0, v2);
-        a1 = f.csub(v0, v2);
-        a2 = f.cadd(v1, v3);
-        a3 = f.csub(v1, v3);
+        if (radix4<INT, false>(f, xr, yr, q4, Ns, wm, 0, two, inverse))
+          radix4<false, false>(f, xr, yr, q4, Ns, wm, 0, two, inverse);
       }
-      // -i a3 (forward) or +i a3 (inverse)
-      const double2 r3 = inverse ? make_double2(-a3.y, a3.x) : make_double2(a3.y, -a3.x);
-      const int d = ((j - kk) << 2) + kk;
-      yr[d] = f.cadd(a0, a2);
-      yr[d + Ns] = f.cadd(a1, r3);
-      yr[d + 2 * Ns] = f.csub(a0, a2);
-      yr[d + 3 * Ns] = f.csub(a1, r3);
     }
     __syncthreads();
     double2 *tmp = x;
@@ -1266,8 +1309,8 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
 // Q: the right-hand side from the predictor's face values q = pd u* + pa e
 // grad psi_old (ux, uy are qx, qy; egx, egy unused): 3 FP64 operations per
 // cell instead of 7
-template <int W, bool Q>
-__global__ void __launch_bounds__(256)
+template <int W, bool Q, bool INT>
+__global__ void __launch_bounds__(256, INT ? 4 : 1)
     k_poisson_fwd(Grid g, const double *__restrict__ sc, int k, const double *__restrict__ ux,
                   const double *__restrict__ uy, const double *__restrict__ egx, const double *__restrict__ egy,
                   const double2 *__restrict__ tw, double2 *__restrict__ spec) {
@@ -1304,7 +1347,7 @@ __global__ void __launch_bounds__(256)
     Ad[c * ny + r] = val;
   }
   __syncthreads();
-  double2 *Z = fft_rows<W>(A, B, M, tw, false, f);
+  double2 *Z = fft_rows<W, INT>(A, B, M, tw, false, f, min(W, g.nx + 1 - I0));
   // the packed transform z_m, m < M; k_poisson_tdm does the real-to-complex
   // split (there the FP64 pipe has room)
   const int M1 = M + 1;
@@ -1316,8 +1359,8 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-template <int W>
-__global__ void __launch_bounds__(256)
+template <int W, bool INT>
+__global__ void __launch_bounds__(256, INT ? 4 : 1)
     k_poisson_inv(Grid g, const double2 *__restrict__ tw, const double2 *__restrict__ spec, double *__restrict__ psi) {
   pdl_entry();
   spec += (size_t)blockIdx.z * (g.css);
@@ -1334,7 +1377,7 @@ __global__ void __launch_bounds__(256)
     A[c * M + mm] = I <= g.nx ? spec[(size_t)(I - 1) * M1 + mm] : make_double2(0., 0.);
   }
   __syncthreads();
-  const double2 *zr = fft_rows<W>(A, B, M, tw, true, f);
+  const double2 *zr = fft_rows<W, INT>(A, B, M, tw, true, f, min(W, g.nx + 1 - I0));
   const double *xd = reinterpret_cast<const double *>(zr);
   for (int t = threadIdx.x; t < W * ny; t += blockDim.x) {
     const int c = t % W, r = t / W;
@@ -2227,6 +2270,17 @@ int tdm_modes_per_block(const Tiles &t, int nx) {
   const int mb = t.tdm_mb > 0 ? t.tdm_mb : poisson_tdm_modes(nx);
   return mb * G > 4 ? 4 / G : mb;  // at most 512 threads a block
 }
+// Whether the stencils, and the transforms, of a launch over these cells share
+// their arithmetic with the integer pipes: only where enough warps are in
+// flight to keep the FP64 unit busy; below that an integer form's longer
+// chain of instructions sets a warp's time.  Measured, us a launch FP64 alone
+// -> shared: 500 x 128 k_momflux 6.9 -> 7.1, k_predict_mf 9.1 -> 9.6,
+// k_poisson_fwd 7.0 -> 7.5; 509 x 256 10.3 -> 9.2, 13.8 -> 13.2, 9.2 -> 10.7;
+// 512 x 512 16.8 -> 13.6, 21.2 -> 19.2, 13.3 -> 13.7 (k_poisson_inv 12.3 ->
+// 11.6); 1000 x 512 27.1 -> 20.4, 36.4 -> 30.2, 20.5 -> 18.4.
+long cells(const Grid &g) { return (long)g.nx * g.ny * g.nc; }
+bool integer_stencils(const Grid &g) { return cells(g) >= 3L << 15; }
+bool integer_transforms(const Grid &g) { return cells(g) >= 1L << 18; }
 int tdm_warps_for(int nx, int ny, int nc) {
   const long systems = 4L * (ny / 4 + 1) * nc;
   int G = 1;
@@ -2234,32 +2288,23 @@ int tdm_warps_for(int nx, int ny, int nc) {
   return G;
 }
 
+template <class... K>
+cudaError_t allow_smem(int bytes, K... kernels) {
+  cudaError_t e = cudaSuccess;
+  ((e = e == cudaSuccess ? cudaFuncSetAttribute(kernels, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : e), ...);
+  return e;
+}
+template <int... W>
+cudaError_t configure_fft(int bytes) {
+  return allow_smem(bytes, k_poisson_fwd<W, false, false>..., k_poisson_fwd<W, true, false>...,
+                    k_poisson_fwd<W, false, true>..., k_poisson_fwd<W, true, true>..., k_poisson_inv<W, false>...,
+                    k_poisson_inv<W, true>...);
+}
+
 cudaError_t configure_kernels() {
   cudaError_t e;
   const int big = 227 * 1024;
-  e = cudaFuncSetAttribute(k_poisson_fwd<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_fwd<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_fwd<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_fwd<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_fwd<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_fwd<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_inv<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_inv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_inv<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_fwd<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_fwd<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_inv<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  e = configure_fft<1, 2, 4, 8>(big);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_poisson_tdm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTdmSmemMax);
   if (e != cudaSuccess) return e;
@@ -2396,9 +2441,15 @@ void launch_stress(cudaStream_t s, const Grid &g, const Metrics &m, const Bufs &
 void launch_momflux(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const Bufs &b,
                     const double *ux, const double *uy, int stress, bool scaled) {
   const dim3 gr = tile_grid(b.tiles, TK_MOMFLUX, g.nx + 1, g.ny, g.nc), bl = tile_block(b.tiles, TK_MOMFLUX);
-  auto k = stress == 2 ? k_momflux<2, false>
-                       : (scaled ? (stress == 1 ? k_momflux<1, true> : k_momflux<0, true>)
-                                 : (stress == 1 ? k_momflux<1, false> : k_momflux<0, false>));
+  // the unscaled forms (full-sync steps) run on the FP64 unit alone
+  auto k = k_momflux<2, false, false>;
+  if (stress != 2 && !scaled) k = stress == 1 ? k_momflux<1, false, false> : k_momflux<0, false, false>;
+  if (stress != 2 && scaled) {
+    if (integer_stencils(g))
+      k = stress == 1 ? k_momflux<1, true, true> : k_momflux<0, true, true>;
+    else
+      k = stress == 1 ? k_momflux<1, true, false> : k_momflux<0, true, false>;
+  }
   launch_pdl(k, gr, bl, 0, s, g, m, ph, ux, uy, b.visux, b.visuy, b.mfluxx, b.mfluxy, b.pxx, b.pyy, b.pxy, b.pyx,
              b.txx, b.txy, b.tyy);
 }
@@ -2408,7 +2459,8 @@ void launch_predict_mf(cudaStream_t s, const Grid &g, const Metrics &m, const Ph
                        const double *den0, const double *den1, const double *psi_old, double *srcux_a,
                        const double *srcux_b, double *srcuy_a, const double *srcuy_b, const double *ifx,
                        const double *ify, bool cached) {
-  auto kern = cached ? k_predict_mf<true> : k_predict_mf<false>;
+  auto kern = integer_stencils(g) ? (cached ? k_predict_mf<true, true> : k_predict_mf<false, true>)
+                               : (cached ? k_predict_mf<true, false> : k_predict_mf<false, false>);
   launch_pdl(kern, tile_grid(b.tiles, TK_PREDICT, g.nx, g.ny, g.nc), tile_block(b.tiles, TK_PREDICT), 0, s, g, m, ph,
              sc, k, ux, uy, ux_out, uy_out, b.pxx, b.pyy, b.pxy, b.pyx, b.p, ifx, ify, den0, den1, psi_old, srcux_a,
              srcux_b, srcuy_a, srcuy_b, b.egx, b.egy, b.coltab, b.qx, b.qy, b.rhofx, b.rhofy, b.dpsix, b.dpsiy);
@@ -2428,8 +2480,8 @@ template <int W, bool Q>
 void poisson_fwd_w(cudaStream_t s, const Grid &g, const Bufs &b, const double *sc, int k, const double *ux,
                    const double *uy) {
   const int nb = (g.nx + W - 1) / W;
-  launch_pdl(k_poisson_fwd<W, Q>, dim3(nb, 1, g.nc), 256, poisson_fft_smem(g.ny, W), s, g, sc, k, ux, uy, b.egx,
-             b.egy, b.twiddle, b.spec);
+  launch_pdl(integer_transforms(g) ? k_poisson_fwd<W, Q, true> : k_poisson_fwd<W, Q, false>, dim3(nb, 1, g.nc), 256,
+             poisson_fft_smem(g.ny, W), s, g, sc, k, ux, uy, b.egx, b.egy, b.twiddle, b.spec);
 }
 
 template <bool Q>
@@ -2484,7 +2536,8 @@ void launch_poisson_tdm(cudaStream_t s, const Grid &g, const Bufs &b) {
 template <int W>
 void poisson_inv_w(cudaStream_t s, const Grid &g, const Bufs &b, double *psi_new) {
   const int nb = (g.nx + W - 1) / W;
-  launch_pdl(k_poisson_inv<W>, dim3(nb, 1, g.nc), 256, poisson_fft_smem(g.ny, W), s, g, b.twiddle, b.spec, psi_new);
+  launch_pdl(integer_transforms(g) ? k_poisson_inv<W, true> : k_poisson_inv<W, false>, dim3(nb, 1, g.nc), 256,
+             poisson_fft_smem(g.ny, W), s, g, b.twiddle, b.spec, psi_new);
 }
 
 void launch_poisson_inv(cudaStream_t s, const Grid &g, const Bufs &b, double *psi_new) {

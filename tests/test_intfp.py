@@ -21,6 +21,7 @@ SBFS_IF void form(int op, double a, double b, double &s, double &t, u32 &bad) {
     case 4: addsub<false>(a, b, s, t, bad); break;
     case 5: s = addp(a, b, bad); break;
     case 6: s = mul<true>(a, b, bad); break;
+    case 8: addsub<false, true>(a, b, s, t, bad); break;
     default: s = mul<false>(a, b, bad);
   }
 }
@@ -55,7 +56,7 @@ extern "C" int run(int op, int n, const double *a, const double *b, double *s, d
   return e;
 }
 """
-OPS = ["add_zero", "add", "sub_zero", "addsub_zero", "addsub", "addp", "mul_zero", "mul"]
+OPS = ["add_zero", "add", "sub_zero", "addsub_zero", "addsub", "addp", "mul_zero", "mul", "addsub_sticky"]
 
 
 def _build(tmp, device):
@@ -124,6 +125,9 @@ def _check(lib, op):
     plain = (np.abs(np.log2(np.abs(a / np.where(b == 0, 1, b)))) < 10) & (np.abs(want) > 1e-6 * np.abs(a)) & \
         (np.abs(diff) > 1e-6 * np.abs(a)) & (np.abs(a) > 1e-30) & (np.abs(a) < 1e30)
     assert plain.sum() > n / 4 and ok[plain].all()
+    if op.endswith("_sticky"):  # never given up for lost bits
+        plain = (np.abs(a) > 1e-30) & (np.abs(a) < 1e30) & (np.abs(b) > 0) & (np.abs(b) < 1e-4 * np.abs(a))
+        assert plain.sum() > n / 16 and ok[plain].all()
     if op.endswith("_zero"):
         assert ok[(a == 0) & (b == 0) & ~np.signbit(a) & ~np.signbit(b)].all()
 
