@@ -1884,6 +1884,7 @@ __global__ void __launch_bounds__(kDtFinThreads)
   __shared__ double wmin[kDtFinThreads / 32];
   __shared__ int wbad[kDtFinThreads / 32];
   __shared__ bool last;
+  __shared__ double dt_sh;
   const double small = 1.e-8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // dt_adv = coef * min(1, min_i hx_i / (max|ux|_i + small), hy / (max|uy| + small))
@@ -1928,38 +1929,47 @@ __global__ void __launch_bounds__(kDtFinThreads)
     dt *= coef_adv;
     dt = fmin(dt, dt_fixed);
     if (by >= kInfBits) atomicOr(status, 1);
-    // per-substage scalars; RK3 coefficients of src/runge_kutta.c:8-15
-    const double al[3] = {32. / 60., 25. / 60., 45. / 60.};
-    const double be[3] = {0. / 60., -17. / 60., -25. / 60.};
     sc[0] = dt;
-    for (int k = 0; k < 3; ++k) {
-      const int ko = (k + 2) % 3;
-      const double dtold = (al[ko] + be[ko]) * dt, dtnew = (al[k] + be[k]) * dt;
-      sc[sc_adt(k)] = al[k] * dt;
-      sc[sc_bdt(k)] = be[k] * dt;
-      sc[sc_gdt(k)] = (al[k] + be[k]) * dt;
-      sc[sc_adt2(k)] = 2. * (al[k] * dt);
-      sc[sc_bdt2(k)] = 2. * (be[k] * dt);
-      sc[sc_gdt2(k)] = 2. * ((al[k] + be[k]) * dt);
-      sc[sc_dtold(k)] = dtold;
-      sc[sc_dtnew(k)] = dtnew;
-      const double cdiv = ph.refden / dtnew * (0.5 / g.ny);
-      const double cadd = -(dtold / dtnew) * (0.5 / g.ny);
-      sc[sc_pdx(k)] = cdiv * g.idx;
-      sc[sc_pdy(k)] = cdiv * g.ihy;
-      sc[sc_pax(k)] = cadd * (g.idx * g.idx);
-      sc[sc_pay(k)] = cadd * (g.ihy * g.ihy);
-      sc[sc_cnew(k)] = dtnew * ph.irefden;
-      sc[sc_cold(k)] = -dtold * ph.irefden;
-      sc[sc_cnewy(k)] = sc[sc_cnew(k)] * g.ihy;
-      sc[sc_coldy(k)] = sc[sc_cold(k)] * g.ihy;
-      sc[sc_gdt2y(k)] = sc[sc_gdt2(k)] * g.ihy;
-      sc[sc_coldyp(k)] = sc[sc_coldy(k)] / sc[sc_pay(k)];
-      sc[sc_rpx(k)] = ph.rref2 * sc[sc_pax(k)];
-      sc[sc_rpy(k)] = ph.rref2 * sc[sc_pay(k)];
-    }
+    dt_sh = dt;
   }
   __syncthreads();
+  // per-substage scalars, one substage a lane (an FP64 instruction takes its
+  // warp's slot once for the three); RK3 coefficients of src/runge_kutta.c:8-15
+  if (tid < 3) {
+    const double dt = dt_sh;
+    const int k = tid, ko = (k + 2) % 3;
+    const double al[3] = {32. / 60., 25. / 60., 45. / 60.};
+    const double be[3] = {0. / 60., -17. / 60., -25. / 60.};
+    const double abo = ko == 0 ? al[0] + be[0] : (ko == 1 ? al[1] + be[1] : al[2] + be[2]);
+    const double ab = k == 0 ? al[0] + be[0] : (k == 1 ? al[1] + be[1] : al[2] + be[2]);
+    const double a = k == 0 ? al[0] : (k == 1 ? al[1] : al[2]), b = k == 0 ? be[0] : (k == 1 ? be[1] : be[2]);
+    const double dtold = abo * dt, dtnew = ab * dt;
+    sc[sc_adt(k)] = a * dt;
+    sc[sc_bdt(k)] = b * dt;
+    sc[sc_gdt(k)] = dtnew;
+    sc[sc_adt2(k)] = 2. * (a * dt);
+    sc[sc_bdt2(k)] = 2. * (b * dt);
+    const double gdt2 = 2. * dtnew;
+    sc[sc_gdt2(k)] = gdt2;
+    sc[sc_dtold(k)] = dtold;
+    sc[sc_dtnew(k)] = dtnew;
+    const double cdiv = ph.refden / dtnew * (0.5 / g.ny);
+    const double cadd = -(dtold / dtnew) * (0.5 / g.ny);
+    const double pax = cadd * (g.idx * g.idx), pay = cadd * (g.ihy * g.ihy);
+    const double cnew = dtnew * ph.irefden, cold = -dtold * ph.irefden, coldy = cold * g.ihy;
+    sc[sc_pdx(k)] = cdiv * g.idx;
+    sc[sc_pdy(k)] = cdiv * g.ihy;
+    sc[sc_pax(k)] = pax;
+    sc[sc_pay(k)] = pay;
+    sc[sc_cnew(k)] = cnew;
+    sc[sc_cold(k)] = cold;
+    sc[sc_cnewy(k)] = cnew * g.ihy;
+    sc[sc_coldy(k)] = coldy;
+    sc[sc_gdt2y(k)] = gdt2 * g.ihy;
+    sc[sc_coldyp(k)] = coldy / pay;
+    sc[sc_rpx(k)] = ph.rref2 * pax;
+    sc[sc_rpy(k)] = ph.rref2 * pay;
+  }
   // reset the scratch for the next launch
   for (int t = tid; t <= g.nx + 5; t += kDtFinThreads) acc[t] = 0ULL;
 }
@@ -2281,6 +2291,16 @@ int tdm_modes_per_block(const Tiles &t, int nx) {
 long cells(const Grid &g) { return (long)g.nx * g.ny * g.nc; }
 bool integer_stencils(const Grid &g) { return cells(g) >= 3L << 15; }
 bool integer_transforms(const Grid &g) { return cells(g) >= 1L << 18; }
+// default pairs per block: as many as shared memory and 512 threads take, but
+// one block a pair while the pairs are too few to give every SM that many
+// (its warps share one FP64 unit a scheduler: 64 x 64 k_poisson_tdm 10.8 ->
+// 7.8 us, 256 x 128 15.7 -> 11.9 us)
+int tdm_modes_for(int nx, int ny, int nc, int G) {
+  const long pairs = (long)(ny / 4 + 1) * nc;
+  int mb = std::min(poisson_tdm_modes(nx), 4 / G);
+  while (mb > 1 && pairs < 152L * mb) mb >>= 1;
+  return mb;
+}
 int tdm_warps_for(int nx, int ny, int nc) {
   const long systems = 4L * (ny / 4 + 1) * nc;
   int G = 1;

@@ -217,6 +217,7 @@ int poisson_tdm_modes(int nx);
 int tdm_chunk(int nx, int G);
 int tdm_group_index(int G);  // 1, 2, 4 -> 0, 1, 2
 int tdm_warps_for(int nx, int ny, int nc);
+int tdm_modes_for(int nx, int ny, int nc, int G);
 int tdm_modes_per_block(const Tiles &t, int nx);
 // the tridiagonal solves run as k_poisson_tdm_cl (switch g_tdm_cluster, tile choice tdm_cl, tdm_g = 4)
 extern int g_tdm_cluster;
