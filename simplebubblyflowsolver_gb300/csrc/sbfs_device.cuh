@@ -224,15 +224,18 @@ struct Fp64Int {
       d = f.sub(a, b);
     }
   }
-  // the same for operands far apart, both parts of a complex pair
-  __device__ __forceinline__ void caddsub(double2 a, double2 b, double2 &s, double2 &d) {
+  // the same for operands far apart
+  __device__ __forceinline__ void addsubs(double a, double b, double &s, double &d) {
     if (INT) {
-      intfp::addsub<false, true>(a.x, b.x, s.x, d.x, bad);
-      intfp::addsub<false, true>(a.y, b.y, s.y, d.y, bad);
+      intfp::addsub<false, true>(a, b, s, d, bad);
     } else {
-      s = f.cadd(a, b);
-      d = f.csub(a, b);
+      s = f.add(a, b);
+      d = f.sub(a, b);
     }
+  }
+  __device__ __forceinline__ void caddsub(double2 a, double2 b, double2 &s, double2 &d) {
+    addsubs(a.x, b.x, s.x, d.x);
+    addsubs(a.y, b.y, s.y, d.y);
   }
   __device__ __forceinline__ double mul(double a, double b) {
     return INT ? intfp::mul<false>(a, b, bad) : f.mul(a, b);

@@ -1391,6 +1391,104 @@ __global__ void __launch_bounds__(256, INT ? 4 : 1)
   }
 }
 
+// Split of the packed transform of a wavenumber pair (real-to-complex, times
+// 2): X_p = E + w^p O and X_{M-p} = conj E + w^{M-p} conj O with E = z_p +
+// conj z_{M-p} and O = -i (z_p - conj z_{M-p}) (the pair's E and O with the
+// signs of their imaginary parts flipped), products in FMAs.  Returns whether
+// an integer form gave up (INT: the four sums and differences).
+template <bool INT>
+__device__ __forceinline__ bool split_pair(const Fp64 &f, double2 zm, double2 zr, double2 wa, double2 wb, double2 &xa,
+                                           double2 &xb) {
+  Fp64Int<INT> n(f);
+  double2 E, O;
+  n.addsubs(zr.x, zm.x, E.x, O.y);
+  n.addsubs(zm.y, zr.y, O.x, E.y);
+  xa = make_double2(fma(wa.x, O.x, fma(-wa.y, O.y, E.x)), fma(wa.x, O.y, fma(wa.y, O.x, E.y)));
+  xb = make_double2(fma(wb.x, O.x, fma(wb.y, O.y, E.x)), fma(wb.y, O.x, fma(-wb.x, O.y, -E.y)));
+  return INT && n.bad != 0;
+}
+
+// The way back, into the packed input of the inverse transform: z_p = E + i D
+// conj w^p and z_{M-p} = conj E - i conj D conj w^{M-p}, with E = X_p + conj
+// X_{M-p}, D = X_p - conj X_{M-p}; products in FMAs
+template <bool INT>
+__device__ __forceinline__ bool merge_pair(const Fp64 &f, double2 Xa, double2 Xb, double2 wa, double2 wb, double2 &za,
+                                           double2 &zb) {
+  Fp64Int<INT> n(f);
+  double2 E, D;
+  n.addsubs(Xa.x, Xb.x, E.x, D.x);
+  n.addsubs(Xa.y, Xb.y, D.y, E.y);
+  za = make_double2(fma(D.x, wa.y, fma(-D.y, wa.x, E.x)), fma(D.y, wa.y, fma(D.x, wa.x, E.y)));
+  zb = make_double2(fma(-D.y, wb.x, fma(-D.x, wb.y, E.x)), fma(D.y, wb.y, fma(-D.x, wb.x, -E.y)));
+  return INT && n.bad != 0;
+}
+
+// One lane's chunk of a system, rows x[0 .. L), factors f[k lanes].  AHEAD:
+// the factors of the next kAhead rows are loaded while those of the present
+// ones are used, since a block's shared memory leaves room for one to three
+// warps a scheduler on large grids, which otherwise wait for them; on short
+// chunks (64 x 64: two rows) its tests cost more than the wait.  One launch
+// of k_poisson_tdm, with the split's sums on the integer pipes: 2048 x 1024
+// 61.7 -> 52.1 us, 4096 x 2048 472 -> 370 us (one warp a scheduler; 326 us
+// with four rows of the split's loads in flight as well).
+constexpr int kAhead = 8;
+template <bool AHEAD, int STEP, class Load, class Use>
+__device__ __forceinline__ void sweep(int L, Load load, Use use) {
+  auto row = [L](int k) { return STEP > 0 ? k : L - 1 - k; };
+  if (!AHEAD) {
+#pragma unroll 8
+    for (int k = 0; k < L; ++k) use(row(k), load(row(k)));
+    return;
+  }
+  decltype(load(0)) c[kAhead], n[kAhead];
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u)
+    if (u < L) c[u] = load(row(u));
+  for (int k0 = 0; k0 < L; k0 += kAhead) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (k0 + kAhead + u < L) n[u] = load(row(k0 + kAhead + u));
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (k0 + u < L) use(row(k0 + u), c[u]);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) c[u] = n[u];
+  }
+}
+// forward from a zero carry, y_k = w_k r_k - v_k y_{k-1}; returns the last y
+template <bool AHEAD>
+__device__ __forceinline__ double tdm_forward(const Fp64 &f64, const double4_32a *__restrict__ f, size_t lanes, int L,
+                                              double *x) {
+  double t = 0.;
+  sweep<AHEAD, 1>(
+      L, [&](int k) { return make_double2(f[k * lanes].x, f[k * lanes].y); },
+      [&](int k, double2 c) {
+        t = fma(-c.y, t, f64.mul(c.x, x[k]));
+        x[k] = t;
+      });
+  return t;
+}
+// the forward solution's fix-up by P_k carry and the backward sweep from a
+// zero carry, x_k = y_k - v_k x_{k+1}; returns the first x
+template <bool AHEAD>
+__device__ __forceinline__ double tdm_backward(const double4_32a *__restrict__ f, size_t lanes, int L, double carry,
+                                               double *x) {
+  double u = 0.;
+  sweep<AHEAD, -1>(
+      L, [&](int k) { return make_double2(f[k * lanes].y, f[k * lanes].z); },
+      [&](int k, double2 c) {
+        u = fma(-c.x, u, fma(c.y, carry, x[k]));
+        x[k] = u;
+      });
+  return u;
+}
+// the backward solution's fix-up by Q_k next
+template <bool AHEAD>
+__device__ __forceinline__ void tdm_fix(const double4_32a *__restrict__ f, size_t lanes, int L, double next, double *x) {
+  sweep<AHEAD, 1>(
+      L, [&](int k) { return f[k * lanes].w; }, [&](int k, double q) { x[k] = fma(q, next, x[k]); });
+}
+
 // Tridiagonal solves along x, one per real system (y wavenumber m, real or
 // imaginary part), one warp per system.  The pivots of the constant operator
 // are precomputed, so the Thomas forward sweep is the first-order linear
@@ -1407,7 +1505,7 @@ __global__ void __launch_bounds__(256, INT ? 4 : 1)
 // Staging: per system a planar array with an odd lane stride S, in shared
 // memory; when four systems of nx rows exceed it (nx above about 6900), in
 // this block's slab of the global buffer stage (L2-resident, same arithmetic).
-template <bool kGlobalStage>
+template <bool kGlobalStage, bool INT>
 __global__ void __launch_bounds__(512)
     k_poisson_tdm(Grid g, int PB, int G, int L, int S, const double4_32a *__restrict__ fac,
                   const double2 *__restrict__ tw, double2 *__restrict__ spec, double *__restrict__ stage) {
@@ -1426,26 +1524,35 @@ __global__ void __launch_bounds__(512)
   // ---- load the packed transform of both wavenumbers of each pair, split
   // it (real-to-complex, times 2: X_m = (z_m + conj z_{M-m}) + w^m (-i)(z_m -
   // conj z_{M-m})) into four planar systems: X_p re, im, X_{M-p} re, im
-  for (int t = threadIdx.x; t < lanes * L * np; t += blockDim.x) {
-    const int i = t / np, q = t - i * np;
-    const int p = p0 + q;
-    const int at = (i / L) * S + (i % L);
-    double2 xa = make_double2(0., 0.), xb = make_double2(0., 0.);
-    if (i < nx) {
-      const double2 zm = sp[(size_t)i * M1 + p];
-      const double2 zr = sp[(size_t)i * M1 + (p == 0 ? 0 : M - p)];
-      const double2 E = make_double2(f64.add(zm.x, zr.x), f64.sub(zm.y, zr.y));
-      const double2 O = make_double2(f64.add(zm.y, zr.y), f64.sub(zr.x, zm.x));  // -i (zm - conj zr)
-      // X_p = E + w^p O; X_{M-p} = conj E + w^{M-p} conj O (the pair's E and O
-      // with the signs of their imaginary parts flipped), products in FMAs
-      const double2 wa = tw[p], wb = tw[M - p];
-      xa = make_double2(fma(wa.x, O.x, fma(-wa.y, O.y, E.x)), fma(wa.x, O.y, fma(wa.y, O.x, E.y)));
-      xb = make_double2(fma(wb.x, O.x, fma(wb.y, O.y, E.x)), fma(wb.y, O.x, fma(-wb.x, O.y, -E.y)));
+  // (kBatch rows' loads in flight: the stores to sm keep the compiler from
+  // moving the next rows' loads above them)
+  constexpr int kBatch = INT ? 4 : 1;
+  const int rows = lanes * L * np;
+  for (int t0 = threadIdx.x; t0 < rows; t0 += kBatch * blockDim.x) {
+    double2 zm[kBatch], zr[kBatch];
+#pragma unroll
+    for (int v = 0; v < kBatch; ++v) {
+      const int t = t0 + v * blockDim.x, i = t / np, p = p0 + (t - i * np);
+      if (t < rows && i < nx) {
+        zm[v] = sp[(size_t)i * M1 + p];
+        zr[v] = sp[(size_t)i * M1 + (p == 0 ? 0 : M - p)];
+      }
     }
-    sm[(4 * q) * sys_len + at] = xa.x;
-    sm[(4 * q + 1) * sys_len + at] = xa.y;
-    sm[(4 * q + 2) * sys_len + at] = xb.x;
-    sm[(4 * q + 3) * sys_len + at] = xb.y;
+#pragma unroll
+    for (int v = 0; v < kBatch; ++v) {
+      const int t = t0 + v * blockDim.x, i = t / np, q = t - i * np, p = p0 + q;
+      if (t >= rows) break;
+      double2 xa = make_double2(0., 0.), xb = make_double2(0., 0.);
+      if (i < nx) {
+        const double2 wa = tw[p], wb = tw[M - p];
+        if (split_pair<INT>(f64, zm[v], zr[v], wa, wb, xa, xb)) split_pair<false>(f64, zm[v], zr[v], wa, wb, xa, xb);
+      }
+      double *o = sm + (size_t)(4 * q) * sys_len + (i / L) * S + (i % L);
+      o[0] = xa.x;
+      o[sys_len] = xa.y;
+      o[2 * sys_len] = xb.x;
+      o[3 * sys_len] = xb.y;
+    }
   }
   __syncthreads();
   // warp -> system (4 per pair) and its part sub of G; chunk j of the
@@ -1460,14 +1567,7 @@ __global__ void __launch_bounds__(512)
   double T = 0., B = 0.;
   if (act) {
     // forward, local from a zero carry
-    double t = 0.;
-#pragma unroll 8
-    for (int k = 0; k < L; ++k) {
-      const double4_32a c = f[(size_t)k * lanes];
-      t = fma(-c.y, t, f64.mul(c.x, x[k]));
-      x[k] = t;
-    }
-    T = t;
+    T = tdm_forward<INT>(f64, f, lanes, L, x);
     B = f[(size_t)(L - 1) * lanes].z;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -1495,15 +1595,7 @@ __global__ void __launch_bounds__(512)
     const double Tu = __shfl_up_sync(0xffffffffu, T, 1), Bu = __shfl_up_sync(0xffffffffu, B, 1);
     const double carry = lane == 0 ? Cin : fma(Bu, Cin, Tu);
     // fix up the forward solution, then the backward sweep from a zero carry
-    double u = 0.;
-#pragma unroll 8
-    for (int k = L - 1; k >= 0; --k) {
-      const double4_32a c = f[(size_t)k * lanes];
-      const double y = fma(c.z, carry, x[k]);
-      u = fma(-c.y, u, y);
-      x[k] = u;
-    }
-    Sx = u;
+    Sx = tdm_backward<INT>(f, lanes, L, carry, x);
     Cc = f[0].w;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -1532,8 +1624,7 @@ __global__ void __launch_bounds__(512)
   if (act) {
     const double Sd = __shfl_down_sync(0xffffffffu, Sx, 1), Cd = __shfl_down_sync(0xffffffffu, Cc, 1);
     const double next = lane == 31 ? Din : fma(Cd, Din, Sd);
-#pragma unroll 8
-    for (int k = 0; k < L; ++k) x[k] = fma(f[(size_t)k * lanes].w, next, x[k]);
+    tdm_fix<INT>(f, lanes, L, next, x);
     if (gauge) {
       for (int k = 0; k < L; ++k) acc += (j * L + k < nx) ? x[k] : 0.;
 #pragma unroll
@@ -1562,18 +1653,11 @@ __global__ void __launch_bounds__(512)
     const int at = (i / L) * S + (i % L);
     const double2 Xa = make_double2(sm[(4 * q) * sys_len + at], sm[(4 * q + 1) * sys_len + at]);
     const double2 Xb = make_double2(sm[(4 * q + 2) * sys_len + at], sm[(4 * q + 3) * sys_len + at]);
-    // z_p = E + i D conj w^p and z_{M-p} = conj E - i conj D conj w^{M-p}, with
-    // E = X_p + conj X_{M-p}, D = X_p - conj X_{M-p}; products in FMAs
-    const double2 E = make_double2(f64.add(Xa.x, Xb.x), f64.sub(Xa.y, Xb.y));
-    const double2 D = make_double2(f64.sub(Xa.x, Xb.x), f64.add(Xa.y, Xb.y));
-    const double2 wa = tw[p];
-    sp[(size_t)i * M1 + p] =
-        make_double2(fma(D.x, wa.y, fma(-D.y, wa.x, E.x)), fma(D.y, wa.y, fma(D.x, wa.x, E.y)));
-    if (p != 0 && 2 * p != M) {
-      const double2 wb = tw[M - p];
-      sp[(size_t)i * M1 + (M - p)] =
-          make_double2(fma(-D.y, wb.x, fma(-D.x, wb.y, E.x)), fma(D.y, wb.y, fma(-D.x, wb.x, -E.y)));
-    }
+    const double2 wa = tw[p], wb = tw[M - p];
+    double2 za, zb;
+    if (merge_pair<INT>(f64, Xa, Xb, wa, wb, za, zb)) merge_pair<false>(f64, Xa, Xb, wa, wb, za, zb);
+    sp[(size_t)i * M1 + p] = za;
+    if (p != 0 && 2 * p != M) sp[(size_t)i * M1 + (M - p)] = zb;
   }
 }
 
@@ -1588,6 +1672,7 @@ __global__ void __launch_bounds__(512)
 // the order k_poisson_tdm<false> combines its warps' at G = 4, so both give
 // the same bits.  L = tdm_chunk(nx, 4), S = L | 1; fac is the G = 4 table.
 constexpr int kTdmCluster = 4;
+template <bool INT>
 __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
     k_poisson_tdm_cl(Grid g, int L, int S, const double4_32a *__restrict__ fac, const double2 *__restrict__ tw,
                      double2 *__restrict__ spec) {
@@ -1612,11 +1697,8 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
     if (i < nx) {
       const double2 zm = sp[(size_t)i * M1 + p];
       const double2 zr = sp[(size_t)i * M1 + (p == 0 ? 0 : M - p)];
-      const double2 E = make_double2(f64.add(zm.x, zr.x), f64.sub(zm.y, zr.y));
-      const double2 O = make_double2(f64.add(zm.y, zr.y), f64.sub(zr.x, zm.x));
       const double2 wa = tw[p], wb = tw[M - p];
-      xa = make_double2(fma(wa.x, O.x, fma(-wa.y, O.y, E.x)), fma(wa.x, O.y, fma(wa.y, O.x, E.y)));
-      xbv = make_double2(fma(wb.x, O.x, fma(wb.y, O.y, E.x)), fma(wb.y, O.x, fma(-wb.x, O.y, -E.y)));
+      if (split_pair<INT>(f64, zm, zr, wa, wb, xa, xbv)) split_pair<false>(f64, zm, zr, wa, wb, xa, xbv);
     }
     smem_cl[0 * sys_len + at] = xa.x;
     smem_cl[1 * sys_len + at] = xa.y;
@@ -1631,14 +1713,7 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
   const double4_32a *f = fac + (size_t)m * L * lanes + j;
   double T, B;
   {
-    double t = 0.;
-#pragma unroll 8
-    for (int k = 0; k < L; ++k) {
-      const double4_32a c = f[(size_t)k * lanes];
-      t = fma(-c.y, t, f64.mul(c.x, x[k]));
-      x[k] = t;
-    }
-    T = t;
+    T = tdm_forward<INT>(f64, f, lanes, L, x);
     B = f[(size_t)(L - 1) * lanes].z;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -1663,15 +1738,7 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
   {
     const double Tu = __shfl_up_sync(0xffffffffu, T, 1), Bu = __shfl_up_sync(0xffffffffu, B, 1);
     const double carry = lane == 0 ? Cin : fma(Bu, Cin, Tu);
-    double u = 0.;
-#pragma unroll 8
-    for (int k = L - 1; k >= 0; --k) {
-      const double4_32a c = f[(size_t)k * lanes];
-      const double y = fma(c.z, carry, x[k]);
-      u = fma(-c.y, u, y);
-      x[k] = u;
-    }
-    Sx = u;
+    Sx = tdm_backward<INT>(f, lanes, L, carry, x);
     Cc = f[0].w;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -1695,8 +1762,7 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
   {
     const double Sd = __shfl_down_sync(0xffffffffu, Sx, 1), Cd = __shfl_down_sync(0xffffffffu, Cc, 1);
     const double next = lane == 31 ? Din : fma(Cd, Din, Sd);
-#pragma unroll 8
-    for (int k = 0; k < L; ++k) x[k] = fma(f[(size_t)k * lanes].w, next, x[k]);
+    tdm_fix<INT>(f, lanes, L, next, x);
   }
   // the singular mode m = 0 (systems 0, 1 of pair 0): zero mean over x,
   // imaginary part 0 (p is the same on the whole cluster)
@@ -1726,16 +1792,11 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
     const int at = (t / L) * S + (t % L);
     const double2 Xa = make_double2(smem_cl[0 * sys_len + at], smem_cl[1 * sys_len + at]);
     const double2 Xb = make_double2(smem_cl[2 * sys_len + at], smem_cl[3 * sys_len + at]);
-    const double2 E = make_double2(f64.add(Xa.x, Xb.x), f64.sub(Xa.y, Xb.y));
-    const double2 D = make_double2(f64.sub(Xa.x, Xb.x), f64.add(Xa.y, Xb.y));
-    const double2 wa = tw[p];
-    sp[(size_t)i * M1 + p] =
-        make_double2(fma(D.x, wa.y, fma(-D.y, wa.x, E.x)), fma(D.y, wa.y, fma(D.x, wa.x, E.y)));
-    if (p != 0 && 2 * p != M) {
-      const double2 wb = tw[M - p];
-      sp[(size_t)i * M1 + (M - p)] =
-          make_double2(fma(-D.y, wb.x, fma(-D.x, wb.y, E.x)), fma(D.y, wb.y, fma(-D.x, wb.x, -E.y)));
-    }
+    const double2 wa = tw[p], wb = tw[M - p];
+    double2 za, zb;
+    if (merge_pair<INT>(f64, Xa, Xb, wa, wb, za, zb)) merge_pair<false>(f64, Xa, Xb, wa, wb, za, zb);
+    sp[(size_t)i * M1 + p] = za;
+    if (p != 0 && 2 * p != M) sp[(size_t)i * M1 + (M - p)] = zb;
   }
 }
 
@@ -2326,10 +2387,8 @@ cudaError_t configure_kernels() {
   const int big = 227 * 1024;
   e = configure_fft<1, 2, 4, 8>(big);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_tdm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTdmSmemMax);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_poisson_tdm_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTdmSmemMax);
-  return e;
+  return allow_smem((int)kTdmSmemMax, k_poisson_tdm<false, false>, k_poisson_tdm<false, true>, k_poisson_tdm_cl<false>,
+                    k_poisson_tdm_cl<true>);
 }
 
 void launch_props(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const Bufs &b, bool den, bool vis,
@@ -2539,17 +2598,17 @@ void launch_poisson_tdm(cudaStream_t s, const Grid &g, const Bufs &b) {
   const double4_32a *fac = reinterpret_cast<const double4_32a *>(b.tdm_fac[tdm_group_index(G)]);
   if (tdm_uses_cluster(b.tiles, g.nx)) {  // four CTAs per pair, four warps each
     const int L = tdm_chunk(g.nx, 4), S = tdm_stride(g.nx, 4);
-    launch_pdl(k_poisson_tdm_cl, dim3(kTdmCluster * pairs, 1, g.nc), 128, 4 * 32 * (size_t)S * sizeof(double), s, g,
+    launch_pdl(integer_transforms(g) ? k_poisson_tdm_cl<true> : k_poisson_tdm_cl<false>, dim3(kTdmCluster * pairs, 1, g.nc), 128, 4 * 32 * (size_t)S * sizeof(double), s, g,
                L, S, fac, b.twiddle, b.spec);
     return;
   }
   if (tdm_global_stage(g.nx, G)) {  // one pair per block, staged in b.tdm_stage
-    launch_pdl(k_poisson_tdm<true>, dim3(pairs, 1, g.nc), 128 * G, 0, s, g, 1, G, tdm_chunk(g.nx, G), tdm_stride(g.nx, G),
+    launch_pdl(integer_transforms(g) ? k_poisson_tdm<true, true> : k_poisson_tdm<true, false>, dim3(pairs, 1, g.nc), 128 * G, 0, s, g, 1, G, tdm_chunk(g.nx, G), tdm_stride(g.nx, G),
                                                                  fac, b.twiddle, b.spec, b.tdm_stage);
     return;
   }
   const int mb = tdm_modes_per_block(b.tiles, g.nx);  // wavenumber pairs per block
-  launch_pdl(k_poisson_tdm<false>, dim3((pairs + mb - 1) / mb, 1, g.nc), 128 * mb * G, poisson_tdm_smem(g.nx, mb, G), s,
+  launch_pdl(integer_transforms(g) ? k_poisson_tdm<false, true> : k_poisson_tdm<false, false>, dim3((pairs + mb - 1) / mb, 1, g.nc), 128 * mb * G, poisson_tdm_smem(g.nx, mb, G), s,
       g, mb, G, tdm_chunk(g.nx, G), tdm_stride(g.nx, G), fac, b.twiddle, b.spec, nullptr);
 }
 
