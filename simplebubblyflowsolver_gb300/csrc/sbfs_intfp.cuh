@@ -146,7 +146,7 @@ SBFS_IF u32 wide(u32 e) { return e - (70u << 20) >= (1900u << 20); }
 // bits of the smaller operand were lost and the sum may end in a tie
 SBFS_IF u32 tie(u32 d, u32 lo) { return (u32)(d - 11u < 46u) & (u32)((lo & 0xffu) == 0u); }
 
-// a + b.  ZERO: both may be zero at once (+0 unless both are -0)
+// a + b.  ZERO: both may be zero at once
 template <bool ZERO>
 SBFS_IF double add(double a, double b, u32 &bad) {
   const u64 ua = bits(a), ub = bits(b);
@@ -165,11 +165,12 @@ SBFS_IF double add(double a, double b, u32 &bad) {
   if (ZERO) {
     const bool none = ((xh & kMag) | low(x)) == 0;
     zero |= none;
-    range = none ? (xh & yh) >> 31 : range;
+    range = none ? 0u : range;
   }
   bad |= range | ((u32)(sh == 0) & (u32)(S != 0)) | tie(d, low((u64)Ys));
   const u64 r = bits(round_pack(S, lead_zeros(sh), xh & 0xfff00000u));
-  return from_words(zero ? 0u : high(r), zero ? 0u : low(r));
+  // a zero sum is -0 only of two -0 (x = -y has one sign of each)
+  return from_words(zero ? xh & yh & kSign : high(r), zero ? 0u : low(r));
 }
 SBFS_IF double negate(double a) {
   const u64 u = bits(a);
@@ -230,7 +231,8 @@ SBFS_IF void addsub(double a, double b, double &s, double &t, u32 &bad) {
   t = from_words(same ? (qz ? 0u : qh ^ flip) : ph ^ flip, same ? ql : pl);
 }
 
-// a b; the operands' magnitudes lie between 2^-256 and 2^256, or are zero (ZERO)
+// a b; |a| lies between 2^-256 and 2^256, and so does |b|, or (ZERO) |b|
+// between 2^-763 and 2^737 and either may be zero
 template <bool ZERO>
 SBFS_IF double mul(double a, double b, u32 &bad) {
   const u64 ua = bits(a), ub = bits(b);
@@ -246,7 +248,7 @@ SBFS_IF double mul(double a, double b, u32 &bad) {
     return from_words(high(r), low(r));
   }
   const bool za = ((ah & kMag) | low(ua)) == 0, zb = ((bh & kMag) | low(ub)) == 0;
-  bad |= ((u32)!za & (u32)(ea - 767u >= 512u)) | ((u32)!zb & (u32)(eb - 767u >= 512u));
+  bad |= ((u32)!za & (u32)(ea - 767u >= 512u)) | ((u32)!zb & (u32)(eb - 260u >= 1500u));
   const bool z = za | zb;
   return from_words(z ? (ah ^ bh) & kSign : high(r), z ? 0u : low(r));
 }
