@@ -203,16 +203,19 @@ size_t case_off(const Ctx &c, const Layout &l) {
 // has not touched yet (a fresh calloc), are made present from the CPU: a copy
 // that finds them missing faults them in one by one over the CPU-GPU link.
 // 67 MB into untouched pages of 64 KB: 55.8 ms, or 2.1 ms here (one thread; 2
-// to 16 threads 1.4 to 2.2) and 0.5 ms for the copy; where all are present the
-// look costs microseconds.  Contents do not change, and a failure only leaves
-// the faults to the copy.
+// to 16 threads 1.4 to 2.2) and 0.5 ms for the copy.  The page in the middle
+// tells whether to look at the others; below 4 MB that look would be a part
+// of the copy's own time that shows (1 to 2 us).  Contents do not change, and
+// a failure only leaves the faults to the copy.
 void make_present(void *p, size_t bytes) {
 #ifdef MADV_POPULATE_WRITE
   static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-  if (bytes == 0) return;
+  if (bytes < (size_t)4 << 20) return;
   const uintptr_t lo = (uintptr_t)p & ~(uintptr_t)(page - 1);
   const uintptr_t hi = ((uintptr_t)p + bytes + page - 1) & ~(uintptr_t)(page - 1);
   const size_t n = (hi - lo) / page;
+  unsigned char mid = 0;
+  if (mincore(reinterpret_cast<void *>(lo + n / 2 * page), page, &mid) != 0 || (mid & 1)) return;
   std::vector<unsigned char> in(n);
   if (mincore(reinterpret_cast<void *>(lo), hi - lo, in.data()) != 0) return;
   for (size_t a = 0; a < n;) {
@@ -1842,11 +1845,15 @@ int sbfs_device_status(int *status) {
   return read_dt_status(*g_ctx, nullptr, status);
 }
 
+bool link_download(Ctx &c, int n, fluid_t *const *f, interface_t *const *itf, const std::vector<int> &slots);
 int sbfs_sync_to_host(const domain_t *d, fluid_t *f, interface_t *itf) {
   Ctx *c = g_ctx.get();
   if (!c || !c->resident) return 0;
   (void)d;
-  if (download_state(*c, f, itf, g_sync_mode == SBFS_SYNC_ALL)) return 1;
+  // (256 x 128 0.15 -> 0.05 ms, 2048 x 1024 0.89 -> 0.67 ms; 4096 x 2048 2.36 -> 2.67 ms)
+  const bool linked =
+      g_sync_mode != SBFS_SYNC_ALL && (long)c->nx * c->ny <= 1L << 22 && link_download(*c, 1, &f, &itf, {0});
+  if (!linked && download_state(*c, f, itf, g_sync_mode == SBFS_SYNC_ALL)) return 1;
   return sync(*c);
 }
 
@@ -1912,6 +1919,35 @@ bool link_tab_fill(Ctx &c, int k, fluid_t *f, interface_t *itf) {
     c.link_prev = c.link_host;
     c.link_epoch = g_reg_epoch;
   }
+  return true;
+}
+
+// the state of every case of a context into the caller's arrays by copy
+// kernels, one launch for two fields of all cases (a copy-engine call per
+// field, case and ghost row otherwise: 32 cases, 105 MB, 6.8 ms, or 1.0 ms so);
+// case i of the n given is this context's slot slots[i], or another's (-1).
+// Says no, with nothing launched, where the GPU cannot address an array.
+bool link_download(Ctx &c, int n, fluid_t *const *f, interface_t *const *itf, const std::vector<int> &slots) {
+  if (!g_host_link) return false;
+  constexpr int kOut = 6;
+  const int slot[kOut] = {HL_UX_OUT, HL_UY_OUT, HL_P_OUT, HL_PSI0_OUT, HL_PSI1_OUT, HL_VOF_OUT};
+  const Layout *lay[kOut] = {&L_UX, &L_UY, &L_P, &L_P, &L_P, &L_VOF};
+  double *const dev[kOut] = {c.U[c.iu], c.V[c.iu], c.b.p, c.PSI[c.ipsi], c.PSI[c.ipsi ^ 1], c.b.vof};
+  for (int i = 0; i < n; ++i) {
+    const int k = slots[i];
+    if (k < 0) continue;
+    const array_t *arr[kOut] = {&f[i]->ux, &f[i]->uy, &f[i]->p, &f[i]->psi[0], &f[i]->psi[1], &itf[i]->vof};
+    for (int q = 0; q < kOut; ++q) {
+      if (!layout_ok(*arr[q], *lay[q]) ||
+          !host_addressable(arr[q]->data, &c.link_tab[(size_t)k * kLinkSlots + slot[q]]))
+        return false;
+      make_present(arr[q]->data, sizeof(double) * (c.nx + lay[q]->ax0 + lay[q]->ax1) *
+                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1));
+    }
+  }
+  for (int q = 0; q < kOut; q += 2)
+    launch_host_rows(c.s, c.g, c.link_tab_dev, false, host_rows(c, slot[q], *lay[q], dev[q]),
+                     host_rows(c, slot[q + 1], *lay[q + 1], dev[q + 1]), 2, kLinkWide);
   return true;
 }
 
@@ -2010,7 +2046,14 @@ int sbfs_batch_sync_to_host(int n, const domain_t *const *domains, fluid_t *cons
   for (int i = 0; i < n; ++i)
     if (b->ident[2 * i] != fluids[i] || b->ident[2 * i + 1] != interfaces[i])
       return fail("case %d is not the one the batch holds", i);
-  if (batch_download(*b, n, fluids, interfaces, g_sync_mode == SBFS_SYNC_ALL)) return 1;
+  bool linked = g_sync_mode != SBFS_SYNC_ALL;
+  for (size_t q = 0; q < b->groups.size() && linked; ++q) {
+    std::vector<int> slots(n, -1);
+    for (int i = 0; i < n; ++i)
+      if (b->group_of[i] == (int)q) slots[i] = b->slot_of[i];
+    linked = link_download(*b->groups[q], n, fluids, interfaces, slots);
+  }
+  if (!linked && batch_download(*b, n, fluids, interfaces, g_sync_mode == SBFS_SYNC_ALL)) return 1;
   for (auto &c : b->groups)
     if (sync(*c)) return 1;
   return 0;
