@@ -1265,21 +1265,122 @@ __device__ __forceinline__ bool radix4(const Fp64 &f, const double2 *xr, double2
   return INT && n.bad != 0;
 }
 
+// The same butterflies with one thread per component and output, for launches
+// of a few warps, whose time is one thread's chain of FP64 instructions (65
+// cycles each): 4 in turn instead of 52 (radix 8, 16 lanes), 6 instead of 24
+// (radix 4 with twiddles, 8 lanes), 2 instead of 16 (without).  Every value
+// comes from the operation that radix8 and radix4 form it with.  Lanes of a
+// butterfly are l = 0, 1, ..; x is the value a lane holds, c the component it
+// belongs to, flip() a sign change where `neg` is set.  rot(z) has component c
+// from z's other one, negated where turn(c) is set.
+__device__ __forceinline__ double flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
+__device__ __forceinline__ double part(double2 z, int c) { return c ? z.y : z.x; }
+__device__ __forceinline__ void put(double2 *z, int c, double x) { reinterpret_cast<double *>(z)[c] = x; }
+
+__device__ __forceinline__ void radix8_lanes(const Fp64 &f, const double2 *xr, double2 *yr, int q8, double c8,
+                                             bool inverse, int l, bool store) {
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int c = l & 1, q = (l >> 1) & 3;
+  const bool odd = l >> 3;  // the lanes of b, else of a
+  auto turn = [inverse](int c) { return (c == 1) != inverse; };
+  // a_q = v_q + v_q+4, b_q = v_q - v_q+4
+  double x = fma(flip(part(xr[(q + 4) * q8], c), odd), f.one, part(xr[q * q8], c));
+  // a: e0 = a0 + a2, e2 = a1 + a3, e1 = a0 - a2, e3 = a1 - a3 in lanes q = 0 .. 3;
+  // b: A0 = b0 + rot b2, P1, A1 = b0 - rot b2 (component 1 - c), P3
+  const bool hi = q >= 2;
+  double o = __shfl_sync(all, x, lane ^ (!odd ? 4 : ((q & 1) ? 1 : 5)));
+  bool nx, no, nr = false;  // signs of x, o and the sum
+  if (!odd) {
+    nx = hi, no = false;
+  } else if (q == 3) {  // forward (y - x, -(x + y)), inverse (-(x + y), x - y)
+    nx = !turn(c), no = false, nr = turn(c);
+  } else if (q == 2) {
+    nx = !turn(1 - c), no = false;
+  } else {
+    nx = false, no = turn(c);
+  }
+  x = flip(fma(flip(x, nx), f.one, flip(o, no)), nr);
+  // a: X0 = e0 + e2, X4 = e0 - e2, X2 = e1 + rot e3, X6 = e1 - rot e3 (component 1 - c);
+  // b: E = P1 + P3 in lanes q = 1, D = P1 - P3 in lanes q = 3
+  o = __shfl_sync(all, x, lane ^ (odd ? 4 : (hi ? 3 : 2)));
+  if (!odd) {
+    nx = q == 1 || (q == 3 && !turn(1 - c));
+    no = q == 2 && turn(c);
+  } else {
+    nx = q == 3, no = false;
+  }
+  const double y = fma(flip(x, nx), f.one, flip(o, no));
+  if (!odd || (q & 1)) x = y;
+  // b: X1, X5 = A0 +- c8 E, X3, X7 = A1 +- c8 rot D
+  o = __shfl_sync(all, x, lane ^ 2);
+  const int oc = hi && (odd || q == 3) ? 1 - c : c;
+  if (odd) {
+    const double m = (q & 1) ? x : o, a = (q & 1) ? o : x;
+    x = fma(flip(c8, q & 1), flip(m, hi && turn(oc)), a);
+  }
+  const int at = odd ? (q == 0 ? 1 : (q == 1 ? 5 : (q == 2 ? 3 : 7))) : (q == 0 ? 0 : (q == 1 ? 4 : (q == 2 ? 2 : 6)));
+  if (store) put(yr + at, oc, x);
+}
+
+template <bool TWIDDLE>
+__device__ __forceinline__ void radix4_lanes(const Fp64 &f, const double2 *xr, double2 *yr, int q, int s,
+                                             const double2 *__restrict__ wm, int e, double two, bool inverse, int l,
+                                             bool store) {
+  const int lane = threadIdx.x & 31;
+  const int c = l & 1;
+  const bool sub = l & 2, h = l & 4;  // the lanes of a1, a3 (else a0, a2); of a2, a3 (else a0, a1)
+  const double2 vb = xr[h ? q : 0], vd = xr[h ? 3 * q : 2 * q];
+  double x;
+  if (TWIDDLE) {
+    const double2 w = wm[(h ? 3 : 2) * e];
+    double b = part(vb, c);
+    if (h) {
+      const double2 w1 = wm[e];
+      b = fma(vb.x, part(w1, c), f.mul(flip(vb.y, c == 0), part(w1, 1 - c)));
+    }
+    const double a = fma(w.x, part(vd, c), fma(flip(w.y, c == 0), part(vd, 1 - c), b));
+    x = fma(two, b, -a);
+    if (!sub) x = a;
+  } else {
+    x = fma(flip(part(vd, c), sub), f.one, part(vb, c));
+  }
+  // X0 = a0 + a2, X1 = a1 + rot a3, X2 = a0 - a2, X3 = a1 - rot a3 (component 1 - c)
+  const double o = __shfl_sync(0xffffffffu, x, lane ^ (sub ? 5 : 4));
+  const int oc = h && sub ? 1 - c : c;
+  const bool turned = sub && ((oc == 1) != inverse);
+  const double a = h ? o : x, r = flip(h ? x : o, turned != h);
+  x = fma(r, f.one, a);
+  if (store) put(yr + ((sub ? 1 : 0) + (h ? 2 : 0)) * s, oc, x);
+}
+
 // Stockham FFT (radix 4, one radix-8 stage first when log2 M is odd) of the
 // first `cols` of W rows of length M in shared memory.  Returns the buffer
 // holding the result.
 // tw: the twiddle buffer, exp(-2 pi i m / 2M) for m = 0..M, then W_M^e for
 // e < M, then their conjugates (the inverse's): one load per twiddle.
-template <int W, bool INT>
+// HOW: a thread's butterflies on the FP64 unit (kFftPlain), shared with the
+// integer pipes (kFftInt), or spread over lanes (kFftLanes).
+enum FftHow { kFftPlain, kFftInt, kFftLanes };
+template <int W, int HOW>
 __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__restrict__ tw, bool inverse, const Fp64 &f,
                              int cols) {
+  constexpr bool INT = HOW == kFftInt;
   const double two = f.reg(2.);
   const double2 *__restrict__ wm = tw + (M + 1) + (inverse ? M : 0);
   int Ns = 1;
   if ((__ffs(M) - 1) & 1) {  // log2 M odd (M >= 8)
     const double c8 = f.reg(0.70710678118654752440);
     const int q8 = M >> 3;
-    for (int t = threadIdx.x; t < cols * q8; t += blockDim.x) {
+    // lanes: whole warps take part in the exchanges, the last ones as copies
+    for (int t = threadIdx.x; HOW == kFftLanes && t < ((16 * cols * q8 + 31) & ~31); t += blockDim.x) {
+      const bool in = t < 16 * cols * q8;
+      const int b = in ? t >> 4 : 0, c = b / q8, j = b - c * q8;
+      radix8_lanes(f, x + c * M + j, y + c * M + 8 * j, q8, c8, inverse, t & 15, in);
+    }
+    for (int t = threadIdx.x; HOW != kFftLanes && t < cols * q8; t += blockDim.x) {
       const int c = t / q8, j = t - c * q8;
       const double2 *xr = x + c * M + j;
       double2 *yr = y + c * M + 8 * j;
@@ -1294,7 +1395,17 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
   const int q4 = M >> 2;
   for (; Ns < M; Ns <<= 2) {
     const int step = M / (4 * Ns);
-    for (int t = threadIdx.x; t < cols * q4; t += blockDim.x) {
+    for (int t = threadIdx.x; HOW == kFftLanes && t < ((8 * cols * q4 + 31) & ~31); t += blockDim.x) {
+      const bool in = t < 8 * cols * q4;
+      const int b = in ? t >> 3 : 0, c = b / q4, j = b - c * q4, kk = j & (Ns - 1);
+      const double2 *xr = x + c * M + j;
+      double2 *yr = y + c * M + ((j - kk) << 2) + kk;
+      if (Ns > 1)
+        radix4_lanes<true>(f, xr, yr, q4, Ns, wm, kk * step, two, inverse, t & 7, in);
+      else
+        radix4_lanes<false>(f, xr, yr, q4, Ns, wm, 0, two, inverse, t & 7, in);
+    }
+    for (int t = threadIdx.x; HOW != kFftLanes && t < cols * q4; t += blockDim.x) {
       const int c = t / q4, j = t - c * q4;
       const int kk = j & (Ns - 1);
       const double2 *xr = x + c * M + j;
@@ -1318,8 +1429,8 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
 // Q: the right-hand side from the predictor's face values q = pd u* + pa e
 // grad psi_old (ux, uy are qx, qy; egx, egy unused): 3 FP64 operations per
 // cell instead of 7
-template <int W, bool Q, bool INT>
-__global__ void __launch_bounds__(256, INT ? 4 : 1)
+template <int W, bool Q, int HOW>
+__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : 1)
     k_poisson_fwd(Grid g, const double *__restrict__ sc, int k, const double *__restrict__ ux,
                   const double *__restrict__ uy, const double *__restrict__ egx, const double *__restrict__ egy,
                   const double2 *__restrict__ tw, double2 *__restrict__ spec) {
@@ -1356,7 +1467,7 @@ __global__ void __launch_bounds__(256, INT ? 4 : 1)
     Ad[c * ny + r] = val;
   }
   __syncthreads();
-  double2 *Z = fft_rows<W, INT>(A, B, M, tw, false, f, min(W, g.nx + 1 - I0));
+  double2 *Z = fft_rows<W, HOW>(A, B, M, tw, false, f, min(W, g.nx + 1 - I0));
   // the packed transform z_m, m < M; k_poisson_tdm does the real-to-complex
   // split (there the FP64 pipe has room)
   const int M1 = M + 1;
@@ -1368,8 +1479,8 @@ __global__ void __launch_bounds__(256, INT ? 4 : 1)
   }
 }
 
-template <int W, bool INT>
-__global__ void __launch_bounds__(256, INT ? 4 : 1)
+template <int W, int HOW>
+__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : 1)
     k_poisson_inv(Grid g, const double2 *__restrict__ tw, const double2 *__restrict__ spec, double *__restrict__ psi) {
   pdl_entry();
   spec += (size_t)blockIdx.z * (g.css);
@@ -1386,7 +1497,7 @@ __global__ void __launch_bounds__(256, INT ? 4 : 1)
     A[c * M + mm] = I <= g.nx ? spec[(size_t)(I - 1) * M1 + mm] : make_double2(0., 0.);
   }
   __syncthreads();
-  const double2 *zr = fft_rows<W, INT>(A, B, M, tw, true, f, min(W, g.nx + 1 - I0));
+  const double2 *zr = fft_rows<W, HOW>(A, B, M, tw, true, f, min(W, g.nx + 1 - I0));
   const double *xd = reinterpret_cast<const double *>(zr);
   for (int t = threadIdx.x; t < W * ny; t += blockDim.x) {
     const int c = t % W, r = t / W;
@@ -2361,6 +2472,16 @@ int tdm_modes_per_block(const Tiles &t, int nx) {
 long cells(const Grid &g) { return (long)g.nx * g.ny * g.nc; }
 bool integer_stencils(const Grid &g) { return cells(g) >= 3L << 15; }
 bool integer_transforms(const Grid &g) { return cells(g) >= 1L << 18; }
+// Whether a launch spreads its butterflies over lanes: its warps issue twice
+// the FP64 instructions, in a quarter of the turns, so it pays while they are
+// few enough a scheduler, W M complex rows a block and that many blocks an SM
+// making at most 256.  Measured, us a launch of k_poisson_fwd: 64 x 64 (64)
+// 6.7 -> 4.8, 256 x 128 (128) 7.2 -> 5.8, 256 x 256 (256) 8.9 -> 8.7, 509 x
+// 256 (512) 9.3 -> 10.4, 128 x 1024 (1024) 17.1 -> 27.6.
+bool lane_transforms(const Grid &g, int w) {
+  const long blocks = (long)((g.nx + w - 1) / w) * g.nc;
+  return w * (g.ny / 2) * ((blocks + 151) / 152) <= 256;
+}
 // default pairs per block: as many as shared memory and 512 threads take, but
 // one block a pair while the pairs are too few to give every SM that many
 // (its warps share one FP64 unit a scheduler: 64 x 64 k_poisson_tdm 10.8 ->
@@ -2386,9 +2507,14 @@ cudaError_t allow_smem(int bytes, K... kernels) {
 }
 template <int... W>
 cudaError_t configure_fft(int bytes) {
-  return allow_smem(bytes, k_poisson_fwd<W, false, false>..., k_poisson_fwd<W, true, false>...,
-                    k_poisson_fwd<W, false, true>..., k_poisson_fwd<W, true, true>..., k_poisson_inv<W, false>...,
-                    k_poisson_inv<W, true>...);
+  const cudaError_t e =
+      allow_smem(bytes, k_poisson_fwd<1, false, kFftLanes>, k_poisson_fwd<2, false, kFftLanes>,
+                 k_poisson_fwd<1, true, kFftLanes>, k_poisson_fwd<2, true, kFftLanes>, k_poisson_inv<1, kFftLanes>,
+                 k_poisson_inv<2, kFftLanes>);
+  if (e != cudaSuccess) return e;
+  return allow_smem(bytes, k_poisson_fwd<W, false, kFftPlain>..., k_poisson_fwd<W, true, kFftPlain>...,
+                    k_poisson_fwd<W, false, kFftInt>..., k_poisson_fwd<W, true, kFftInt>...,
+                    k_poisson_inv<W, kFftPlain>..., k_poisson_inv<W, kFftInt>...);
 }
 
 cudaError_t configure_kernels() {
@@ -2569,8 +2695,9 @@ template <int W, bool Q>
 void poisson_fwd_w(cudaStream_t s, const Grid &g, const Bufs &b, const double *sc, int k, const double *ux,
                    const double *uy) {
   const int nb = (g.nx + W - 1) / W;
-  launch_pdl(integer_transforms(g) ? k_poisson_fwd<W, Q, true> : k_poisson_fwd<W, Q, false>, dim3(nb, 1, g.nc), 256,
-             poisson_fft_smem(g.ny, W), s, g, sc, k, ux, uy, b.egx, b.egy, b.twiddle, b.spec);
+  auto kern = integer_transforms(g) ? k_poisson_fwd<W, Q, kFftInt> : k_poisson_fwd<W, Q, kFftPlain>;
+  if (W <= 2 && lane_transforms(g, W)) kern = k_poisson_fwd<(W <= 2 ? W : 2), Q, kFftLanes>;
+  launch_pdl(kern, dim3(nb, 1, g.nc), 256, poisson_fft_smem(g.ny, W), s, g, sc, k, ux, uy, b.egx, b.egy, b.twiddle, b.spec);
 }
 
 template <bool Q>
@@ -2625,8 +2752,9 @@ void launch_poisson_tdm(cudaStream_t s, const Grid &g, const Bufs &b) {
 template <int W>
 void poisson_inv_w(cudaStream_t s, const Grid &g, const Bufs &b, double *psi_new) {
   const int nb = (g.nx + W - 1) / W;
-  launch_pdl(integer_transforms(g) ? k_poisson_inv<W, true> : k_poisson_inv<W, false>, dim3(nb, 1, g.nc), 256,
-             poisson_fft_smem(g.ny, W), s, g, b.twiddle, b.spec, psi_new);
+  auto kern = integer_transforms(g) ? k_poisson_inv<W, kFftInt> : k_poisson_inv<W, kFftPlain>;
+  if (W <= 2 && lane_transforms(g, W)) kern = k_poisson_inv<(W <= 2 ? W : 2), kFftLanes>;
+  launch_pdl(kern, dim3(nb, 1, g.nc), 256, poisson_fft_smem(g.ny, W), s, g, b.twiddle, b.spec, psi_new);
 }
 
 void launch_poisson_inv(cudaStream_t s, const Grid &g, const Bufs &b, double *psi_new) {
