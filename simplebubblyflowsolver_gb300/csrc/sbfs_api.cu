@@ -112,7 +112,7 @@ struct Ctx {
   // faces, the next substage's k_props beside the predictor, the Poisson
   // solve and the correction (fork / join events)
   cudaStream_t s2 = nullptr;
-  cudaEvent_t evf = nullptr, evd = nullptr, evp = nullptr, evx = nullptr, evF = nullptr;
+  cudaEvent_t evf = nullptr, evd = nullptr, evp = nullptr, evx = nullptr, evF = nullptr, evt = nullptr;
   bool props_ahead = false;  // the next substage's k_props is already on the side stream
   bool geo_ahead = false;    // the next substage's interface geometry and force are already on the side stream
   // device-resident steps: the last step formed the next step's first-substage
@@ -155,6 +155,7 @@ struct Ctx {
     if (e1) cudaEventDestroy(e1);
     if (evf) cudaEventDestroy(evf);
     if (evd) cudaEventDestroy(evd);
+    if (evt) cudaEventDestroy(evt);
     if (evp) cudaEventDestroy(evp);
     if (evx) cudaEventDestroy(evx);
     if (evF) cudaEventDestroy(evF);
@@ -523,6 +524,7 @@ int build_ctx(Ctx *c, const domain_t *d, int nc) {
   CK(cudaStreamCreateWithPriority(&c->s2, cudaStreamNonBlocking, prio_lo));
   CK(cudaEventCreateWithFlags(&c->evf, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&c->evd, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&c->evt, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&c->evp, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&c->evx, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&c->evF, cudaEventDisableTiming));
@@ -1010,6 +1012,7 @@ void enqueue_substage(Ctx &c, int k, bool par, bool wait_dt) {
   // substage the last device-resident step's (the same condition as its
   // geometry, pre_first)
   const bool cached = k > 0 || c.pre_first;
+  if (wait_dt) cudaStreamWaitEvent(c.s, c.evt, 0);
   timed(c, KC_PREDICT, [&] {
     launch_predict_mf(c.s, c.g, c.m, c.ph, b, sc, k, ux, uy, uxs, uys, den0, den1, psio, sxa, sxb, sya, syb, ifx,
                       ify, cached);
@@ -1037,8 +1040,12 @@ void enqueue_step(Ctx &c) {
     cudaEventRecord(c.evf, c.s);
     cudaStreamWaitEvent(c.s2, c.evf, 0);
     if (c.link) cudaStreamWaitEvent(c.s2, c.evh[1], 0);
-    launch_decide_dt(c.s2, c.g, c.m, c.ph, c.b, c.U[c.iu], c.V[c.iu], c.dt_fixed, g_coef[0]);
+    // the VOF update waits for the scalars (evd), the predictor for the column tables (evt)
+    launch_decide_dt_raw(c.s2, c.g, c.m, c.ph, c.U[c.iu], c.V[c.iu], c.b.dt_acc, c.b.scalars, c.b.status, c.dt_fixed,
+                         g_coef[0], nullptr);
     cudaEventRecord(c.evd, c.s2);
+    launch_decide_dt_tab(c.s2, c.g, c.m, c.b.scalars, c.b.coltab);
+    cudaEventRecord(c.evt, c.s2);
   } else {
     if (c.link) cudaStreamWaitEvent(c.s, c.evh[1], 0);
     timed(c, KC_DECIDE_DT,

@@ -107,8 +107,13 @@ template <bool DEN, bool VIS, bool GRAD, bool SCALED = false>
 __global__ void __launch_bounds__(BX *BY) k_props(Grid g, Metrics m, Phys ph0, const double *__restrict__ vof,
                                                   double *__restrict__ den, double *__restrict__ visux,
                                                   double *__restrict__ visuy, double *__restrict__ dvof,
-                                                  int compact) {
+                                                  int compact, int *__restrict__ counts) {
   pdl_entry();
+  // the interface cell and face counts k_curv_list adds to start at zero (a
+  // memset between the two would end their programmatic dependency: 5 us on
+  // the side stream of a 64 x 64 step)
+  if (counts && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y < 2)
+    counts[threadIdx.y * g.nc + blockIdx.z] = 0;
   const Phys ph = zphys(g, ph0);
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
   const int J = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -2071,12 +2076,12 @@ __global__ void __launch_bounds__(kDtFinThreads)
   // dt_adv = coef * min(1, min_i hx_i / (max|ux|_i + small), hy / (max|uy| + small))
   double d = 1.;
   int bad = 0;
-  const int i = blockIdx.x * kDtFinThreads + tid + 2;
-  if (i <= g.nx) {
-    // the column maxima are final (the stream order) and were formed at L2
-    const unsigned long long b = __ldcg(acc + i);
+  const int i = blockIdx.x * kDtFinThreads + tid + 2;  // column i, and nx + 1 for the uy quotient
+  if (i <= g.nx + 1) {
+    // the maxima are final (the stream order) and were formed at L2
+    const unsigned long long b = __ldcg(acc + (i <= g.nx ? i : g.nx + 2));
     bad = b >= kInfBits ? 1 : 0;
-    d = m.hxxf[i] / (__longlong_as_double((long long)b) + small);
+    d = (i <= g.nx ? m.hxxf[i] : g.hy) / (__longlong_as_double((long long)b) + small);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -2093,64 +2098,69 @@ __global__ void __launch_bounds__(kDtFinThreads)
       d = fmin(d, wmin[w]);
       bad |= wbad[w];
     }
-    // a positive d (or 1): the least bit pattern is the least value
-    atomicMax(acc + g.nx + 4, ~(unsigned long long)dbits(d));
     if (bad) atomicOr(status, 1);
-    __threadfence();
-    const unsigned int done = atomicAdd(reinterpret_cast<unsigned int *>(acc + g.nx + 5), 1u);
-    last = (done == gridDim.x - 1);
+    last = true;
+    if (gridDim.x > 1) {
+      // a positive d (or 1): the least bit pattern is the least value
+      atomicMax(acc + g.nx + 4, ~(unsigned long long)dbits(d));
+      __threadfence();
+      const unsigned int done = atomicAdd(reinterpret_cast<unsigned int *>(acc + g.nx + 5), 1u);
+      last = (done == gridDim.x - 1);
+    }
+    dt_sh = d;
   }
   __syncthreads();
   if (!last) return;
-  __threadfence();
-  if (tid == 0) {
-    const double dmin = __longlong_as_double((long long)~__ldcg(acc + g.nx + 4));
-    const unsigned long long by = __ldcg(acc + g.nx + 2);
-    double dt = fmin(dmin, g.hy / (__longlong_as_double((long long)by) + small));
+  // per-substage scalars; RK3 coefficients of src/runge_kutta.c:8-15.  Lane k
+  // < 3 takes substage k, lane k + 3 its dtold / dtnew beside lane k's refden
+  // / dtnew (an FP64 instruction takes the warp's slot once for all of them)
+  if (warp == 0) {
+    double dt = dt_sh;
+    if (gridDim.x > 1) {
+      __threadfence();
+      dt = __longlong_as_double((long long)~__ldcg(acc + g.nx + 4));
+    }
     dt *= coef_adv;
     dt = fmin(dt, dt_fixed);
-    if (by >= kInfBits) atomicOr(status, 1);
-    sc[0] = dt;
-    dt_sh = dt;
-  }
-  __syncthreads();
-  // per-substage scalars, one substage a lane (an FP64 instruction takes its
-  // warp's slot once for the three); RK3 coefficients of src/runge_kutta.c:8-15
-  if (tid < 3) {
-    const double dt = dt_sh;
-    const int k = tid, ko = (k + 2) % 3;
+    const int k = lane % 3, ko = (k + 2) % 3;
     const double al[3] = {32. / 60., 25. / 60., 45. / 60.};
     const double be[3] = {0. / 60., -17. / 60., -25. / 60.};
     const double abo = ko == 0 ? al[0] + be[0] : (ko == 1 ? al[1] + be[1] : al[2] + be[2]);
     const double ab = k == 0 ? al[0] + be[0] : (k == 1 ? al[1] + be[1] : al[2] + be[2]);
     const double a = k == 0 ? al[0] : (k == 1 ? al[1] : al[2]), b = k == 0 ? be[0] : (k == 1 ? be[1] : be[2]);
     const double dtold = abo * dt, dtnew = ab * dt;
-    sc[sc_adt(k)] = a * dt;
-    sc[sc_bdt(k)] = b * dt;
-    sc[sc_gdt(k)] = dtnew;
-    sc[sc_adt2(k)] = 2. * (a * dt);
-    sc[sc_bdt2(k)] = 2. * (b * dt);
-    const double gdt2 = 2. * dtnew;
-    sc[sc_gdt2(k)] = gdt2;
-    sc[sc_dtold(k)] = dtold;
-    sc[sc_dtnew(k)] = dtnew;
-    const double cdiv = ph.refden / dtnew * (0.5 / g.ny);
-    const double cadd = -(dtold / dtnew) * (0.5 / g.ny);
-    const double pax = cadd * (g.idx * g.idx), pay = cadd * (g.ihy * g.ihy);
-    const double cnew = dtnew * ph.irefden, cold = -dtold * ph.irefden, coldy = cold * g.ihy;
-    sc[sc_pdx(k)] = cdiv * g.idx;
-    sc[sc_pdy(k)] = cdiv * g.ihy;
-    sc[sc_pax(k)] = pax;
-    sc[sc_pay(k)] = pay;
-    sc[sc_cnew(k)] = cnew;
-    sc[sc_cold(k)] = cold;
-    sc[sc_cnewy(k)] = cnew * g.ihy;
-    sc[sc_coldy(k)] = coldy;
-    sc[sc_gdt2y(k)] = gdt2 * g.ihy;
-    sc[sc_coldyp(k)] = coldy / pay;
-    sc[sc_rpx(k)] = ph.rref2 * pax;
-    sc[sc_rpy(k)] = ph.rref2 * pay;
+    const double quo = (lane < 3 ? ph.refden : dtold) / dtnew;
+    const double ratio = __shfl_down_sync(0xffffffffu, quo, 3);
+    if (lane < 3) {
+      const double gdt2 = 2. * dtnew;
+      const double cdiv = quo * (0.5 / g.ny);
+      const double cadd = -ratio * (0.5 / g.ny);
+      const double pax = cadd * (g.idx * g.idx), pay = cadd * (g.ihy * g.ihy);
+      const double cnew = dtnew * ph.irefden, cold = -dtold * ph.irefden, coldy = cold * g.ihy;
+      if (k == 0) sc[0] = dt;
+      sc[sc_adt(k)] = a * dt;
+      sc[sc_bdt(k)] = b * dt;
+      sc[sc_gdt(k)] = dtnew;
+      sc[sc_adt2(k)] = 2. * (a * dt);
+      sc[sc_bdt2(k)] = 2. * (b * dt);
+      sc[sc_gdt2(k)] = gdt2;
+      sc[sc_dtold(k)] = dtold;
+      sc[sc_dtnew(k)] = dtnew;
+      sc[sc_pdx(k)] = cdiv * g.idx;
+      sc[sc_pdy(k)] = cdiv * g.ihy;
+      sc[sc_pax(k)] = pax;
+      sc[sc_pay(k)] = pay;
+      sc[sc_cnew(k)] = cnew;
+      sc[sc_cold(k)] = cold;
+      sc[sc_cnewy(k)] = cnew * g.ihy;
+      sc[sc_coldy(k)] = coldy;
+      sc[sc_gdt2y(k)] = gdt2 * g.ihy;
+      sc[sc_coldyp(k)] = coldy / pay;
+      sc[sc_rpx(k)] = ph.rref2 * pax;
+      sc[sc_rpy(k)] = ph.rref2 * pay;
+    }
   }
+  __syncthreads();
   // reset the scratch for the next launch
   for (int t = tid; t <= g.nx + 5; t += kDtFinThreads) acc[t] = 0ULL;
 }
@@ -2529,24 +2539,25 @@ cudaError_t configure_kernels() {
 void launch_props(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const Bufs &b, bool den, bool vis,
                   bool grad, double *den_out, bool scaled) {
   const dim3 gr = tile_grid(b.tiles, TK_PROPS, g.nx + 2, g.ny, g.nc), bl = tile_block(b.tiles, TK_PROPS);
+  int *counts = vis && grad ? b.icount : nullptr;  // a step's: the geometry follows
   if (scaled && vis && grad && !den)
     launch_pdl(k_props<false, true, true, true>, gr, bl, 0, s, g, m, ph, b.vof, den_out, b.visux, b.visuy, b.dvof,
-               compaction(b.tiles));
+               compaction(b.tiles), counts);
   else if (den && vis && grad)
     launch_pdl(k_props<true, true, true>, gr, bl, 0, s, g, m, ph, b.vof, den_out, b.visux, b.visuy, b.dvof,
-               compaction(b.tiles));
+               compaction(b.tiles), counts);
   else if (vis && grad)
     launch_pdl(k_props<false, true, true>, gr, bl, 0, s, g, m, ph, b.vof, den_out, b.visux, b.visuy, b.dvof,
-               compaction(b.tiles));
+               compaction(b.tiles), counts);
   else if (den)
     launch_pdl(k_props<true, false, false>, gr, bl, 0, s, g, m, ph, b.vof, den_out, b.visux, b.visuy, b.dvof,
-               compaction(b.tiles));
+               compaction(b.tiles), counts);
   else if (vis)
     launch_pdl(k_props<false, true, false>, gr, bl, 0, s, g, m, ph, b.vof, den_out, b.visux, b.visuy, b.dvof,
-               compaction(b.tiles));
+               compaction(b.tiles), counts);
   else if (grad)
     launch_pdl(k_props<false, false, true>, gr, bl, 0, s, g, m, ph, b.vof, den_out, b.visux, b.visuy, b.dvof,
-               compaction(b.tiles));
+               compaction(b.tiles), counts);
 }
 
 void launch_normal_curv(cudaStream_t s, const Grid &g, const Metrics &m, const Bufs &b, bool normal, bool curv,
@@ -2583,7 +2594,6 @@ void launch_interface_stage(cudaStream_t s, const Grid &g, const Metrics &m, con
                             const double *ux, const double *uy, const double *den0, int stage) {
   const dim3 gr = tile_grid(b.tiles, TK_FLUX_FORCE, g.nx, g.ny, g.nc), bl = tile_block(b.tiles, TK_FLUX_FORCE);
   if (stage == 0) {
-    cudaMemsetAsync(b.icount, 0, sizeof(int) * 2 * g.nc, s);  // cell and face counts
     launch_pdl(k_curv_list<true>, tile_grid(b.tiles, TK_CURV_LIST, g.nx, g.ny, g.nc), tile_block(b.tiles, TK_CURV_LIST),
                0, s, g, m, b.vof, b.dvof, ux, uy, b.curv, b.ilist, b.icount, b.flist, b.fcount, (double *)nullptr,
                compaction(b.tiles));
@@ -2600,7 +2610,6 @@ void launch_interface_stage(cudaStream_t s, const Grid &g, const Metrics &m, con
 }
 
 void launch_geometry(cudaStream_t s, const Grid &g, const Metrics &m, const Bufs &b) {
-  cudaMemsetAsync(b.icount, 0, sizeof(int) * 2 * g.nc, s);  // cell and face counts
   launch_pdl(k_curv_list<false>, tile_grid(b.tiles, TK_CURV_LIST, g.nx, g.ny, g.nc), tile_block(b.tiles, TK_CURV_LIST),
              0, s, g, m, b.vof, b.dvof, (const double *)nullptr, (const double *)nullptr, b.curv, b.ilist, b.icount,
              b.flist, b.fcount, b.tf, compaction(b.tiles));
@@ -2799,11 +2808,14 @@ void launch_decide_dt_raw(cudaStream_t s, const Grid &g, const Metrics &m, const
   const int gx = (g.nx + BX) / BX;
   while (gy > 1 && gx * gy * g.nc > 16 * 152) gy = (gy + 1) / 2;
   launch_pdl(k_decide_dt, dim3(gx, gy, g.nc), dim3(BX, BY), 0, s, g, ux, uy, acc);
-  launch_pdl(k_decide_dt_fin, dim3((g.nx - 1 + kDtFinThreads - 1) / kDtFinThreads, 1, g.nc), dim3(kDtFinThreads), 0, s,
-             g, m, ph, acc, sc, status, dt_fixed, coef_adv);
-  if (coltab)
-    launch_pdl(k_decide_dt_tab, dim3((g.nx + 2 + kDtFinThreads - 1) / kDtFinThreads, 1, g.nc), dim3(kDtFinThreads), 0,
-               s, g, m, (const double *)sc, coltab);
+  launch_pdl(k_decide_dt_fin, dim3((g.nx + kDtFinThreads - 1) / kDtFinThreads, 1, g.nc), dim3(kDtFinThreads), 0, s, g, m,
+             ph, acc, sc, status, dt_fixed, coef_adv);
+  if (coltab) launch_decide_dt_tab(s, g, m, sc, coltab);
+}
+
+void launch_decide_dt_tab(cudaStream_t s, const Grid &g, const Metrics &m, const double *sc, double *coltab) {
+  launch_pdl(k_decide_dt_tab, dim3((g.nx + 2 + kDtFinThreads - 1) / kDtFinThreads, 1, g.nc), dim3(kDtFinThreads), 0, s, g,
+             m, sc, coltab);
 }
 
 void launch_face_factor(cudaStream_t s, const Grid &g, const Phys &ph, const Bufs &b, const double *den,

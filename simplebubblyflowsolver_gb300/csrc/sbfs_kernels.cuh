@@ -164,6 +164,7 @@ void launch_decide_dt(cudaStream_t s, const Grid &g, const Metrics &m, const Phy
 void launch_decide_dt_raw(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const double *ux,
                           const double *uy, unsigned long long *acc, double *sc, int *status, double dt_fixed,
                           double coef_adv, double *coltab);
+void launch_decide_dt_tab(cudaStream_t s, const Grid &g, const Metrics &m, const double *sc, double *coltab);
 // e grad psi_old at the faces (b.egx, b.egy) from a density field and psi_old,
 // as k_predict_mf stores it (fine-grained entry points)
 void launch_face_factor(cudaStream_t s, const Grid &g, const Phys &ph, const Bufs &b, const double *den,
