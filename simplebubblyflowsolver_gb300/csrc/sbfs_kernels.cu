@@ -868,16 +868,16 @@ struct MomOut {
   double xx, yy, xy, yx;
 };
 
-// the four fluxes of one thread; returns whether an integer form gave up.
+// the four fluxes of one thread (PART 1: the corner's two, 2: the centre's); returns whether an integer form gave up.
 // Of the 27 FP64 operations (SCALED) the four sum-and-difference pairs of the
 // velocities and four of the products run on the integer pipes.  2048 x 1024
 // swarm, one launch: 110.6 us all in FP64 (FP64 unit 85% busy); 69.1 us with
 // a fifth product on the integer side (integer pipes 90%, FP64 73%), 73.6 us
 // with one sum more; 65.9 us as it stands (89%, 82%).
-template <bool INT, bool SCALED>
+template <bool INT, bool SCALED, int PART = 0>
 __device__ __forceinline__ bool momflux_cell(const Fp64 &f, const MomIn &in, const Phys &ph, MomOut &o) {
   Fp64Int<INT> q(f);
-  {
+  if (PART != 2) {  // corner
     double su, du, sw, dw;
     q.template addsub<true>(in.u0, in.us, su, du);  // zero along the walls
     q.addsub(in.w0, in.ww, sw, dw);
@@ -887,7 +887,7 @@ __device__ __forceinline__ bool momflux_cell(const Fp64 &f, const MomIn &in, con
     o.xy = fma(-q.mul(in.rq, fy), su, t4);
     o.yx = fma(-fx, sw, t4);
   }
-  {
+  if (PART != 1) {  // centre
     double su, du, sw, dw;
     q.addsub(in.u1, in.u0, su, du);
     q.addsub(in.w1, in.w0, sw, dw);
@@ -911,14 +911,18 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   const double *__restrict__ c4nuc = SCALED ? m.c4nucs : m.c4nuc + (size_t)blockIdx.z * g.cm;
   const double *__restrict__ c2nuf = SCALED ? m.c2nufs : m.c2nuf + (size_t)blockIdx.z * g.cm;
   const int I = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int J = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  // SPLIT (small launches): a thread takes the corner or the centre, the
+  // blocks of odd index the centres (see k_predict_mf)
+  constexpr bool SPLIT = !INT && SCALED;
+  const bool corner = !SPLIT || !(blockIdx.y & 1);
+  const int J = (SPLIT ? blockIdx.y >> 1 : blockIdx.y) * blockDim.y + threadIdx.y + 1;
   if (I > g.nx + 1 || J > g.ny) return;
   const Fp64 f(I);
   const int zr = blockIdx.z * g.ny;  // first row of this case
   const int r = J - 1 + zr, rm = wrap(J - 1, g.ny) + zr, rp = wrap(J + 1, g.ny) + zr;
-  const bool centre = I <= g.nx;
+  const bool centre = I <= g.nx && (!SPLIT || !corner);
   // centre (I, J); the threads of the last face have none and take the column before
-  const int Ic = centre ? I : I - 2;
+  const int Ic = I <= g.nx ? I : I - 2;
   auto load = [&](int r, int rm, int rp) {
     MomIn in;
     in.u0 = ux[ix(g, r, I - 1)];  // ux at face I, row J
@@ -938,7 +942,7 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
     in.c2 = c2nuf[I];
     // centre
     in.u1 = ux[ix(g, r, Ic)];
-    in.w1 = uy[ix(g, rp, centre ? I : Ic)];
+    in.w1 = uy[ix(g, rp, Ic)];
     in.vx1 = visux[ix(g, r, Ic)];
     in.vyn = visuy[ix(g, rp, I)];
     in.mx1 = mfx[ix(g, r, Ic)];
@@ -948,13 +952,20 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   };
   MomIn in = load(r, rm, rp);
   MomOut o;
-  if (momflux_cell<INT, SCALED>(f, in, ph, o)) {
+  if (SPLIT) {
+    if (corner)
+      momflux_cell<false, SCALED, 1>(f, in, ph, o);
+    else
+      momflux_cell<false, SCALED, 2>(f, in, ph, o);
+  } else if (momflux_cell<INT, SCALED>(f, in, ph, o)) {
     in = load(reread(r), reread(rm), reread(rp));
     momflux_cell<false, SCALED>(f, in, ph, o);
   }
-  pxy[ix(g, r, I - 1)] = o.xy;
-  pyx[ix(g, r, I - 1)] = o.yx;
-  if (STRESS == 2 || (STRESS == 1 && (I == 1 || I == g.nx + 1))) {
+  if (corner) {
+    pxy[ix(g, r, I - 1)] = o.xy;
+    pyx[ix(g, r, I - 1)] = o.yx;
+  }
+  if (corner && (STRESS == 2 || (STRESS == 1 && (I == 1 || I == g.nx + 1)))) {
     // txy = 0.5 (mu_s + mu_n) du/dy + 0.5 (mu_w + mu_e) dv/dx
     const MomIn in = load(reread(r), reread(rm), reread(rp));
     const double sx = in.vxs + in.vx0, sy = in.vyw + in.vy0, du = in.u0 - in.us, dw = in.w0 - in.ww;
@@ -1044,7 +1055,11 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   // the Poisson right-hand side's face values q = pd u* + pa e grad psi_old
   // (k_poisson_fwd<W, true> takes their differences across each cell)
   const int I = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int J = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  // FP64 alone (small launches): a thread takes one of the two faces, the
+  // blocks of odd index the uy faces, so that a warp's chain of instructions
+  // and its loads are half as long
+  const bool do_x = INT || !(blockIdx.y & 1), do_y = INT || (blockIdx.y & 1);
+  const int J = (INT ? blockIdx.y : blockIdx.y >> 1) * blockDim.y + threadIdx.y + 1;
   if (I > g.nx || J > g.ny) return;
   const Fp64 f(I);
   const int zr = blockIdx.z * g.ny;  // first row of this case
@@ -1077,7 +1092,7 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   }
   const double ps0 = CACHED && I != 1 && I != g.nx ? 0. : psio[ix(g, r, I)];
   // ---- ux at face I
-  if (I >= 2) {
+  if (do_x && I >= 2) {
     auto load = [&](int r, int rm, int rp) {
       PredIn in;
       in.u0 = ux[ix(g, r, I - 1)];
@@ -1102,7 +1117,7 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
     qx[ix(g, r, I - 1)] = o.q;
   }
   // ---- uy at face (I, J - 1/2)
-  {
+  if (do_y) {
     auto coefs = [&](PredIn &in) {
       in.cd = m.q4c[I], in.co = q4y, in.gp = sc[sc_gdt2y(k)], in.rp = sc[sc_rpy(k)], in.pa = sc[sc_pay(k)],
       in.pd = sc[sc_pdy(k)];
@@ -1146,14 +1161,14 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   }
   // walls: impermeable, no-slip; the wall faces' e grad psi_old (zero for a
   // Neumann psi_old, computed as the reference does)
-  if (I == 1) {
+  if (do_x && I == 1) {
     ux_out[ix(g, r, 0)] = 0.;
     uy_out[ix(g, r, 0)] = 0.;
     const double e = fma(rpx, rcp_nr(den1[ix(g, r, 0)] + den1[ix(g, r, 1)]), -pax) * (ps0 - psio[ix(g, r, 0)]);
     egx[ix(g, r, 0)] = e;
     qx[ix(g, r, 0)] = fma(sc[sc_pdx(k)], 0., e);
   }
-  if (I == g.nx) {
+  if (do_x && I == g.nx) {
     ux_out[ix(g, r, g.nx)] = 0.;
     uy_out[ix(g, r, g.nx + 1)] = 0.;
     const double e =
@@ -2664,7 +2679,8 @@ void launch_stress(cudaStream_t s, const Grid &g, const Metrics &m, const Bufs &
 
 void launch_momflux(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const Bufs &b,
                     const double *ux, const double *uy, int stress, bool scaled) {
-  const dim3 gr = tile_grid(b.tiles, TK_MOMFLUX, g.nx + 1, g.ny, g.nc), bl = tile_block(b.tiles, TK_MOMFLUX);
+  dim3 gr = tile_grid(b.tiles, TK_MOMFLUX, g.nx + 1, g.ny, g.nc), bl = tile_block(b.tiles, TK_MOMFLUX);
+  if (scaled && stress != 2 && !integer_stencils(g)) gr.y *= 2;  // the corner or the centre a thread
   // the unscaled forms (full-sync steps) run on the FP64 unit alone
   auto k = k_momflux<2, false, false>;
   if (stress != 2 && !scaled) k = stress == 1 ? k_momflux<1, false, false> : k_momflux<0, false, false>;
@@ -2685,7 +2701,9 @@ void launch_predict_mf(cudaStream_t s, const Grid &g, const Metrics &m, const Ph
                        const double *ify, bool cached) {
   auto kern = integer_stencils(g) ? (cached ? k_predict_mf<true, true> : k_predict_mf<false, true>)
                                : (cached ? k_predict_mf<true, false> : k_predict_mf<false, false>);
-  launch_pdl(kern, tile_grid(b.tiles, TK_PREDICT, g.nx, g.ny, g.nc), tile_block(b.tiles, TK_PREDICT), 0, s, g, m, ph,
+  dim3 gr = tile_grid(b.tiles, TK_PREDICT, g.nx, g.ny, g.nc);
+  if (!integer_stencils(g)) gr.y *= 2;  // one face a thread
+  launch_pdl(kern, gr, tile_block(b.tiles, TK_PREDICT), 0, s, g, m, ph,
              sc, k, ux, uy, ux_out, uy_out, b.pxx, b.pyy, b.pxy, b.pyx, b.p, ifx, ify, den0, den1, psi_old, srcux_a,
              srcux_b, srcuy_a, srcuy_b, b.egx, b.egy, b.coltab, b.qx, b.qy, b.rhofx, b.rhofy, b.dpsix, b.dpsiy);
 }
