@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 #include "sbfs_kernels.cuh"
 
@@ -858,6 +859,12 @@ __global__ void __launch_bounds__(BX *BY)
 // thread (I, J): I = 1..nx+1 handles the corner (I, J - 1/2) and, for I <= nx,
 // the centre (I, J)
 // ---------------------------------------------------------------------------
+// HOW the momentum kernels run a cell (chosen in stencil_how): both parts of
+// it (the corner and the centre; the ux and the uy face) in one thread, shared
+// with the integer pipes; one part a thread, the blocks of even and odd row
+// index taking one each, so that a warp's chain of instructions and loads is
+// half as long, shared or on the FP64 unit alone
+enum MomHow { kMomWhole, kMomSplitInt, kMomSplit };
 struct MomIn {
   double u0, us, u1, w0, ww, w1;        // ux at face I: row J, row J-1; at face I+1.  uy: cell I, I-1; row J+1/2
   double vx0, vxs, vx1, vy0, vyw, vyn;  // viscosities, likewise
@@ -898,8 +905,8 @@ __device__ __forceinline__ bool momflux_cell(const Fp64 &f, const MomIn &in, con
   return INT && q.bad != 0;
 }
 
-template <int STRESS, bool SCALED, bool INT>
-__global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
+template <int STRESS, bool SCALED, int HOW>
+__global__ void __launch_bounds__(BX *BY, SCALED && HOW == kMomWhole ? 5 : 1)
     k_momflux(Grid g, Metrics m, Phys ph0, const double *__restrict__ ux, const double *__restrict__ uy,
               const double *__restrict__ visux, const double *__restrict__ visuy, const double *__restrict__ mfx,
               const double *__restrict__ mfy, double *__restrict__ pxx, double *__restrict__ pyy,
@@ -911,9 +918,8 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   const double *__restrict__ c4nuc = SCALED ? m.c4nucs : m.c4nuc + (size_t)blockIdx.z * g.cm;
   const double *__restrict__ c2nuf = SCALED ? m.c2nufs : m.c2nuf + (size_t)blockIdx.z * g.cm;
   const int I = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  // SPLIT (small launches): a thread takes the corner or the centre, the
-  // blocks of odd index the centres (see k_predict_mf)
-  constexpr bool SPLIT = !INT && SCALED;
+  // the unscaled forms (full-sync steps) run whole, on the FP64 unit alone
+  constexpr bool SPLIT = SCALED && HOW != kMomWhole, INT = SCALED && HOW != kMomSplit;
   const bool corner = !SPLIT || !(blockIdx.y & 1);
   const int J = (SPLIT ? blockIdx.y >> 1 : blockIdx.y) * blockDim.y + threadIdx.y + 1;
   if (I > g.nx + 1 || J > g.ny) return;
@@ -952,22 +958,25 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   };
   MomIn in = load(r, rm, rp);
   MomOut o;
-  if (SPLIT) {
-    if (corner)
-      momflux_cell<false, SCALED, 1>(f, in, ph, o);
-    else
-      momflux_cell<false, SCALED, 2>(f, in, ph, o);
-  } else if (momflux_cell<INT, SCALED>(f, in, ph, o)) {
-    in = load(reread(r), reread(rm), reread(rp));
-    momflux_cell<false, SCALED>(f, in, ph, o);
-  }
+  auto cell = [&](auto part) {
+    if (momflux_cell<INT, SCALED, part>(f, in, ph, o)) {
+      in = load(reread(r), reread(rm), reread(rp));
+      momflux_cell<false, SCALED, part>(f, in, ph, o);
+    }
+  };
+  if (!SPLIT)
+    cell(std::integral_constant<int, 0>());
+  else if (corner)
+    cell(std::integral_constant<int, 1>());
+  else
+    cell(std::integral_constant<int, 2>());
   if (corner) {
     pxy[ix(g, r, I - 1)] = o.xy;
     pyx[ix(g, r, I - 1)] = o.yx;
   }
   if (corner && (STRESS == 2 || (STRESS == 1 && (I == 1 || I == g.nx + 1)))) {
     // txy = 0.5 (mu_s + mu_n) du/dy + 0.5 (mu_w + mu_e) dv/dx
-    const MomIn in = load(reread(r), reread(rm), reread(rp));
+    if (!SPLIT) in = load(reread(r), reread(rm), reread(rp));
     const double sx = in.vxs + in.vx0, sy = in.vyw + in.vy0, du = in.u0 - in.us, dw = in.w0 - in.ww;
     txy[ix(g, r, I - 1)] = SCALED ? fma(sx, du * (g.hihy * ph.inuy2), sy * (dw * (m.hihxxf[I] * ph.inuy4)))
                                   : fma(sx, du * g.hihy, sy * (dw * m.hihxxf[I]));
@@ -1037,8 +1046,8 @@ __device__ __forceinline__ bool predict_face(const Fp64 &f, const PredIn &in, do
   return INT && n.bad != 0;
 }
 
-template <bool CACHED, bool INT>
-__global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
+template <bool CACHED, int HOW>
+__global__ void __launch_bounds__(BX *BY, HOW == kMomWhole ? 5 : 1)
     k_predict_mf(Grid g, Metrics m, Phys ph0, const double *__restrict__ sc, int k, const double *__restrict__ ux,
                  const double *__restrict__ uy, double *__restrict__ ux_out, double *__restrict__ uy_out,
                  const double *__restrict__ pxx, const double *__restrict__ pyy, const double *__restrict__ pxy,
@@ -1055,11 +1064,9 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   // the Poisson right-hand side's face values q = pd u* + pa e grad psi_old
   // (k_poisson_fwd<W, true> takes their differences across each cell)
   const int I = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  // FP64 alone (small launches): a thread takes one of the two faces, the
-  // blocks of odd index the uy faces, so that a warp's chain of instructions
-  // and its loads are half as long
-  const bool do_x = INT || !(blockIdx.y & 1), do_y = INT || (blockIdx.y & 1);
-  const int J = (INT ? blockIdx.y : blockIdx.y >> 1) * blockDim.y + threadIdx.y + 1;
+  constexpr bool WHOLE = HOW == kMomWhole, INT = HOW != kMomSplit;
+  const bool do_x = WHOLE || !(blockIdx.y & 1), do_y = WHOLE || (blockIdx.y & 1);
+  const int J = (WHOLE ? blockIdx.y : blockIdx.y >> 1) * blockDim.y + threadIdx.y + 1;
   if (I > g.nx || J > g.ny) return;
   const Fp64 f(I);
   const int zr = blockIdx.z * g.ny;  // first row of this case
@@ -1073,9 +1080,9 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
   // (y faces): e pa = (2 rho_ref pa) / (2 rho) - pa
   const double rpx = sc[sc_rpx(k)], pax = sc[sc_pax(k)];
   const double q4y = f.reg(g.q4y), hgrav = f.reg(ph.hgrav);
-  __shared__ double yb[INT ? 11 : 1][BX * BY];
+  __shared__ double yb[WHOLE ? 11 : 1][BX * BY];
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  if (INT) {
+  if (WHOLE) {
     async_copy(&yb[0][tid], uy + ix(g, r, I));
     async_copy(&yb[1][tid], ifrcy + ix(g, r, I - 1));
     async_copy(&yb[2][tid], pyx + ix(g, r, I));
@@ -1136,7 +1143,7 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
       return in;
     };
     PredOut o;
-    if (INT) {
+    if (WHOLE) {
       async_wait();
       PredIn in;
       in.u0 = yb[0][tid], in.frc = yb[1][tid];
@@ -1150,8 +1157,8 @@ __global__ void __launch_bounds__(BX *BY, INT ? 5 : 1)
       coefs(in);
       if (predict_face<true, false>(f, in, hgrav, adt2, bdt2, k, o))
         predict_face<false, false>(f, load(reread(r), reread(rm)), hgrav, adt2, bdt2, k, o);
-    } else {
-      predict_face<false, false>(f, load(r, rm), hgrav, adt2, bdt2, k, o);
+    } else if (predict_face<INT, false>(f, load(r, rm), hgrav, adt2, bdt2, k, o)) {
+      predict_face<false, false>(f, load(reread(r), reread(rm)), hgrav, adt2, bdt2, k, o);
     }
     sry[ix(g, r, I)] = o.rho1;
     uy_out[ix(g, r, I)] = o.u;
@@ -2489,13 +2496,21 @@ int tdm_modes_per_block(const Tiles &t, int nx) {
 // Whether the stencils, and the transforms, of a launch over these cells share
 // their arithmetic with the integer pipes: only where enough warps are in
 // flight to keep the FP64 unit busy; below that an integer form's longer
-// chain of instructions sets a warp's time.  Measured, us a launch FP64 alone
-// -> shared: 500 x 128 k_momflux 6.9 -> 7.1, k_predict_mf 9.1 -> 9.6,
-// k_poisson_fwd 7.0 -> 7.5; 509 x 256 10.3 -> 9.2, 13.8 -> 13.2, 9.2 -> 10.7;
-// 512 x 512 16.8 -> 13.6, 21.2 -> 19.2, 13.3 -> 13.7 (k_poisson_inv 12.3 ->
-// 11.6); 1000 x 512 27.1 -> 20.4, 36.4 -> 30.2, 20.5 -> 18.4.
+// chain of instructions sets a warp's time.  Measured, us a launch, one part
+// a thread on the FP64 unit, shared, and both parts shared: k_momflux 256 x
+// 128 5.0, 4.5, 6.5; 500 x 128 6.7, 6.0, 7.1; 509 x 256 9.3, 8.0, 8.8; 512 x
+// 512 16.2, 12.8, 13.4; k_predict_mf 6.7, 6.1, 8.4; 9.0, 8.5, 9.6; 12.8, 13.0,
+// 13.3; 20.6, 21.0, 19.2.  The lines follow the whole step, whose side stream
+// runs beside the predictor: us with one part on the FP64 unit and shared, 256
+// x 128 113.7, 115.9; 500 x 128 160.0, 153.6; 509 x 256 244.6, 237.3, and
+// 220.3 with both shared.  k_poisson_fwd in a thread, FP64 alone and shared:
+// 509 x 256 9.2, 10.7; 512 x 512 13.3, 13.7 (k_poisson_inv 12.3, 11.6); 1000 x 512 20.5,
+// 18.4.
 long cells(const Grid &g) { return (long)g.nx * g.ny * g.nc; }
 bool integer_stencils(const Grid &g) { return cells(g) >= 3L << 15; }
+MomHow stencil_how(const Grid &g) {
+  return integer_stencils(g) ? kMomWhole : (cells(g) >= 3L << 14 ? kMomSplitInt : kMomSplit);
+}
 bool integer_transforms(const Grid &g) { return cells(g) >= 1L << 18; }
 // Whether a launch spreads its butterflies over lanes: its warps issue twice
 // the FP64 instructions, in a quarter of the turns, so it pays while they are
@@ -2680,15 +2695,17 @@ void launch_stress(cudaStream_t s, const Grid &g, const Metrics &m, const Bufs &
 void launch_momflux(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const Bufs &b,
                     const double *ux, const double *uy, int stress, bool scaled) {
   dim3 gr = tile_grid(b.tiles, TK_MOMFLUX, g.nx + 1, g.ny, g.nc), bl = tile_block(b.tiles, TK_MOMFLUX);
-  if (scaled && stress != 2 && !integer_stencils(g)) gr.y *= 2;  // the corner or the centre a thread
-  // the unscaled forms (full-sync steps) run on the FP64 unit alone
-  auto k = k_momflux<2, false, false>;
-  if (stress != 2 && !scaled) k = stress == 1 ? k_momflux<1, false, false> : k_momflux<0, false, false>;
+  auto k = k_momflux<2, false, kMomWhole>;
+  if (stress != 2 && !scaled) k = stress == 1 ? k_momflux<1, false, kMomWhole> : k_momflux<0, false, kMomWhole>;
   if (stress != 2 && scaled) {
-    if (integer_stencils(g))
-      k = stress == 1 ? k_momflux<1, true, true> : k_momflux<0, true, true>;
+    const MomHow how = stencil_how(g);
+    if (how == kMomWhole)
+      k = stress == 1 ? k_momflux<1, true, kMomWhole> : k_momflux<0, true, kMomWhole>;
+    else if (how == kMomSplitInt)
+      k = stress == 1 ? k_momflux<1, true, kMomSplitInt> : k_momflux<0, true, kMomSplitInt>;
     else
-      k = stress == 1 ? k_momflux<1, true, false> : k_momflux<0, true, false>;
+      k = stress == 1 ? k_momflux<1, true, kMomSplit> : k_momflux<0, true, kMomSplit>;
+    if (how != kMomWhole) gr.y *= 2;
   }
   launch_pdl(k, gr, bl, 0, s, g, m, ph, ux, uy, b.visux, b.visuy, b.mfluxx, b.mfluxy, b.pxx, b.pyy, b.pxy, b.pyx,
              b.txx, b.txy, b.tyy);
@@ -2699,10 +2716,12 @@ void launch_predict_mf(cudaStream_t s, const Grid &g, const Metrics &m, const Ph
                        const double *den0, const double *den1, const double *psi_old, double *srcux_a,
                        const double *srcux_b, double *srcuy_a, const double *srcuy_b, const double *ifx,
                        const double *ify, bool cached) {
-  auto kern = integer_stencils(g) ? (cached ? k_predict_mf<true, true> : k_predict_mf<false, true>)
-                               : (cached ? k_predict_mf<true, false> : k_predict_mf<false, false>);
+  const MomHow how = stencil_how(g);
+  auto kern = cached ? k_predict_mf<true, kMomSplit> : k_predict_mf<false, kMomSplit>;
+  if (how == kMomSplitInt) kern = cached ? k_predict_mf<true, kMomSplitInt> : k_predict_mf<false, kMomSplitInt>;
+  if (how == kMomWhole) kern = cached ? k_predict_mf<true, kMomWhole> : k_predict_mf<false, kMomWhole>;
   dim3 gr = tile_grid(b.tiles, TK_PREDICT, g.nx, g.ny, g.nc);
-  if (!integer_stencils(g)) gr.y *= 2;  // one face a thread
+  if (how != kMomWhole) gr.y *= 2;
   launch_pdl(kern, gr, tile_block(b.tiles, TK_PREDICT), 0, s, g, m, ph,
              sc, k, ux, uy, ux_out, uy_out, b.pxx, b.pyy, b.pxy, b.pyx, b.p, ifx, ify, den0, den1, psi_old, srcux_a,
              srcux_b, srcuy_a, srcuy_b, b.egx, b.egy, b.coltab, b.qx, b.qy, b.rhofx, b.rhofy, b.dpsix, b.dpsiy);
