@@ -114,6 +114,7 @@ struct Ctx {
   cudaStream_t s2 = nullptr;
   cudaEvent_t evf = nullptr, evd = nullptr, evp = nullptr, evx = nullptr, evF = nullptr, evt = nullptr;
   bool props_ahead = false;  // the next substage's k_props is already on the side stream
+  bool bulk_first = false;   // this step's first bulk fluxes are on the side stream, before decide_dt
   bool geo_ahead = false;    // the next substage's interface geometry and force are already on the side stream
   // device-resident steps: the last step formed the next step's first-substage
   // geometry and force (into IFX[2]) from its final vof and density, for the
@@ -941,7 +942,7 @@ void enqueue_substage(Ctx &c, int k, bool par, bool wait_dt) {
     }
     if (c.link && k == 0) cudaStreamWaitEvent(c.s, c.evh[1], 0);  // the velocity is in
     timed(c, KC_FACE_FLUX, [&] { launch_face_flux(c.s, c.g, b, ux, uy); });
-    const bool bulk_here = !par || (k == 0 && c.link);
+    const bool bulk_here = !par || (k == 0 && c.link && !c.bulk_first);
     if (par && !pre && !bulk_here) cudaStreamWaitEvent(c.s, c.evx, 0);
     if (bulk_here) timed(c, KC_BULK_FLUX, [&] { launch_bulk_flux(c.s, c.g, c.m, c.ph, b, ux, uy); });
     if (wait_dt) cudaStreamWaitEvent(c.s, c.evd, 0);
@@ -1035,11 +1036,21 @@ void enqueue_step(Ctx &c) {
   const bool par = !g_prof.on;
   c.props_ahead = false;
   c.geo_ahead = false;
+  c.bulk_first = false;
   if (c.link) link_in(c);
   if (par) {
     cudaEventRecord(c.evf, c.s);
     cudaStreamWaitEvent(c.s2, c.evf, 0);
     if (c.link) cudaStreamWaitEvent(c.s2, c.evh[1], 0);
+    // a small host-linked step's bulk fluxes ahead of decide_dt, which its VOF
+    // update does not wait for as long as for the listed faces and them in turn
+    // (256 x 128 11.7 -> 9.5 us from the velocity's arrival to the VOF update;
+    // on a large grid both take longer than the geometry)
+    c.bulk_first = c.link && g_geo_ahead && (long)c.nx * c.ny * c.nc < 3L << 15;
+    if (c.bulk_first) {
+      launch_bulk_flux(c.s2, c.g, c.m, c.ph, c.b, c.U[c.iu], c.V[c.iu]);
+      cudaEventRecord(c.evx, c.s2);
+    }
     // the VOF update waits for the scalars (evd), the predictor for the column tables (evt)
     launch_decide_dt_raw(c.s2, c.g, c.m, c.ph, c.U[c.iu], c.V[c.iu], c.b.dt_acc, c.b.scalars, c.b.status, c.dt_fixed,
                          g_coef[0], nullptr);
@@ -1056,10 +1067,10 @@ void enqueue_step(Ctx &c) {
   if (par && g_geo_ahead && c.make_next) cudaStreamWaitEvent(c.s, c.evp, 0);
   if (c.link) {
     // the velocity and p of the last correction, then the copy stream joins
+    // (with them the scalars and the status, which read_dt_status copies after other steps)
     launch_host_rows(c.s, c.g, c.link_tab_dev, false, host_rows(c, HL_UX_OUT, L_UX, c.U[c.iu]),
-                     host_rows(c, HL_UY_OUT, L_UY, c.V[c.iu]), 2, kLinkWide);
-    launch_host_rows(c.s, c.g, c.link_tab_dev, false, host_rows(c, HL_P_OUT, L_P, c.b.p), HostRows{}, 1,
-                     kLinkWide);
+                     host_rows(c, HL_UY_OUT, L_UY, c.V[c.iu]), 3, kLinkWide, host_rows(c, HL_P_OUT, L_P, c.b.p),
+                     c.b.scalars, c.small_host, kScalars * c.nc + (c.nc + 1) / 2);
     cudaEventRecord(c.evh[4], c.s3);
     cudaStreamWaitEvent(c.s, c.evh[4], 0);
   }
@@ -1378,8 +1389,9 @@ int download_state(Ctx &c, fluid_t *f, interface_t *itf, bool all) {
   return 0;
 }
 
-int read_dt_status(Ctx &c, double *dt, int *status) {
-  CK(cudaMemcpyAsync(c.small_host, c.b.scalars, sizeof(double) * (kScalars + 1), cudaMemcpyDeviceToHost, c.s));
+// copied: the step left them in small_host (a host-linked step)
+int read_dt_status(Ctx &c, double *dt, int *status, bool copied = false) {
+  if (!copied) CK(cudaMemcpyAsync(c.small_host, c.b.scalars, sizeof(double) * (kScalars + 1), cudaMemcpyDeviceToHost, c.s));
   if (sync(c)) return 1;
   if (dt) *dt = c.small_host[0];
   if (status) memcpy(status, c.small_host + kScalars, sizeof(int));
@@ -1527,8 +1539,9 @@ int batch_download(Batch &b, int n, fluid_t *const *f, interface_t *const *itf, 
 }
 
 // dt of every case after the last step; fails on a non-finite velocity
-int batch_read_dt(Batch &b, int n, double *dts) {
+int batch_read_dt(Batch &b, int n, double *dts, bool copied = false) {
   for (auto &c : b.groups) {
+    if (copied) break;  // the host-linked step left them in small_host
     const size_t bytes = sizeof(double) * (size_t)kScalars * c->nc + sizeof(int) * c->nc;
     CK(cudaMemcpyAsync(c->small_host, c->b.scalars, bytes, cudaMemcpyDeviceToHost, c->s));
   }
@@ -1930,7 +1943,7 @@ bool link_tab_fill(Ctx &c, int k, fluid_t *f, interface_t *itf) {
 }
 
 // the state of every case of a context into the caller's arrays by copy
-// kernels, one launch for two fields of all cases (a copy-engine call per
+// kernels, one launch for three fields of all cases (a copy-engine call per
 // field, case and ghost row otherwise: 32 cases, 105 MB, 6.8 ms, or 1.0 ms so);
 // case i of the n given is this context's slot slots[i], or another's (-1).
 // Says no, with nothing launched, where the GPU cannot address an array.
@@ -1952,9 +1965,10 @@ bool link_download(Ctx &c, int n, fluid_t *const *f, interface_t *const *itf, co
                                      (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1));
     }
   }
-  for (int q = 0; q < kOut; q += 2)
+  for (int q = 0; q < kOut; q += 3)
     launch_host_rows(c.s, c.g, c.link_tab_dev, false, host_rows(c, slot[q], *lay[q], dev[q]),
-                     host_rows(c, slot[q + 1], *lay[q + 1], dev[q + 1]), 2, kLinkWide);
+                     host_rows(c, slot[q + 1], *lay[q + 1], dev[q + 1]), 3, kLinkWide,
+                     host_rows(c, slot[q + 2], *lay[q + 2], dev[q + 2]));
   return true;
 }
 
@@ -1973,7 +1987,7 @@ int integrate(const domain_t *d, fluid_t *f, interface_t *itf, double *dt) {
     c->resident = true;
     swap_data(f->psi[0], f->psi[1]);
     int status = 0;
-    if (read_dt_status(*c, dt, &status)) return 1;
+    if (read_dt_status(*c, dt, &status, true)) return 1;
     if (status & 1) return fail("non-finite velocity detected by decide_dt");
     return 0;
   }
@@ -2009,7 +2023,7 @@ int sbfs_integrate_batch(int n, const domain_t *const *domains, fluid_t *const *
       c->resident = true;
     }
     for (int i = 0; i < n; ++i) swap_data(fluids[i]->psi[0], fluids[i]->psi[1]);
-    return batch_read_dt(*b, n, dts);
+    return batch_read_dt(*b, n, dts, true);
   }
   bool upload = g_sync_mode != SBFS_SYNC_NONE;
   for (auto &c : b->groups) upload = upload || !c->resident;

@@ -2896,14 +2896,18 @@ void launch_bc_vof(cudaStream_t s, const Grid &g, double *vof) {
 // (what the reference's halo exchange leaves there, src/halo.c:18-76).  Case
 // z of a batch is blockIdx.y: its arrays are tab[z * kLinkSlots + slot], its
 // device rows start at dev + z * cs1.  Each thread keeps four loads in flight:
-// the link's latency is microseconds.
+// the link's latency is microseconds.  nwords doubles from words to
+// words_host (page-locked) come along.
 template <bool kIn>
-__global__ void __launch_bounds__(256) k_host_rows(Grid g, double *const *tab, HostRows a, HostRows b, int nf) {
+__global__ void __launch_bounds__(256) k_host_rows(Grid g, double *const *tab, HostRows a, HostRows b, HostRows c, int nf,
+                                                   const double *words, double *words_host, int nwords) {
   pdl_entry();
+  if (blockIdx.x == 0 && blockIdx.y == 0)
+    for (int t = threadIdx.x; t < nwords; t += blockDim.x) words_host[t] = words[t];
   const int z = blockIdx.y;
   const int stride = gridDim.x * blockDim.x;
   for (int q = 0; q < nf; ++q) {
-    const HostRows f = q == 0 ? a : b;
+    const HostRows f = q == 0 ? a : (q == 1 ? b : c);
     double *h = tab[(size_t)z * kLinkSlots + f.slot];
     double *dev = f.dev + (size_t)z * g.cs1;
     const int n = (kIn ? g.ny : g.ny + f.ay0 + f.ay1) * f.row;
@@ -2933,12 +2937,12 @@ __global__ void __launch_bounds__(256) k_host_rows(Grid g, double *const *tab, H
 }
 
 void launch_host_rows(cudaStream_t s, const Grid &g, double *const *tab, bool in, HostRows a, HostRows b, int nf,
-                      int width) {
+                      int width, HostRows c, const double *words, double *words_host, int nwords) {
   const dim3 grid(std::max(1, width / g.nc), g.nc);
   if (in)
-    launch_pdl(k_host_rows<true>, grid, 256, 0, s, g, tab, a, b, nf);
+    launch_pdl(k_host_rows<true>, grid, 256, 0, s, g, tab, a, b, c, nf, words, words_host, nwords);
   else
-    launch_pdl(k_host_rows<false>, grid, 256, 0, s, g, tab, a, b, nf);
+    launch_pdl(k_host_rows<false>, grid, 256, 0, s, g, tab, a, b, c, nf, words, words_host, nwords);
 }
 
 }  // namespace sbfs

@@ -249,9 +249,11 @@ struct HostRows {
   int slot, row, ay0, ay1;
   double *dev;
 };
-// nf (1 or 2) fields of every case, host -> device when in, else device ->
+// nf (1 to 3) fields of every case, host -> device when in, else device ->
 // host, on about `width` blocks (at least one per case)
+// and nwords doubles of the device to page-locked host memory with them
 void launch_host_rows(cudaStream_t s, const Grid &g, double *const *tab, bool in, HostRows a, HostRows b, int nf,
-                      int width);
+                      int width, HostRows c = HostRows{}, const double *words = nullptr, double *words_host = nullptr,
+                      int nwords = 0);
 
 }  // namespace sbfs
