@@ -264,6 +264,87 @@ int d2h(Ctx &c, array_t &a, const Layout &l, const double *dev) {
   return 0;
 }
 
+// host memory the GPU can address: any on a system whose GPU reads pageable
+// memory through the host page tables, else memory registered with CUDA
+int g_pageable = -1, g_pageable_dev = -1;  // the attribute of device g_pageable_dev
+bool host_addressable(void *p, double **dev) {
+  int d = 0;
+  if (cudaGetDevice(&d) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (d != g_pageable_dev) {
+    int v = 0;
+    g_pageable = cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccess, d) == cudaSuccess && v == 1;
+    g_pageable_dev = d;
+    cudaGetLastError();
+  }
+  if (g_pageable && g_host_link == 1) {
+    *dev = static_cast<double *>(p);
+    return true;
+  }
+  // registered (or cudaHostAlloc'd) memory and its device address
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeHost || !at.devicePointer) return false;
+  *dev = static_cast<double *>(at.devicePointer);
+  return true;
+}
+
+// the arrays of a fine-grained call, in or out: in one launch where the GPU
+// can address them all and none is so large that the copy engines are as fast
+// (see sbfs_sync_to_host), else one by one.  The host arrays are in use until
+// the call's last sync.  scalars: the pinned scalars and column coefficients
+// put_scalars left in small_host go with the arrays in.
+struct Xfer {
+  const array_t *a;
+  const Layout *l;
+  double *dev;
+};
+int transfer(Ctx &c, std::initializer_list<Xfer> list, bool in, bool scalars = false) {
+  HostFields fs;
+  int n = 0;
+  bool link = g_host_link && c.nc == 1 && (long)c.nx * c.ny <= 1L << 22 && list.size() + 2 <= kHostFields;
+  for (const Xfer &x : list) {
+    if (!layout_ok(*x.a, *x.l)) {
+      cudaStreamSynchronize(c.s);  // the arrays in
+      return fail("array layout does not match the reference's (nadds/size)");
+    }
+    HostField &f = fs.f[n++];
+    if (!link || !host_addressable(x.a->data, &f.h)) {
+      link = false;
+      break;
+    }
+    f.dev = x.dev;
+    f.row = (c.nx + x.l->ax0 + x.l->ax1) * x.l->nc;
+    f.rows = c.ny;
+    f.pitch = pitch_of(c, *x.l);
+    f.ay0 = x.l->ay0;
+    f.ay1 = x.l->ay1;
+    if (!in) make_present(x.a->data, sizeof(double) * f.row * (size_t)(f.rows + f.ay0 + f.ay1));
+  }
+  if (!link) {
+    for (const Xfer &x : list)
+      if (in ? h2d(c, *x.a, *x.l, x.dev) : d2h(c, const_cast<array_t &>(*x.a), *x.l, x.dev)) return 1;
+  }
+  if (scalars) {
+    double *const ct = c.b.coltab + (size_t)ct_cnewx(0) * c.g.ct, *const h = c.small_host;
+    const int nct = 2 * c.g.ct;
+    if (link) {
+      fs.f[n++] = HostField{h, c.b.scalars, kScalars, 1, (size_t)kScalars, 0, 0};
+      fs.f[n++] = HostField{h + kScalars, ct, nct, 1, (size_t)nct, 0, 0};
+    } else {
+      CK(cudaMemcpyAsync(c.b.scalars, h, sizeof(double) * kScalars, cudaMemcpyHostToDevice, c.s));
+      CK(cudaMemcpyAsync(ct, h + kScalars, sizeof(double) * nct, cudaMemcpyHostToDevice, c.s));
+    }
+  }
+  if (link) launch_host_fields(c.s, fs, n, in);
+  return 0;
+}
+
 int sync(Ctx &c) {
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c.s));
@@ -601,7 +682,8 @@ int build_ctx(Ctx *c, const domain_t *d, int nc) {
   b.scalars = tmp;
   b.status = reinterpret_cast<int *>(tmp + (size_t)kScalars * nc);
   if (dalloc(*c, &b.coltab, (size_t)3 * kColTabs * g.ct * nc)) return 1;
-  CK(cudaMallocHost(&c->small_host, sizeof(double) * ((size_t)kScalars * nc + nc / 2 + 2)));
+  // (with room for put_scalars' column coefficients of a single case)
+  CK(cudaMallocHost(&c->small_host, sizeof(double) * ((size_t)kScalars * nc + nc / 2 + 2 + 2 * (size_t)g.ct)));
   if (nc > 1) {
     void *q = nullptr;
     CK(cudaMalloc(&q, sizeof(Phys) * nc));
@@ -663,9 +745,9 @@ Ctx *get_ctx(const domain_t *d, const fluid_t *f, const interface_t *itf) {
 
 // scalars block for a fine-grained call: substage k of step size dt, and/or
 // explicit dt_old / dt_new in slot 0 (the same expressions as the step kernel)
-int put_scalars(Ctx &c, double dt, int k, double dt_old, double dt_new) {
+void put_scalars(Ctx &c, double dt, int k, double dt_old, double dt_new) {
   double *h = c.small_host;
-  for (int i = 0; i < kScalars; ++i) h[i] = 0.;
+  for (int i = 0; i < kScalars + 2 * c.g.ct; ++i) h[i] = 0.;
   h[0] = dt;
   if (k >= 0) {
     h[sc_adt(k)] = RK_A[k] * dt;
@@ -694,21 +776,14 @@ int put_scalars(Ctx &c, double dt, int k, double dt_old, double dt_new) {
     h[sc_rpy(0)] = c.ph.rref2 * h[sc_pay(0)];
     // the correction's per-column coefficients of slot 0, as k_decide_dt
     // writes them for the fused step
-    std::vector<double> ct(2 * (size_t)g.ct, 0.);
+    double *ct = h + kScalars;
     const double cop = h[sc_cold(0)] / h[sc_pax(0)];
     for (int I = 1; I <= c.nx + 1; ++I) {
       const double ih = 1. / c.hxxf[I - 1];
       ct[I] = h[sc_cnew(0)] * ih;
       ct[g.ct + I] = cop * ih;
     }
-    CK(cudaMemcpyAsync(c.b.coltab + (size_t)ct_cnewx(0) * g.ct, ct.data(), sizeof(double) * ct.size(),
-                       cudaMemcpyHostToDevice, c.s));
-    CK(cudaStreamSynchronize(c.s));  // ct dies here
   }
-  CK(cudaMemcpyAsync(c.b.scalars, h, sizeof(double) * kScalars, cudaMemcpyHostToDevice, c.s));
-  // h is reused by the next call: wait for the copy
-  CK(cudaStreamSynchronize(c.s));
-  return 0;
 }
 
 void swap_data(array_t &a, array_t &b) {
@@ -1877,36 +1952,6 @@ int sbfs_sync_to_host(const domain_t *d, fluid_t *f, interface_t *itf) {
   return sync(*c);
 }
 
-// host memory the GPU can address: any on a system whose GPU reads pageable
-// memory through the host page tables, else memory registered with CUDA
-int g_pageable = -1, g_pageable_dev = -1;  // the attribute of device g_pageable_dev
-bool host_addressable(void *p, double **dev) {
-  int d = 0;
-  if (cudaGetDevice(&d) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  if (d != g_pageable_dev) {
-    int v = 0;
-    g_pageable = cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccess, d) == cudaSuccess && v == 1;
-    g_pageable_dev = d;
-    cudaGetLastError();
-  }
-  if (g_pageable && g_host_link == 1) {
-    *dev = static_cast<double *>(p);
-    return true;
-  }
-  // registered (or cudaHostAlloc'd) memory and its device address
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  if (at.type != cudaMemoryTypeHost || !at.devicePointer) return false;
-  *dev = static_cast<double *>(at.devicePointer);
-  return true;
-}
-
 // fills the link table of case k for a strict-mode step, or says the step
 // cannot be host-linked (then the state goes through cudaMemcpy as before)
 bool link_tab_fill(Ctx &c, int k, fluid_t *f, interface_t *itf) {
@@ -2171,7 +2216,7 @@ int decide_dt(const domain_t *d, const fluid_t *f, const interface_t *itf, doubl
   if (!c) return 1;
   c->resident = false;
   state_touched(*c);
-  if (h2d(*c, f->ux, L_UX, c->b.ux) || h2d(*c, f->uy, L_UY, c->b.uy)) return 1;
+  if (transfer(*c, {{&f->ux, &L_UX, c->b.ux}, {&f->uy, &L_UY, c->b.uy}}, true)) return 1;
   launch_decide_dt(c->s, c->g, c->m, c->ph, c->b, c->b.ux, c->b.uy, c->dt_fixed, g_coef[0]);
   int status = 0;
   if (read_dt_status(*c, dt, &status)) return 1;
@@ -2189,9 +2234,9 @@ int fluid_compute_density(const domain_t *d, fluid_t *f, const interface_t *itf,
   if (!c) return 1;
   c->resident = false;
   state_touched(*c);
-  if (h2d(*c, itf->vof, L_VOF, c->b.vof)) return 1;
+  if (transfer(*c, {{&itf->vof, &L_VOF, c->b.vof}}, true)) return 1;
   launch_props(c->s, c->g, c->m, c->ph, c->b, true, false, false, c->b.den0);
-  if (d2h(*c, f->den[index], L_DEN, c->b.den0)) return 1;
+  if (transfer(*c, {{&f->den[index], &L_DEN, c->b.den0}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2201,9 +2246,9 @@ int fluid_compute_viscosity(const domain_t *d, fluid_t *f, const interface_t *it
   if (!c) return 1;
   c->resident = false;
   state_touched(*c);
-  if (h2d(*c, itf->vof, L_VOF, c->b.vof)) return 1;
+  if (transfer(*c, {{&itf->vof, &L_VOF, c->b.vof}}, true)) return 1;
   launch_props(c->s, c->g, c->m, c->ph, c->b, false, true, false, nullptr);
-  if (d2h(*c, f->visux, L_VISUX, c->b.visux) || d2h(*c, f->visuy, L_VISUY, c->b.visuy)) return 1;
+  if (transfer(*c, {{&f->visux, &L_VISUX, c->b.visux}, {&f->visuy, &L_VISUY, c->b.visuy}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2214,12 +2259,11 @@ int interface_compute_curvature_tensor(const domain_t *d, interface_t *itf) {
   c->resident = false;
   state_touched(*c);
   // cells outside the interface band keep their previous normal, as in the reference
-  if (h2d(*c, itf->vof, L_VOF, c->b.vof) || h2d(*c, itf->normal, L_NORMAL, c->b.normal)) return 1;
+  if (transfer(*c, {{&itf->vof, &L_VOF, c->b.vof}, {&itf->normal, &L_NORMAL, c->b.normal}}, true)) return 1;
   launch_props(c->s, c->g, c->m, c->ph, c->b, false, false, true, nullptr);
   launch_normal_curv(c->s, c->g, c->m, c->b, true, true, false);
-  if (d2h(*c, itf->dvof, L_DVOF, c->b.dvof) || d2h(*c, itf->normal, L_NORMAL, c->b.normal) ||
-      d2h(*c, itf->curv, L_CURV, c->b.curv))
-    return 1;
+  if (transfer(*c, {{&itf->dvof, &L_DVOF, c->b.dvof}, {&itf->normal, &L_NORMAL, c->b.normal},
+                    {&itf->curv, &L_CURV, c->b.curv}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2229,11 +2273,10 @@ int interface_compute_force(const domain_t *d, const fluid_t *f, interface_t *it
   if (!c) return 1;
   c->resident = false;
   state_touched(*c);
-  if (h2d(*c, f->den[0], L_DEN, c->b.den0) || h2d(*c, itf->vof, L_VOF, c->b.vof) ||
-      h2d(*c, itf->curv, L_CURV, c->b.curv))
-    return 1;
+  if (transfer(*c, {{&f->den[0], &L_DEN, c->b.den0}, {&itf->vof, &L_VOF, c->b.vof},
+                    {&itf->curv, &L_CURV, c->b.curv}}, true)) return 1;
   launch_flux_force(c->s, c->g, c->m, c->ph, c->b, c->b.ux, c->b.uy, c->b.den0, false, true, false);
-  if (d2h(*c, itf->ifrcx, L_IFRCX, c->b.ifrcx) || d2h(*c, itf->ifrcy, L_IFRCY, c->b.ifrcy)) return 1;
+  if (transfer(*c, {{&itf->ifrcx, &L_IFRCX, c->b.ifrcx}, {&itf->ifrcy, &L_IFRCY, c->b.ifrcy}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2247,16 +2290,14 @@ int interface_update_vof(const domain_t *d, const size_t rkstep, const double dt
   state_touched(*c);
   if (rkstep != 0) swap_data(itf->src[0], itf->src[1]);
   Bufs &b = c->b;
-  if (h2d(*c, f->ux, L_UX, b.ux) || h2d(*c, f->uy, L_UY, b.uy) || h2d(*c, itf->vof, L_VOF, b.vof) ||
-      h2d(*c, itf->normal, L_NORMAL, b.normal) || h2d(*c, itf->src[1], L_SRC, b.srcvof[1]))
-    return 1;
-  if (put_scalars(*c, dt, (int)rkstep, 0., 0.)) return 1;
+  put_scalars(*c, dt, (int)rkstep, 0., 0.);
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->vof, &L_VOF, b.vof},
+                    {&itf->normal, &L_NORMAL, b.normal}, {&itf->src[1], &L_SRC, b.srcvof[1]}}, true, true)) return 1;
   launch_flux_force(c->s, c->g, c->m, c->ph, b, b.ux, b.uy, b.den0, true, false, false);
   launch_vof_advance(c->s, c->g, c->m, c->ph, b, b.scalars, (int)rkstep, b.srcvof[0], b.srcvof[1], false, b.ux,
                      b.uy, nullptr);
-  if (d2h(*c, itf->fluxx, L_FLUXX, b.fluxx) || d2h(*c, itf->fluxy, L_FLUXY, b.fluxy) ||
-      d2h(*c, itf->src[0], L_SRC, b.srcvof[0]) || d2h(*c, itf->vof, L_VOF, b.vof))
-    return 1;
+  if (transfer(*c, {{&itf->fluxx, &L_FLUXX, b.fluxx}, {&itf->fluxy, &L_FLUXY, b.fluxy},
+                    {&itf->src[0], &L_SRC, b.srcvof[0]}, {&itf->vof, &L_VOF, b.vof}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2267,11 +2308,10 @@ int interface_compute_mass_flux(const domain_t *d, const fluid_t *f, interface_t
   c->resident = false;
   state_touched(*c);
   Bufs &b = c->b;
-  if (h2d(*c, f->ux, L_UX, b.ux) || h2d(*c, f->uy, L_UY, b.uy) || h2d(*c, itf->fluxx, L_FLUXX, b.fluxx) ||
-      h2d(*c, itf->fluxy, L_FLUXY, b.fluxy))
-    return 1;
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->fluxx, &L_FLUXX, b.fluxx},
+                    {&itf->fluxy, &L_FLUXY, b.fluxy}}, true)) return 1;
   launch_mass_flux_inplace(c->s, c->g, c->ph, b, b.ux, b.uy);
-  if (d2h(*c, itf->fluxx, L_FLUXX, b.fluxx) || d2h(*c, itf->fluxy, L_FLUXY, b.fluxy)) return 1;
+  if (transfer(*c, {{&itf->fluxx, &L_FLUXX, b.fluxx}, {&itf->fluxy, &L_FLUXY, b.fluxy}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2288,22 +2328,20 @@ int fluid_predict_field(const domain_t *d, const size_t rkstep, const double dt,
     swap_data(f->srcuy[0], f->srcuy[1]);
   }
   Bufs &b = c->b;
-  if (h2d(*c, f->ux, L_UX, b.ux) || h2d(*c, f->uy, L_UY, b.uy) || h2d(*c, f->visux, L_VISUX, b.visux) ||
-      h2d(*c, f->visuy, L_VISUY, b.visuy) || h2d(*c, itf->fluxx, L_FLUXX, b.mfluxx) ||
-      h2d(*c, itf->fluxy, L_FLUXY, b.mfluxy) || h2d(*c, f->p, L_P, b.p) || h2d(*c, itf->ifrcx, L_IFRCX, b.ifrcx) ||
-      h2d(*c, itf->ifrcy, L_IFRCY, b.ifrcy) || h2d(*c, f->den[0], L_DEN, b.den0) ||
-      h2d(*c, f->den[1], L_DEN, b.den1) || h2d(*c, f->srcux[1], L_SRCUX, b.srcux[1]) ||
-      h2d(*c, f->srcuy[1], L_SRCUY, b.srcuy[1]))
-    return 1;
-  if (put_scalars(*c, dt, (int)rkstep, 0., 0.)) return 1;
+  put_scalars(*c, dt, (int)rkstep, 0., 0.);
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&f->visux, &L_VISUX, b.visux},
+                    {&f->visuy, &L_VISUY, b.visuy}, {&itf->fluxx, &L_FLUXX, b.mfluxx},
+                    {&itf->fluxy, &L_FLUXY, b.mfluxy}, {&f->p, &L_P, b.p}, {&itf->ifrcx, &L_IFRCX, b.ifrcx},
+                    {&itf->ifrcy, &L_IFRCY, b.ifrcy}, {&f->den[0], &L_DEN, b.den0},
+                    {&f->den[1], &L_DEN, b.den1}, {&f->srcux[1], &L_SRCUX, b.srcux[1]},
+                    {&f->srcuy[1], &L_SRCUY, b.srcuy[1]}}, true, true)) return 1;
   launch_stress(c->s, c->g, c->m, b, b.ux, b.uy);
   launch_predict(c->s, c->g, c->m, c->ph, b, b.scalars, (int)rkstep, b.ux, b.uy, b.ux_star, b.uy_star, b.mfluxx,
                  b.mfluxy, b.den0, b.den1, b.srcux[0], b.srcux[1], b.srcux[2], b.srcuy[0], b.srcuy[1], b.srcuy[2]);
-  if (d2h(*c, f->txx, L_TXX, b.txx) || d2h(*c, f->txy, L_TXY, b.txy) || d2h(*c, f->tyy, L_TYY, b.tyy) ||
-      d2h(*c, f->srcux[0], L_SRCUX, b.srcux[0]) || d2h(*c, f->srcux[2], L_SRCUX, b.srcux[2]) ||
-      d2h(*c, f->srcuy[0], L_SRCUY, b.srcuy[0]) || d2h(*c, f->srcuy[2], L_SRCUY, b.srcuy[2]) ||
-      d2h(*c, f->ux, L_UX, b.ux_star) || d2h(*c, f->uy, L_UY, b.uy_star))
-    return 1;
+  if (transfer(*c, {{&f->txx, &L_TXX, b.txx}, {&f->txy, &L_TXY, b.txy}, {&f->tyy, &L_TYY, b.tyy},
+                    {&f->srcux[0], &L_SRCUX, b.srcux[0]}, {&f->srcux[2], &L_SRCUX, b.srcux[2]},
+                    {&f->srcuy[0], &L_SRCUY, b.srcuy[0]}, {&f->srcuy[2], &L_SRCUY, b.srcuy[2]},
+                    {&f->ux, &L_UX, b.ux_star}, {&f->uy, &L_UY, b.uy_star}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2314,13 +2352,12 @@ int fluid_compute_potential(const domain_t *d, const double dt_old, const double
   c->resident = false;
   state_touched(*c);
   Bufs &b = c->b;
-  if (h2d(*c, f->ux, L_UX, b.ux) || h2d(*c, f->uy, L_UY, b.uy) || h2d(*c, f->psi[0], L_P, b.psi0) ||
-      h2d(*c, f->den[1], L_DEN, b.den1))
-    return 1;
-  if (put_scalars(*c, 0., -1, dt_old, dt_new)) return 1;
+  put_scalars(*c, 0., -1, dt_old, dt_new);
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&f->psi[0], &L_P, b.psi0},
+                    {&f->den[1], &L_DEN, b.den1}}, true, true)) return 1;
   launch_face_factor(c->s, c->g, c->ph, b, b.den1, b.psi0);
   launch_poisson(c->s, c->g, b, b.scalars, 0, b.ux, b.uy, b.psi1);
-  if (d2h(*c, f->psi[1], L_P, b.psi1)) return 1;
+  if (transfer(*c, {{&f->psi[1], &L_P, b.psi1}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2331,13 +2368,12 @@ int fluid_correct_velocity(const domain_t *d, const double dt_old, const double 
   c->resident = false;
   state_touched(*c);
   Bufs &b = c->b;
-  if (h2d(*c, f->ux, L_UX, b.ux) || h2d(*c, f->uy, L_UY, b.uy) || h2d(*c, f->psi[0], L_P, b.psi0) ||
-      h2d(*c, f->psi[1], L_P, b.psi1) || h2d(*c, f->den[1], L_DEN, b.den1))
-    return 1;
-  if (put_scalars(*c, 0., -1, dt_old, dt_new)) return 1;
+  put_scalars(*c, 0., -1, dt_old, dt_new);
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&f->psi[0], &L_P, b.psi0},
+                    {&f->psi[1], &L_P, b.psi1}, {&f->den[1], &L_DEN, b.den1}}, true, true)) return 1;
   launch_face_factor(c->s, c->g, c->ph, b, b.den1, b.psi0);
   launch_correct(c->s, c->g, c->m, b, b.scalars, 0, b.ux, b.uy, b.psi1, false, false);
-  if (d2h(*c, f->ux, L_UX, b.ux) || d2h(*c, f->uy, L_UY, b.uy)) return 1;
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}}, false)) return 1;
   return sync(*c);
 }
 
@@ -2347,9 +2383,9 @@ int fluid_update_pressure(const domain_t *d, fluid_t *f) {
   if (!c) return 1;
   c->resident = false;
   state_touched(*c);
-  if (h2d(*c, f->p, L_P, c->b.p) || h2d(*c, f->psi[1], L_P, c->b.psi1)) return 1;
+  if (transfer(*c, {{&f->p, &L_P, c->b.p}, {&f->psi[1], &L_P, c->b.psi1}}, true)) return 1;
   launch_pressure(c->s, c->g, c->b, c->b.psi1);
-  if (d2h(*c, f->p, L_P, c->b.p)) return 1;
+  if (transfer(*c, {{&f->p, &L_P, c->b.p}}, false)) return 1;
   if (sync(*c)) return 1;
   swap_data(f->psi[0], f->psi[1]);
   return 0;

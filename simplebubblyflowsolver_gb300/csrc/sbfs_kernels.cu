@@ -2945,4 +2945,44 @@ void launch_host_rows(cudaStream_t s, const Grid &g, double *const *tab, bool in
     launch_pdl(k_host_rows<false>, grid, 256, 0, s, g, tab, a, b, c, nf, words, words_host, nwords);
 }
 
+// the same for the fine-grained entry points: field blockIdx.y of the list, a
+// launch instead of a copy-engine call per field and ghost row (300 x 256
+// curvature call, 6 MB over the link: 192 us with five copies and eight ghost
+// rows, 72 us)
+template <bool kIn>
+__global__ void __launch_bounds__(256) k_host_fields(const __grid_constant__ HostFields fs) {
+  pdl_entry();
+  const HostField &f = fs.f[blockIdx.y];
+  const int stride = gridDim.x * blockDim.x;
+  const int n = (kIn ? f.rows : f.rows + f.ay0 + f.ay1) * f.row;
+  for (int t0 = blockIdx.x * blockDim.x + threadIdx.x; t0 < n; t0 += 4 * stride) {
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = t0 + u * stride;
+      if (t >= n) break;
+      const int r = t / f.row, i = t - r * f.row;
+      v[u] = kIn ? f.h[(size_t)(r + f.ay0) * f.row + i] : f.dev[wrap(r - f.ay0 + 1, f.rows) * f.pitch + i];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = t0 + u * stride;
+      if (t >= n) break;
+      const int r = t / f.row, i = t - r * f.row;
+      if (kIn)
+        f.dev[r * f.pitch + i] = v[u];
+      else
+        f.h[t] = v[u];
+    }
+  }
+}
+
+void launch_host_fields(cudaStream_t s, const HostFields &fs, int n, bool in) {
+  const dim3 grid(std::max(16, 4 * 152 / n), n);
+  if (in)
+    launch_pdl(k_host_fields<true>, grid, 256, 0, s, fs);
+  else
+    launch_pdl(k_host_fields<false>, grid, 256, 0, s, fs);
+}
+
 }  // namespace sbfs

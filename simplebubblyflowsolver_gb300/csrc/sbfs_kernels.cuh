@@ -256,4 +256,18 @@ void launch_host_rows(cudaStream_t s, const Grid &g, double *const *tab, bool in
                       int width, HostRows c = HostRows{}, const double *words = nullptr, double *words_host = nullptr,
                       int nwords = 0);
 
+// host arrays <-> device fields of the fine-grained entry points, up to
+// kHostFields in one launch
+struct HostField {
+  double *h, *dev;
+  int row, rows;       // doubles a row, interior rows
+  size_t pitch;        // of the device rows
+  int ay0, ay1;        // host ghost rows
+};
+constexpr int kHostFields = 16;
+struct HostFields {
+  HostField f[kHostFields];
+};
+void launch_host_fields(cudaStream_t s, const HostFields &fs, int n, bool in);
+
 }  // namespace sbfs
