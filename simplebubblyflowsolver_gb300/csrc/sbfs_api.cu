@@ -644,6 +644,8 @@ int build_ctx(Ctx *c, const domain_t *d, int nc) {
   b.tiles = default_tiles(c->ny);
   b.tiles.tdm_g = tdm_warps_for(c->nx, c->ny, nc);
   b.tiles.tdm_mb = tdm_modes_for(c->nx, c->ny, nc, b.tiles.tdm_g);
+  // at two warps a system the pairs' clusters only while the pairs leave SMs idle
+  b.tiles.tdm_cl = b.tiles.tdm_g == 4 || (long)(c->ny / 4 + 1) * nc <= 152;
   double **scal[] = {&b.ux, &b.uy, &b.p, &b.psi0, &b.psi1, &b.vof, &b.ux_star, &b.uy_star, &b.den0, &b.den1,
                      &b.visux, &b.visuy, &b.txx, &b.txy, &b.tyy, &b.curv, &b.ifrcx, &b.ifrcy, &b.fluxx, &b.fluxy,
                      &b.mfluxx, &b.mfluxy, &b.srcux[0], &b.srcux[1], &b.srcux[2], &b.srcuy[0], &b.srcuy[1],

@@ -1602,39 +1602,89 @@ __device__ __forceinline__ void sweep(int L, Load load, Use use) {
     for (int u = 0; u < kAhead; ++u) c[u] = n[u];
   }
 }
-// forward from a zero carry, y_k = w_k r_k - v_k y_{k-1}; returns the last y
-template <bool AHEAD>
-__device__ __forceinline__ double tdm_forward(const Fp64 &f64, const double4_32a *__restrict__ f, size_t lanes, int L,
-                                              double *x) {
-  double t = 0.;
-  sweep<AHEAD, 1>(
-      L, [&](int k) { return make_double2(f[k * lanes].x, f[k * lanes].y); },
-      [&](int k, double2 c) {
-        t = fma(-c.y, t, f64.mul(c.x, x[k]));
-        x[k] = t;
-      });
-  return t;
-}
-// the forward solution's fix-up by P_k carry and the backward sweep from a
-// zero carry, x_k = y_k - v_k x_{k+1}; returns the first x
-template <bool AHEAD>
-__device__ __forceinline__ double tdm_backward(const double4_32a *__restrict__ f, size_t lanes, int L, double carry,
-                                               double *x) {
-  double u = 0.;
-  sweep<AHEAD, -1>(
-      L, [&](int k) { return make_double2(f[k * lanes].y, f[k * lanes].z); },
-      [&](int k, double2 c) {
-        u = fma(-c.x, u, fma(c.y, carry, x[k]));
-        x[k] = u;
-      });
-  return u;
-}
-// the backward solution's fix-up by Q_k next
-template <bool AHEAD>
-__device__ __forceinline__ void tdm_fix(const double4_32a *__restrict__ f, size_t lanes, int L, double next, double *x) {
-  sweep<AHEAD, 1>(
-      L, [&](int k) { return f[k * lanes].w; }, [&](int k, double q) { x[k] = fma(q, next, x[k]); });
-}
+// Chunk<INT> holds a lane's rows and factors between the sweeps.  Small
+// launches (not INT) with chunks of up to kReg rows keep both in registers,
+// the factors loaded before the split's rows arrive: three trips to L2 and
+// back, and the rows' to shared memory, leave the chain (k_poisson_tdm on
+// 256 x 128 11.8 -> 9.0 us with the pairs' clusters at two
+// warps a system, on 509 x 256 14.0 -> 11.4 us).
+template <bool INT>
+struct Chunk {
+  static constexpr int kReg = INT ? 1 : 4;
+  const Fp64 &f64;
+  const double4_32a *__restrict__ f;
+  size_t lanes;
+  int L;
+  double *x;
+  bool reg;
+  double4_32a c[kReg];
+  double r[kReg];
+  __device__ __forceinline__ Chunk(const Fp64 &f_, const double4_32a *fac, size_t lanes_, int L_, double *x_, bool act)
+      : f64(f_), f(fac), lanes(lanes_), L(L_), x(x_), reg(!INT && L_ <= kReg) {
+    if (reg && act) {
+#pragma unroll
+      for (int k = 0; k < kReg; ++k)
+        if (k < L) c[k] = f[k * lanes];
+    }
+  }
+  // forward from a zero carry, y_k = w_k r_k - v_k y_{k-1}; returns the last y
+  __device__ __forceinline__ double forward() {
+    double t = 0.;
+    if (reg) {
+#pragma unroll
+      for (int k = 0; k < kReg; ++k)
+        if (k < L) t = r[k] = fma(-c[k].y, t, f64.mul(c[k].x, x[k]));
+      return t;
+    }
+    sweep<INT, 1>(
+        L, [&](int k) { return make_double2(f[k * lanes].x, f[k * lanes].y); },
+        [&](int k, double2 q) {
+          t = fma(-q.y, t, f64.mul(q.x, x[k]));
+          x[k] = t;
+        });
+    return t;
+  }
+  // the forward solution's fix-up by P_k carry and the backward sweep from a
+  // zero carry, x_k = y_k - v_k x_{k+1}; returns the first x
+  __device__ __forceinline__ double backward(double carry) {
+    double u = 0.;
+    if (reg) {
+#pragma unroll
+      for (int k = kReg - 1; k >= 0; --k)
+        if (k < L) u = r[k] = fma(-c[k].y, u, fma(c[k].z, carry, r[k]));
+      return u;
+    }
+    sweep<INT, -1>(
+        L, [&](int k) { return make_double2(f[k * lanes].y, f[k * lanes].z); },
+        [&](int k, double2 q) {
+          u = fma(-q.x, u, fma(q.y, carry, x[k]));
+          x[k] = u;
+        });
+    return u;
+  }
+  // the backward solution's fix-up by Q_k next
+  __device__ __forceinline__ void fix(double next) {
+    if (reg) {
+#pragma unroll
+      for (int k = 0; k < kReg; ++k)
+        if (k < L) x[k] = fma(c[k].w, next, r[k]);
+      return;
+    }
+    sweep<INT, 1>(
+        L, [&](int k) { return f[k * lanes].w; }, [&](int k, double q) { x[k] = fma(q, next, x[k]); });
+  }
+  // P of the last row and Q of the first
+  __device__ __forceinline__ double last_p() const {
+    if (reg) {
+      double v = c[0].z;
+#pragma unroll
+      for (int k = 1; k < kReg; ++k) v = k < L ? c[k].z : v;
+      return v;
+    }
+    return f[(size_t)(L - 1) * lanes].z;
+  }
+  __device__ __forceinline__ double first_q() const { return reg ? c[0].w : f[0].w; }
+};
 
 // Tridiagonal solves along x, one per real system (y wavenumber m, real or
 // imaginary part), one warp per system.  The pivots of the constant operator
@@ -1668,6 +1718,16 @@ __global__ void __launch_bounds__(512)
   double *sm = kGlobalStage ? stage + ((size_t)blockIdx.z * gridDim.x + blockIdx.x) * 4 * PB * sys_len
                             : reinterpret_cast<double *>(smem_d2);
   double2 *sp = spec + (size_t)blockIdx.z * g.css;
+  // warp -> system (4 per pair) and its part sub of G; chunk j of the
+  // system = this lane's L rows
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sys = warp / G, sub = warp - sys * G, j = sub * 32 + lane;
+  const bool act = sys < 4 * np;  // warp-uniform
+  const int pq = p0 + (sys >> 2);
+  const int m = (sys & 2) ? M - pq : pq;  // the wavenumber of this system
+  double *x = sm + sys * sys_len + j * S;
+  const double4_32a *f = fac + (size_t)m * L * lanes + j;
+  Chunk<INT> ch(f64, f, lanes, L, x, act);
   // ---- load the packed transform of both wavenumbers of each pair, split
   // it (real-to-complex, times 2: X_m = (z_m + conj z_{M-m}) + w^m (-i)(z_m -
   // conj z_{M-m})) into four planar systems: X_p re, im, X_{M-p} re, im
@@ -1702,20 +1762,11 @@ __global__ void __launch_bounds__(512)
     }
   }
   __syncthreads();
-  // warp -> system (4 per pair) and its part sub of G; chunk j of the
-  // system = this lane's L rows
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sys = warp / G, sub = warp - sys * G, j = sub * 32 + lane;
-  const bool act = sys < 4 * np;  // warp-uniform
-  const int pq = p0 + (sys >> 2);
-  const int m = (sys & 2) ? M - pq : pq;  // the wavenumber of this system
-  double *x = sm + sys * sys_len + j * S;
-  const double4_32a *f = fac + (size_t)m * L * lanes + j;
   double T = 0., B = 0.;
   if (act) {
     // forward, local from a zero carry
-    T = tdm_forward<INT>(f64, f, lanes, L, x);
-    B = f[(size_t)(L - 1) * lanes].z;
+    T = ch.forward();
+    B = ch.last_p();
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const double Tp = __shfl_up_sync(0xffffffffu, T, d), Bp = __shfl_up_sync(0xffffffffu, B, d);
@@ -1742,8 +1793,8 @@ __global__ void __launch_bounds__(512)
     const double Tu = __shfl_up_sync(0xffffffffu, T, 1), Bu = __shfl_up_sync(0xffffffffu, B, 1);
     const double carry = lane == 0 ? Cin : fma(Bu, Cin, Tu);
     // fix up the forward solution, then the backward sweep from a zero carry
-    Sx = tdm_backward<INT>(f, lanes, L, carry, x);
-    Cc = f[0].w;
+    Sx = ch.backward(carry);
+    Cc = ch.first_q();
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const double Sp = __shfl_down_sync(0xffffffffu, Sx, d), Cp = __shfl_down_sync(0xffffffffu, Cc, d);
@@ -1771,7 +1822,7 @@ __global__ void __launch_bounds__(512)
   if (act) {
     const double Sd = __shfl_down_sync(0xffffffffu, Sx, 1), Cd = __shfl_down_sync(0xffffffffu, Cc, 1);
     const double next = lane == 31 ? Din : fma(Cd, Din, Sd);
-    tdm_fix<INT>(f, lanes, L, next, x);
+    ch.fix(next);
     if (gauge) {
       for (int k = 0; k < L; ++k) acc += (j * L + k < nx) ? x[k] : 0.;
 #pragma unroll
@@ -1818,9 +1869,8 @@ __global__ void __launch_bounds__(512)
 // the other CTAs come through distributed shared memory and are combined in
 // the order k_poisson_tdm<false> combines its warps' at G = 4, so both give
 // the same bits.  L = tdm_chunk(nx, 4), S = L | 1; fac is the G = 4 table.
-constexpr int kTdmCluster = 4;
-template <bool INT>
-__global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
+template <bool INT, int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(128)
     k_poisson_tdm_cl(Grid g, int L, int S, const double4_32a *__restrict__ fac, const double2 *__restrict__ tw,
                      double2 *__restrict__ spec) {
   pdl_entry();
@@ -1832,10 +1882,16 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
   const Fp64 f64(blockIdx.x + threadIdx.x);
   const int nx = g.nx, M = g.ny / 2, M1 = M + 1;
   const int rank = (int)cl.block_rank();
-  const int p = (int)blockIdx.x / kTdmCluster;  // the pair (p, M - p), p = 0 .. M/2
+  const int p = (int)blockIdx.x / CL;  // the pair (p, M - p), p = 0 .. M/2
   const int rows = 32 * L, r0 = rank * rows;   // this CTA's rows r0 .. r0 + rows - 1
   const int sys_len = 32 * S;
   double2 *sp = spec + (size_t)blockIdx.z * g.css;
+  const int sys = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lanes = 32 * CL, j = rank * 32 + lane;  // chunk of the system
+  const int m = (sys & 2) ? M - p : p;
+  double *x = smem_cl + sys * sys_len + lane * S;
+  const double4_32a *f = fac + (size_t)m * L * lanes + j;
+  Chunk<INT> ch(f64, f, lanes, L, x, true);
   // ---- load and split (as in k_poisson_tdm), this CTA's rows
   for (int t = threadIdx.x; t < rows; t += blockDim.x) {
     const int i = r0 + t;
@@ -1853,15 +1909,10 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
     smem_cl[3 * sys_len + at] = xbv.y;
   }
   __syncthreads();
-  const int sys = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int lanes = 32 * kTdmCluster, j = rank * 32 + lane;  // chunk of the system
-  const int m = (sys & 2) ? M - p : p;
-  double *x = smem_cl + sys * sys_len + lane * S;
-  const double4_32a *f = fac + (size_t)m * L * lanes + j;
   double T, B;
   {
-    T = tdm_forward<INT>(f64, f, lanes, L, x);
-    B = f[(size_t)(L - 1) * lanes].z;
+    T = ch.forward();
+    B = ch.last_p();
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const double Tp = __shfl_up_sync(0xffffffffu, T, d), Bp = __shfl_up_sync(0xffffffffu, B, d);
@@ -1885,8 +1936,8 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
   {
     const double Tu = __shfl_up_sync(0xffffffffu, T, 1), Bu = __shfl_up_sync(0xffffffffu, B, 1);
     const double carry = lane == 0 ? Cin : fma(Bu, Cin, Tu);
-    Sx = tdm_backward<INT>(f, lanes, L, carry, x);
-    Cc = f[0].w;
+    Sx = ch.backward(carry);
+    Cc = ch.first_q();
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const double Sp = __shfl_down_sync(0xffffffffu, Sx, d), Cp = __shfl_down_sync(0xffffffffu, Cc, d);
@@ -1902,14 +1953,14 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
   }
   cl.sync();
   double Din = 0.;
-  for (int q = kTdmCluster - 1; q > rank; --q) {
+  for (int q = CL - 1; q > rank; --q) {
     const double *o = cl.map_shared_rank(&xb[sys][0], q);
     Din = fma(o[1], Din, o[0]);
   }
   {
     const double Sd = __shfl_down_sync(0xffffffffu, Sx, 1), Cd = __shfl_down_sync(0xffffffffu, Cc, 1);
     const double next = lane == 31 ? Din : fma(Cd, Din, Sd);
-    tdm_fix<INT>(f, lanes, L, next, x);
+    ch.fix(next);
   }
   // the singular mode m = 0 (systems 0, 1 of pair 0): zero mean over x,
   // imaginary part 0 (p is the same on the whole cluster)
@@ -1925,7 +1976,7 @@ __global__ void __cluster_dims__(kTdmCluster, 1, 1) __launch_bounds__(128)
     cl.sync();
     if (gauge) {
       acc = 0.;
-      for (int q = 0; q < kTdmCluster; ++q) acc += *cl.map_shared_rank(&xg[sys], q);
+      for (int q = 0; q < CL; ++q) acc += *cl.map_shared_rank(&xg[sys], q);
       const double mean = (sys & 1) ? 0. : acc / nx;
       for (int k = 0; k < L; ++k) x[k] = (sys & 1) ? 0. : x[k] - mean;
     }
@@ -2562,8 +2613,8 @@ cudaError_t configure_kernels() {
   const int big = 227 * 1024;
   e = configure_fft<1, 2, 4, 8>(big);
   if (e != cudaSuccess) return e;
-  return allow_smem((int)kTdmSmemMax, k_poisson_tdm<false, false>, k_poisson_tdm<false, true>, k_poisson_tdm_cl<false>,
-                    k_poisson_tdm_cl<true>);
+  return allow_smem((int)kTdmSmemMax, k_poisson_tdm<false, false>, k_poisson_tdm<false, true>, k_poisson_tdm_cl<false, 4>,
+                    k_poisson_tdm_cl<true, 4>, k_poisson_tdm_cl<false, 2>, k_poisson_tdm_cl<true, 2>);
 }
 
 void launch_props(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const Bufs &b, bool den, bool vis,
@@ -2771,18 +2822,20 @@ void launch_poisson_fwd_q(cudaStream_t s, const Grid &g, const Bufs &b, const do
 int g_tdm_cluster = 1;
 
 bool tdm_uses_cluster(const Tiles &t, int nx) {
-  return g_tdm_cluster && t.tdm_cl && t.tdm_g == 4 &&
-         4 * 32 * (size_t)tdm_stride(nx, 4) * sizeof(double) <= kTdmSmemMax;
+  return g_tdm_cluster && t.tdm_cl && t.tdm_g >= 2 &&
+         4 * 32 * (size_t)tdm_stride(nx, t.tdm_g) * sizeof(double) <= kTdmSmemMax;
 }
 
 void launch_poisson_tdm(cudaStream_t s, const Grid &g, const Bufs &b) {
   const int G = b.tiles.tdm_g > 0 ? b.tiles.tdm_g : 1;
   const int pairs = g.ny / 4 + 1;
   const double4_32a *fac = reinterpret_cast<const double4_32a *>(b.tdm_fac[tdm_group_index(G)]);
-  if (tdm_uses_cluster(b.tiles, g.nx)) {  // four CTAs per pair, four warps each
-    const int L = tdm_chunk(g.nx, 4), S = tdm_stride(g.nx, 4);
-    launch_pdl(integer_transforms(g) ? k_poisson_tdm_cl<true> : k_poisson_tdm_cl<false>, dim3(kTdmCluster * pairs, 1, g.nc), 128, 4 * 32 * (size_t)S * sizeof(double), s, g,
-               L, S, fac, b.twiddle, b.spec);
+  if (tdm_uses_cluster(b.tiles, g.nx)) {  // G CTAs per pair, four warps each
+    const int L = tdm_chunk(g.nx, G), S = tdm_stride(g.nx, G);
+    auto kern = G == 4 ? k_poisson_tdm_cl<false, 4> : k_poisson_tdm_cl<false, 2>;
+    if (integer_transforms(g)) kern = G == 4 ? k_poisson_tdm_cl<true, 4> : k_poisson_tdm_cl<true, 2>;
+    launch_pdl(kern, dim3(G * pairs, 1, g.nc), 128, 4 * 32 * (size_t)S * sizeof(double), s, g, L, S, fac, b.twiddle,
+               b.spec);
     return;
   }
   if (tdm_global_stage(g.nx, G)) {  // one pair per block, staged in b.tdm_stage

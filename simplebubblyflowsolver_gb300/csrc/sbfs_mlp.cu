@@ -418,7 +418,7 @@ __global__ void k_mlp_adam(float *__restrict__ p, const float *__restrict__ gblk
 // tiles' gradients and the Adam step, of which every block does a share, and
 // between that and the next batch's weights.  The same sums in the same order
 // as k_mlp_grad and k_mlp_adam, whose two launches a batch cost more than the
-// batch: an epoch of 64 batches of 1024 rows 1240 us in launches, 700 us here.
+// batch: an epoch of 64 batches of 1024 rows 1240 us in launches, 680 us here.
 // (Its step: 1 us for the weights, 5 us for the tile, 4 us for the barriers
 // and the Adam step.)  The next batch's rows load during the Adam step.
 constexpr int kEpochBlocks = 8, kEpochSteps = 128, kEpochTiles = 16;
