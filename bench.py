@@ -432,14 +432,15 @@ def roofline_of(prof, lib, cells, grid, step_ms):
     out = {"bound": "fp64", "kernel": dom, "achieved": None, "peak": round(fp64_peak, 1), "unit": "GFLOP/s",
            "frac": None, "traffic": tr["traffic"] if tr else None, "fp64_flop_per_launch": None,
            "peak_source": "measured live: FP64 FMA loop on this GPU (sbfs_measure_fp64_peak), of measured",
-           "flop_source": "ncu DADD + DMUL + 2 DFMA thread instructions on this grid (profiles/kernel_traffic.txt)",
+           "flop_source": "the algorithm's FP64 operations on this grid (ncu DADD + DMUL + 2 DFMA with all of them on the "
+                          "FP64 unit; part now runs on the integer pipes, bit for bit; profiles/kernel_traffic.txt)",
            "avg_launch_ms": round(dom_avg_s * 1e3, 4), "share": round(dom_ms / total, 4), "hbm": hbm,
            "shares": {k: round(v[0] / total, 4) for k, v in sorted(prof.items(), key=lambda kv: -kv[1][0])}}
     if tr:
         ach = tr["fp64_flop"] / dom_avg_s / 1e9
         out.update(achieved=round(ach, 1), frac=round(ach / fp64_peak, 4), fp64_flop_per_launch=tr["fp64_flop"])
         if tr.get("fp64_inst"):
-            # DADD and DMUL take an FP64 issue slot like an FMA: the fraction of
+            # instructions the FP64 unit runs (not those on the integer pipes): the fraction of
             # the pipe's instruction rate (peak / 2 FMA per second) the kernel issues
             out["issue_frac"] = round(tr["fp64_inst"] / dom_avg_s / 1e9 / (fp64_peak / 2.0), 4)
     # step-wide: every launch class of a step (decide_dt once, the rest three times)
@@ -454,9 +455,9 @@ def roofline_of(prof, lib, cells, grid, step_ms):
                        "fused_hbm_frac": round(720.0 * cells / (step_ms / 1e3) / 1e9 / hbm_peak, 4),
                        "dram_bytes_per_cell_step": round(sum(traffic[k]["traffic"] * n for k, n in per.items())
                                                          / cells, 1),
-                       "note": "fp64_frac: the step's FP64 flops (ncu, FMA = 2) over its device time and the live "
-                               "FMA rate; fp64_issue_frac: its FP64 instructions (an FMA, DADD or DMUL each takes "
-                               "one issue slot) over the FMA instruction rate; fused_hbm_frac: 720 B per cell-step "
+                       "note": "fp64_frac: the algorithm's FP64 flops (FMA = 2) over the step's device time and the "
+                               "live FMA rate; fp64_issue_frac: the instructions the FP64 unit runs (the rest is on "
+                               "the integer pipes) over the FMA instruction rate; fused_hbm_frac: 720 B per cell-step "
                                "(the fused-minimum dataflow) over the measured HBM bandwidth"}
     return out
 
@@ -523,7 +524,7 @@ def metric_arms(args, lib):
             "steps": steps, "train_s": round(train_s, 1), "train_final_loss": hist[-1],
             "training": dict(tstats, note="the closure's training on the GPU: data generation (exact-area and "
                              "solver-advected circles, relaxed drops) and the Adam epochs (1024-row batches, "
-                             "one gradient and one update launch each); rows_per_s = epochs x rows / training s"),
+                             "up to 128 of them a launch); rows_per_s = epochs x rows / training s"),
             "static_drop_64": dict(drop, steps=nsteps, note="kappa: rms relative error of the curvature the "
                                    "last substage used in the interface cells (exact 1/r = 4); umax_mean: "
                                    "max |u| sampled 20 times over the run, averaged (parasitic currents); "
