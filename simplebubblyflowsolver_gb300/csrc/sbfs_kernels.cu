@@ -4,7 +4,9 @@
 // multiply-adds per second, measured) bounds this solver, not HBM (a first
 // version of the momentum kernel ran its FP64 pipe at 86% of peak with DRAM
 // at 9%), so every kernel is written to spend as few FP64 instructions per
-// cell as the discretisation allows:
+// cell as the discretisation allows, and on large launches half of the sums
+// and products of the largest kernels run on the integer pipes beside it, bit
+// for bit (sbfs_intfp.cuh):
 //   * the reference's metric factors are folded into one coefficient per
 //     column or per grid (see sbfs_device.cuh), and constant factors such
 //     as the 0.5 of face averages are folded into those coefficients;
@@ -113,8 +115,10 @@ __global__ void __launch_bounds__(BX *BY) k_props(Grid g, Metrics m, Phys ph0, c
   // the interface cell and face counts k_curv_list adds to start at zero (a
   // memset between the two would end their programmatic dependency: 5 us on
   // the side stream of a 64 x 64 step)
-  if (counts && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y < 2)
-    counts[threadIdx.y * g.nc + blockIdx.z] = 0;
+  if (counts && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+    counts[blockIdx.z] = 0;
+    counts[g.nc + blockIdx.z] = 0;
+  }
   const Phys ph = zphys(g, ph0);
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
   const int J = blockIdx.y * blockDim.y + threadIdx.y + 1;
