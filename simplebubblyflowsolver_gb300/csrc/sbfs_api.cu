@@ -201,34 +201,26 @@ size_t case_off(const Ctx &c, const Layout &l) {
   return (size_t)c.kcase * (l.nc == 1 ? c.g.cs1 : (l.nc == 2 ? c.g.cs2 : c.g.cs3));
 }
 
-// Pages of a host array that the GPU is about to write, and that the program
-// has not touched yet (a fresh calloc), are made present from the CPU: a copy
-// that finds them missing faults them in one by one over the CPU-GPU link.
-// 67 MB into untouched pages of 64 KB: 55.8 ms, or 2.1 ms here (one thread; 2
-// to 16 threads 1.4 to 2.2) and 0.5 ms for the copy.  The page in the middle
-// tells whether to look at the others; below 4 MB that look would be a part
-// of the copy's own time that shows (1 to 2 us).  Contents do not change, and
-// a failure only leaves the faults to the copy.
-void make_present(void *p, size_t bytes) {
-#ifdef MADV_POPULATE_WRITE
+// Pages of a large host array that the GPU is about to read or write are made
+// present from the CPU: a copy that finds some missing (a fresh calloc) or
+// unmapped (the kernel's NUMA balancing takes them away from time to time)
+// faults them in one by one over the CPU-GPU link.  67 MB into untouched pages
+// of 64 KB: 55.8 ms, or 2.1 ms here (one thread; 2 to 16 threads 1.4 to 2.2)
+// and 0.5 ms for the copy; 0.26 ms where all are present.  Segments on a
+// 4096 x 2048 grid, 39 ms each: two in five took 50 to 120 ms without.  Below
+// 4 MB the walk would be a part of the copy's own time that shows.  Contents do
+// not change, and a failure only leaves the faults to the copy.
+void make_present(const void *p, size_t bytes, bool write) {
+#if defined(MADV_POPULATE_READ) && defined(MADV_POPULATE_WRITE)
   static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
   if (bytes < (size_t)4 << 20) return;
   const uintptr_t lo = (uintptr_t)p & ~(uintptr_t)(page - 1);
   const uintptr_t hi = ((uintptr_t)p + bytes + page - 1) & ~(uintptr_t)(page - 1);
-  const size_t n = (hi - lo) / page;
-  unsigned char mid = 0;
-  if (mincore(reinterpret_cast<void *>(lo + n / 2 * page), page, &mid) != 0 || (mid & 1)) return;
-  std::vector<unsigned char> in(n);
-  if (mincore(reinterpret_cast<void *>(lo), hi - lo, in.data()) != 0) return;
-  for (size_t a = 0; a < n;) {
-    size_t b = a;
-    while (b < n && (in[b] & 1) == (in[a] & 1)) ++b;
-    if (!(in[a] & 1)) madvise(reinterpret_cast<void *>(lo + a * page), (b - a) * page, MADV_POPULATE_WRITE);
-    a = b;
-  }
+  madvise(reinterpret_cast<void *>(lo), hi - lo, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ);
 #else
   (void)p;
   (void)bytes;
+  (void)write;
 #endif
 }
 
@@ -237,6 +229,7 @@ int h2d(Ctx &c, const array_t &a, const Layout &l, double *dev) {
   if (!layout_ok(a, l)) return fail("array layout does not match the reference's (nadds/size)");
   const size_t row = (size_t)(c.nx + l.ax0 + l.ax1) * l.nc;
   const double *src = static_cast<const double *>(a.data) + (size_t)l.ay0 * row;
+  make_present(src, sizeof(double) * row * (size_t)c.ny, false);
   dev += case_off(c, l);
   CK(cudaMemcpy2DAsync(dev, sizeof(double) * pitch_of(c, l), src, sizeof(double) * row, sizeof(double) * row, c.ny,
                        cudaMemcpyHostToDevice, c.s));
@@ -249,7 +242,7 @@ int d2h(Ctx &c, array_t &a, const Layout &l, const double *dev) {
   const size_t row = (size_t)(c.nx + l.ax0 + l.ax1) * l.nc;
   const size_t pitch = sizeof(double) * pitch_of(c, l);
   double *dst = static_cast<double *>(a.data);
-  make_present(dst, sizeof(double) * row * (size_t)(c.ny + l.ay0 + l.ay1));
+  make_present(dst, sizeof(double) * row * (size_t)(c.ny + l.ay0 + l.ay1), true);
   dev += case_off(c, l);
   CK(cudaMemcpy2DAsync(dst + (size_t)l.ay0 * row, sizeof(double) * row, dev, pitch, sizeof(double) * row, c.ny,
                        cudaMemcpyDeviceToHost, c.s));
@@ -324,7 +317,7 @@ int transfer(Ctx &c, std::initializer_list<Xfer> list, bool in, bool scalars = f
     f.pitch = pitch_of(c, *x.l);
     f.ay0 = x.l->ay0;
     f.ay1 = x.l->ay1;
-    if (!in) make_present(x.a->data, sizeof(double) * f.row * (size_t)(f.rows + f.ay0 + f.ay1));
+    make_present(x.a->data, sizeof(double) * f.row * (size_t)(f.rows + f.ay0 + f.ay1), !in);
   }
   if (!link) {
     for (const Xfer &x : list)
@@ -1971,7 +1964,7 @@ bool link_tab_fill(Ctx &c, int k, fluid_t *f, interface_t *itf) {
     // other arrays than the step before (whose psi arrays come swapped)
     if (q >= HL_UX_OUT && tab[q] != prev && tab[q] != psi_prev[0] && tab[q] != psi_prev[1])
       make_present(arr[q]->data, sizeof(double) * (c.nx + lay[q]->ax0 + lay[q]->ax1) *
-                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1));
+                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1), true);
   }
   if (c.nc == 1 && (c.link_host != c.link_prev || c.link_epoch != g_reg_epoch)) {
     // page-locked or pageable: the copy engines move them differently, and a
@@ -2009,7 +2002,8 @@ bool link_download(Ctx &c, int n, fluid_t *const *f, interface_t *const *itf, co
           !host_addressable(arr[q]->data, &c.link_tab[(size_t)k * kLinkSlots + slot[q]]))
         return false;
       make_present(arr[q]->data, sizeof(double) * (c.nx + lay[q]->ax0 + lay[q]->ax1) *
-                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1));
+                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1),
+                   true);
     }
   }
   for (int q = 0; q < kOut; q += 3)
