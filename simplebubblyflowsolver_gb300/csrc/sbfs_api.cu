@@ -260,7 +260,9 @@ int d2h(Ctx &c, array_t &a, const Layout &l, const double *dev) {
 // host memory the GPU can address: any on a system whose GPU reads pageable
 // memory through the host page tables, else memory registered with CUDA
 int g_pageable = -1, g_pageable_dev = -1;  // the attribute of device g_pageable_dev
+// (the copy kernels move doubles: an array off their boundaries is left to the copy engines)
 bool host_addressable(void *p, double **dev) {
+  if (reinterpret_cast<uintptr_t>(p) % sizeof(double) != 0) return false;
   int d = 0;
   if (cudaGetDevice(&d) != cudaSuccess) {
     cudaGetLastError();
