@@ -201,22 +201,42 @@ size_t case_off(const Ctx &c, const Layout &l) {
   return (size_t)c.kcase * (l.nc == 1 ? c.g.cs1 : (l.nc == 2 ? c.g.cs2 : c.g.cs3));
 }
 
-// Pages of a large host array that the GPU is about to read or write are made
-// present from the CPU: a copy that finds some missing (a fresh calloc) or
-// unmapped (the kernel's NUMA balancing takes them away from time to time)
-// faults them in one by one over the CPU-GPU link.  67 MB into untouched pages
-// of 64 KB: 55.8 ms, or 2.1 ms here (one thread; 2 to 16 threads 1.4 to 2.2)
-// and 0.5 ms for the copy; 0.26 ms where all are present.  Segments on a
-// 4096 x 2048 grid, 39 ms each: two in five took 50 to 120 ms without.  Below
-// 4 MB the walk would be a part of the copy's own time that shows.  Contents do
-// not change, and a failure only leaves the faults to the copy.
+// Pages that a large host array does not have yet (a fresh calloc) are made
+// present from the CPU before the GPU reads or writes it: a copy that finds
+// them missing faults them in one by one over the CPU-GPU link (67 MB of 64 KB
+// pages: 55.8 ms, or 2.1 ms here and 0.5 ms for the copy; 2 to 16 threads 1.4
+// to 2.2).  mincore tells which are missing: its look at the first, middle and
+// last page takes 0.4 us each, and decides whether to look at all (3 us for 67
+// MB).  To populate without looking walks the pages of every array at every
+// copy, page-locked ones too: a download of a 4096 x 2048 state 2.46 ms
+// instead of 2.32, a step with every array synchronised on 2048 x 1024 5.97
+// instead of 5.78.  Below 4 MB even the look would show.  Pages that are
+// present and all the same fault when the GPU comes to them (the 4096 x 2048
+// state between two segments, at times) are not helped by this.
+// write: the call writes the array, so its pages must not be the shared page
+// of zeros that a read maps.  Contents do not change, and a failure only
+// leaves the faults to the copy.
 void make_present(const void *p, size_t bytes, bool write) {
 #if defined(MADV_POPULATE_READ) && defined(MADV_POPULATE_WRITE)
   static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
   if (bytes < (size_t)4 << 20) return;
   const uintptr_t lo = (uintptr_t)p & ~(uintptr_t)(page - 1);
   const uintptr_t hi = ((uintptr_t)p + bytes + page - 1) & ~(uintptr_t)(page - 1);
-  madvise(reinterpret_cast<void *>(lo), hi - lo, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ);
+  unsigned char in[1024];
+  bool missing = false;
+  for (uintptr_t at : {lo, lo + (hi - lo) / page / 2 * page, hi - page}) {
+    if (mincore(reinterpret_cast<void *>(at), page, in) != 0) return;
+    missing |= !(in[0] & 1);
+  }
+  for (uintptr_t at = lo; missing && at < hi; at += sizeof(in) * page) {
+    const size_t n = std::min(sizeof(in), (size_t)(hi - at) / page);
+    if (mincore(reinterpret_cast<void *>(at), n * page, in) != 0) return;
+    for (size_t a = 0, b = 0; a < n; a = b) {
+      while (b < n && (in[b] & 1) == (in[a] & 1)) ++b;
+      if (!(in[a] & 1))
+        madvise(reinterpret_cast<void *>(at + a * page), (b - a) * page, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ);
+    }
+  }
 #else
   (void)p;
   (void)bytes;
@@ -224,12 +244,12 @@ void make_present(const void *p, size_t bytes, bool write) {
 #endif
 }
 
-// host array (reference layout, rows J = 1 - ay0 .. ny + ay1) -> device rows J = 1..ny
-int h2d(Ctx &c, const array_t &a, const Layout &l, double *dev) {
+// host array (reference layout, rows J = 1 - ay0 .. ny + ay1) -> device rows J = 1..ny; back: it is written later
+int h2d(Ctx &c, const array_t &a, const Layout &l, double *dev, bool back = false) {
   if (!layout_ok(a, l)) return fail("array layout does not match the reference's (nadds/size)");
   const size_t row = (size_t)(c.nx + l.ax0 + l.ax1) * l.nc;
   const double *src = static_cast<const double *>(a.data) + (size_t)l.ay0 * row;
-  make_present(src, sizeof(double) * row * (size_t)c.ny, false);
+  make_present(src, sizeof(double) * row * (size_t)c.ny, back);
   dev += case_off(c, l);
   CK(cudaMemcpy2DAsync(dev, sizeof(double) * pitch_of(c, l), src, sizeof(double) * row, sizeof(double) * row, c.ny,
                        cudaMemcpyHostToDevice, c.s));
@@ -298,6 +318,7 @@ struct Xfer {
   const array_t *a;
   const Layout *l;
   double *dev;
+  bool back = false;  // of an array in: the call writes it as well
 };
 int transfer(Ctx &c, std::initializer_list<Xfer> list, bool in, bool scalars = false) {
   HostFields fs;
@@ -319,11 +340,11 @@ int transfer(Ctx &c, std::initializer_list<Xfer> list, bool in, bool scalars = f
     f.pitch = pitch_of(c, *x.l);
     f.ay0 = x.l->ay0;
     f.ay1 = x.l->ay1;
-    make_present(x.a->data, sizeof(double) * f.row * (size_t)(f.rows + f.ay0 + f.ay1), !in);
+    make_present(x.a->data, sizeof(double) * f.row * (size_t)(f.rows + f.ay0 + f.ay1), !in || x.back);
   }
   if (!link) {
     for (const Xfer &x : list)
-      if (in ? h2d(c, *x.a, *x.l, x.dev) : d2h(c, const_cast<array_t &>(*x.a), *x.l, x.dev)) return 1;
+      if (in ? h2d(c, *x.a, *x.l, x.dev, x.back) : d2h(c, const_cast<array_t &>(*x.a), *x.l, x.dev)) return 1;
   }
   if (scalars) {
     double *const ct = c.b.coltab + (size_t)ct_cnewx(0) * c.g.ct, *const h = c.small_host;
@@ -1426,8 +1447,10 @@ int launch_step(Ctx &c) {
 
 int upload_fields(Ctx &c, const fluid_t *f, const interface_t *itf) {
   state_touched(c);
-  return h2d(c, f->ux, L_UX, c.U[c.iu]) || h2d(c, f->uy, L_UY, c.V[c.iu]) || h2d(c, f->p, L_P, c.b.p) ||
-         h2d(c, f->psi[0], L_P, c.PSI[c.ipsi]) || h2d(c, itf->vof, L_VOF, c.b.vof);
+  const bool back = g_sync_mode != SBFS_SYNC_NONE;
+  return h2d(c, f->ux, L_UX, c.U[c.iu], back) || h2d(c, f->uy, L_UY, c.V[c.iu], back) ||
+         h2d(c, f->p, L_P, c.b.p, back) || h2d(c, f->psi[0], L_P, c.PSI[c.ipsi], back) ||
+         h2d(c, itf->vof, L_VOF, c.b.vof, back);
 }
 
 int upload_state(Ctx &c, const fluid_t *f, const interface_t *itf) {
@@ -1942,7 +1965,7 @@ int sbfs_sync_to_host(const domain_t *d, fluid_t *f, interface_t *itf) {
   Ctx *c = g_ctx.get();
   if (!c || !c->resident) return 0;
   (void)d;
-  // (256 x 128 0.15 -> 0.05 ms, 2048 x 1024 0.89 -> 0.67 ms; 4096 x 2048 2.36 -> 2.67 ms)
+  // (256 x 128 0.15 -> 0.05 ms, 2048 x 1024 0.85 -> 0.64 ms; 4096 x 2048 2.36 -> 2.67 ms)
   const bool linked =
       g_sync_mode != SBFS_SYNC_ALL && (long)c->nx * c->ny <= 1L << 22 && link_download(*c, 1, &f, &itf, {0});
   if (!linked && download_state(*c, f, itf, g_sync_mode == SBFS_SYNC_ALL)) return 1;
@@ -1958,13 +1981,10 @@ bool link_tab_fill(Ctx &c, int k, fluid_t *f, interface_t *itf) {
   const Layout *lay[HL_COUNT] = {&L_UX, &L_UY, &L_P, &L_P, &L_VOF, &L_UX, &L_UY, &L_P, &L_P, &L_P, &L_VOF};
   if (c.nc == 1) c.link_host.assign(HL_COUNT, nullptr);
   double **tab = c.link_tab + (size_t)k * kLinkSlots;
-  double *const psi_prev[2] = {tab[HL_PSI0_OUT], tab[HL_PSI1_OUT]};
   for (int q = 0; q < HL_COUNT; ++q) {
-    double *const prev = tab[q];
     if (!layout_ok(*arr[q], *lay[q]) || !host_addressable(arr[q]->data, &tab[q])) return false;
     if (c.nc == 1) c.link_host[q] = arr[q]->data;
-    // other arrays than the step before (whose psi arrays come swapped)
-    if (q >= HL_UX_OUT && tab[q] != prev && tab[q] != psi_prev[0] && tab[q] != psi_prev[1])
+    if (q >= HL_UX_OUT)  // the arrays in are among them
       make_present(arr[q]->data, sizeof(double) * (c.nx + lay[q]->ax0 + lay[q]->ax1) *
                                      (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1), true);
   }
@@ -2257,7 +2277,7 @@ int interface_compute_curvature_tensor(const domain_t *d, interface_t *itf) {
   c->resident = false;
   state_touched(*c);
   // cells outside the interface band keep their previous normal, as in the reference
-  if (transfer(*c, {{&itf->vof, &L_VOF, c->b.vof}, {&itf->normal, &L_NORMAL, c->b.normal}}, true)) return 1;
+  if (transfer(*c, {{&itf->vof, &L_VOF, c->b.vof}, {&itf->normal, &L_NORMAL, c->b.normal, true}}, true)) return 1;
   launch_props(c->s, c->g, c->m, c->ph, c->b, false, false, true, nullptr);
   launch_normal_curv(c->s, c->g, c->m, c->b, true, true, false);
   if (transfer(*c, {{&itf->dvof, &L_DVOF, c->b.dvof}, {&itf->normal, &L_NORMAL, c->b.normal},
@@ -2289,7 +2309,7 @@ int interface_update_vof(const domain_t *d, const size_t rkstep, const double dt
   if (rkstep != 0) swap_data(itf->src[0], itf->src[1]);
   Bufs &b = c->b;
   put_scalars(*c, dt, (int)rkstep, 0., 0.);
-  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->vof, &L_VOF, b.vof},
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->vof, &L_VOF, b.vof, true},
                     {&itf->normal, &L_NORMAL, b.normal}, {&itf->src[1], &L_SRC, b.srcvof[1]}}, true, true)) return 1;
   launch_flux_force(c->s, c->g, c->m, c->ph, b, b.ux, b.uy, b.den0, true, false, false);
   launch_vof_advance(c->s, c->g, c->m, c->ph, b, b.scalars, (int)rkstep, b.srcvof[0], b.srcvof[1], false, b.ux,
@@ -2306,8 +2326,8 @@ int interface_compute_mass_flux(const domain_t *d, const fluid_t *f, interface_t
   c->resident = false;
   state_touched(*c);
   Bufs &b = c->b;
-  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->fluxx, &L_FLUXX, b.fluxx},
-                    {&itf->fluxy, &L_FLUXY, b.fluxy}}, true)) return 1;
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->fluxx, &L_FLUXX, b.fluxx, true},
+                    {&itf->fluxy, &L_FLUXY, b.fluxy, true}}, true)) return 1;
   launch_mass_flux_inplace(c->s, c->g, c->ph, b, b.ux, b.uy);
   if (transfer(*c, {{&itf->fluxx, &L_FLUXX, b.fluxx}, {&itf->fluxy, &L_FLUXY, b.fluxy}}, false)) return 1;
   return sync(*c);
@@ -2327,7 +2347,7 @@ int fluid_predict_field(const domain_t *d, const size_t rkstep, const double dt,
   }
   Bufs &b = c->b;
   put_scalars(*c, dt, (int)rkstep, 0., 0.);
-  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&f->visux, &L_VISUX, b.visux},
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux, true}, {&f->uy, &L_UY, b.uy, true}, {&f->visux, &L_VISUX, b.visux},
                     {&f->visuy, &L_VISUY, b.visuy}, {&itf->fluxx, &L_FLUXX, b.mfluxx},
                     {&itf->fluxy, &L_FLUXY, b.mfluxy}, {&f->p, &L_P, b.p}, {&itf->ifrcx, &L_IFRCX, b.ifrcx},
                     {&itf->ifrcy, &L_IFRCY, b.ifrcy}, {&f->den[0], &L_DEN, b.den0},
@@ -2367,7 +2387,7 @@ int fluid_correct_velocity(const domain_t *d, const double dt_old, const double 
   state_touched(*c);
   Bufs &b = c->b;
   put_scalars(*c, 0., -1, dt_old, dt_new);
-  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&f->psi[0], &L_P, b.psi0},
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux, true}, {&f->uy, &L_UY, b.uy, true}, {&f->psi[0], &L_P, b.psi0},
                     {&f->psi[1], &L_P, b.psi1}, {&f->den[1], &L_DEN, b.den1}}, true, true)) return 1;
   launch_face_factor(c->s, c->g, c->ph, b, b.den1, b.psi0);
   launch_correct(c->s, c->g, c->m, b, b.scalars, 0, b.ux, b.uy, b.psi1, false, false);
@@ -2381,7 +2401,7 @@ int fluid_update_pressure(const domain_t *d, fluid_t *f) {
   if (!c) return 1;
   c->resident = false;
   state_touched(*c);
-  if (transfer(*c, {{&f->p, &L_P, c->b.p}, {&f->psi[1], &L_P, c->b.psi1}}, true)) return 1;
+  if (transfer(*c, {{&f->p, &L_P, c->b.p, true}, {&f->psi[1], &L_P, c->b.psi1}}, true)) return 1;
   launch_pressure(c->s, c->g, c->b, c->b.psi1);
   if (transfer(*c, {{&f->p, &L_P, c->b.p}}, false)) return 1;
   if (sync(*c)) return 1;
@@ -2395,7 +2415,7 @@ static int bc_call(const domain_t *d, array_t *a, const Layout &l, int kind) {
   c->resident = false;
   state_touched(*c);
   double *buf = c->b.txy;  // scratch
-  if (h2d(*c, *a, l, buf)) return 1;
+  if (h2d(*c, *a, l, buf, true)) return 1;
   if (kind == 0) launch_bc_ux(c->s, c->g, buf);
   else if (kind == 1) launch_bc_uy(c->s, c->g, buf);
   else if (kind == 2) launch_bc_neumann(c->s, c->g, buf);

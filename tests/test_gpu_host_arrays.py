@@ -1,5 +1,5 @@
 """Host arrays as callers may hold them, against ordinary ones bit for bit: off the 8-byte boundaries of their
-doubles (a field inside a packed record), which only the copy engines can move."""
+doubles (a field inside a packed record), which only the copy engines can move; with pages missing, or page-locked."""
 import numpy as np
 import pytest
 
@@ -115,3 +115,40 @@ def test_off_boundary_downloads(libs):
     _same(out[0], out[1], FIELDS)
     for x, y in zip(*batch):
         _same(x, y, FIELDS)
+
+
+# 640 x 1024: 5.3 MB an array, so pages are looked at
+@pytest.mark.parametrize("pages", ["untouched", "some", "locked"])
+def test_large_arrays_with_missing_pages(libs, pages):
+    """downloads and steps into arrays that have no pages, some, or page-locked ones, as into ordinary ones"""
+    gpu = libs[0]
+    st = _start(libs, 640, 1024)
+    ordinary, other = clone(st), clone(st)
+    for s in FIELDS:
+        ordinary.field(s)[...] = 1.0  # every page written
+    if pages != "locked":
+        for s in FIELDS:
+            shape = other.field(s).shape
+            new = np.zeros(shape)  # fresh mapping, no page of it touched
+            if pages == "some":
+                new[:shape[0] // 3] = 1.0
+            other._buffers[new.ctypes.data] = new
+            other._array_t(s).data = new.ctypes.data
+    else:
+        gpu.pin_host_state(other)
+    gpu.set_sync_mode(SYNC_NONE)
+    try:
+        gpu.invalidate_device()
+        gpu.run_steps_timed(st, 1)
+        for o in (ordinary, other):
+            gpu.sync_to_host(o)
+        _same(ordinary, other, FIELDS)
+        for mode in (SYNC_ALL, SYNC_STATE):
+            gpu.set_sync_mode(mode)
+            assert gpu.integrate(ordinary) == gpu.integrate(other)
+            _same(ordinary, other, FIELDS)
+    finally:
+        gpu.set_sync_mode(SYNC_STATE)
+        if pages == "locked":
+            gpu.unpin_host_state(other)
+        gpu.release()
