@@ -137,6 +137,8 @@ __host__ __device__ constexpr int sc_gdt2y(int k) { return 49 + k; }
 __host__ __device__ constexpr int sc_coldyp(int k) { return 52 + k; }
 __host__ __device__ constexpr int sc_rpx(int k) { return 55 + k; }
 __host__ __device__ constexpr int sc_rpy(int k) { return 58 + k; }
+// not zero where ux was zero everywhere at the start of the step (see still() in sbfs_kernels.cu)
+constexpr int kScStill = 61;
 // per-column coefficients of substage k (Bufs::coltab, kColTabs tables of
 // Grid::ct doubles per substage, I = 0..nx+1), written with the scalars:
 // 2 gamma dt / HXXF(I) (ux pressure term), cnew / HXXF(I) and (cold / pax) /

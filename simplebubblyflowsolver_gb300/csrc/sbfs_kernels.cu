@@ -42,6 +42,12 @@ constexpr int BX = 32, BY = 8;
 
 __device__ __forceinline__ size_t ix(const Grid &g, int row, int col) { return (size_t)row * g.p1 + col; }
 __device__ __forceinline__ bool same(double a, double b) { return dbits(a) == dbits(b); }
+// all of them zero, of either sign (by words)
+template <class... T>
+__device__ __forceinline__ bool zeros(T... x) {
+  const unsigned hi = (... | intfp::high(intfp::bits(x))), lo = (... | intfp::low(intfp::bits(x)));
+  return ((hi << 1) | lo) == 0u;
+}
 
 // Interface-branch compaction.  An FP64 instruction costs its warp an issue
 // slot however few of its lanes run it (measured: eight FMA chains on 1 to
@@ -879,6 +885,18 @@ struct MomOut {
   double xx, yy, xy, yx;
 };
 
+// A step whose ux is zero everywhere (fluid at rest, or moving along y only)
+// has zeros where the integer forms of the momentum kernels take none, in
+// every cell: decide_dt says so (kScStill), and such a step runs on the FP64
+// unit from the start.  2048 x 1024 at rest, a step: 2185 us with the integer
+// forms tried first, 1531 us without; 509 x 256 220 and 179 us.  Both paths
+// use the cell's loaded inputs, so that the loads stay ahead of the branch,
+// and take the registers of four blocks an SM.  A step in motion, 1000 x 512
+// and 509 x 256: without the branch 472 and 207 us (five blocks), with it 472
+// and 212 us (five), 467 and 205 us (four); the zeros looked for in each
+// cell's own values, 483 and 211 us (five).
+__device__ __forceinline__ bool still(const double *__restrict__ sc) { return __double2hiint(sc[kScStill]) != 0; }
+
 // the four fluxes of one thread (PART 1: the corner's two, 2: the centre's); returns whether an integer form gave up.
 // Of the 27 FP64 operations (SCALED) the four sum-and-difference pairs of the
 // velocities and four of the products run on the integer pipes.  2048 x 1024
@@ -910,13 +928,15 @@ __device__ __forceinline__ bool momflux_cell(const Fp64 &f, const MomIn &in, con
 }
 
 template <int STRESS, bool SCALED, int HOW>
-__global__ void __launch_bounds__(BX *BY, SCALED && HOW == kMomWhole ? 5 : 1)
-    k_momflux(Grid g, Metrics m, Phys ph0, const double *__restrict__ ux, const double *__restrict__ uy,
+__global__ void __launch_bounds__(BX *BY, SCALED && HOW == kMomWhole ? 4 : 1)
+    k_momflux(Grid g, Metrics m, Phys ph0, const double *__restrict__ sc, const double *__restrict__ ux,
+              const double *__restrict__ uy,
               const double *__restrict__ visux, const double *__restrict__ visuy, const double *__restrict__ mfx,
               const double *__restrict__ mfy, double *__restrict__ pxx, double *__restrict__ pyy,
               double *__restrict__ pxy, double *__restrict__ pyx, double *__restrict__ txx, double *__restrict__ txy,
               double *__restrict__ tyy) {
   pdl_entry();
+  sc += (size_t)blockIdx.z * (kScalars);
   const Phys ph = zphys(g, ph0);
   static_assert(!(SCALED && STRESS == 2), "the reference-form stresses take unscaled viscosities");
   const double *__restrict__ c4nuc = SCALED ? m.c4nucs : m.c4nuc + (size_t)blockIdx.z * g.cm;
@@ -960,13 +980,13 @@ __global__ void __launch_bounds__(BX *BY, SCALED && HOW == kMomWhole ? 5 : 1)
     in.c4 = c4nuc[Ic];
     return in;
   };
+  const bool at_rest = INT && !SPLIT && still(sc);
   MomIn in = load(r, rm, rp);
   MomOut o;
   auto cell = [&](auto part) {
-    if (momflux_cell<INT, SCALED, part>(f, in, ph, o)) {
-      in = load(reread(r), reread(rm), reread(rp));
-      momflux_cell<false, SCALED, part>(f, in, ph, o);
-    }
+    bool redo = at_rest;
+    if (!redo && (redo = momflux_cell<INT, SCALED, part>(f, in, ph, o))) in = load(reread(r), reread(rm), reread(rp));
+    if (redo) momflux_cell<false, SCALED, part>(f, in, ph, o);
   };
   if (!SPLIT)
     cell(std::integral_constant<int, 0>());
@@ -1029,7 +1049,8 @@ struct PredOut {
 // launch: 137.4 us all in FP64; with the integer forms 119.8 us, the loads of
 // the second face then exposed (warps waiting on global memory 6.5 of 9.6
 // cycles an issue); 106 us with those loads in flight during the first face
-// (yb); 99.7 us at five blocks an SM and the pressure difference in FP64.
+// (yb); 99.7 us at five blocks an SM and the pressure difference in FP64 (four
+// since: still()).
 template <bool INT, bool GRAV>
 __device__ __forceinline__ bool predict_face(const Fp64 &f, const PredIn &in, double hgrav, double adt2, double bdt2,
                                              int k, PredOut &o) {
@@ -1051,7 +1072,7 @@ __device__ __forceinline__ bool predict_face(const Fp64 &f, const PredIn &in, do
 }
 
 template <bool CACHED, int HOW>
-__global__ void __launch_bounds__(BX *BY, HOW == kMomWhole ? 5 : 1)
+__global__ void __launch_bounds__(BX *BY, HOW == kMomWhole ? 4 : 1)
     k_predict_mf(Grid g, Metrics m, Phys ph0, const double *__restrict__ sc, int k, const double *__restrict__ ux,
                  const double *__restrict__ uy, double *__restrict__ ux_out, double *__restrict__ uy_out,
                  const double *__restrict__ pxx, const double *__restrict__ pyy, const double *__restrict__ pxy,
@@ -1101,6 +1122,7 @@ __global__ void __launch_bounds__(BX *BY, HOW == kMomWhole ? 5 : 1)
       async_copy(&yb[10][tid], dpy + ix(g, r, I));
     }
   }
+  const bool at_rest = INT && still(sc);
   const double ps0 = CACHED && I != 1 && I != g.nx ? 0. : psio[ix(g, r, I)];
   // ---- ux at face I
   if (do_x && I >= 2) {
@@ -1119,8 +1141,11 @@ __global__ void __launch_bounds__(BX *BY, HOW == kMomWhole ? 5 : 1)
       return in;
     };
     PredOut o;
-    if (predict_face<INT, true>(f, load(r, rm, rp), hgrav, adt2, bdt2, k, o))
-      predict_face<false, true>(f, load(reread(r), reread(rm), reread(rp)), hgrav, adt2, bdt2, k, o);
+    PredIn in = load(r, rm, rp);
+    bool redo = INT && at_rest;
+    if (!redo && (redo = predict_face<INT, true>(f, in, hgrav, adt2, bdt2, k, o)))
+      in = load(reread(r), reread(rm), reread(rp));
+    if (redo) predict_face<false, true>(f, in, hgrav, adt2, bdt2, k, o);
     srx[ix(g, r, I - 1)] = o.rho1;
     ux_out[ix(g, r, I - 1)] = o.u;
     sxa[ix(g, r, I - 2)] = o.a;
@@ -1147,9 +1172,9 @@ __global__ void __launch_bounds__(BX *BY, HOW == kMomWhole ? 5 : 1)
       return in;
     };
     PredOut o;
+    PredIn in;
     if (WHOLE) {
       async_wait();
-      PredIn in;
       in.u0 = yb[0][tid], in.frc = yb[1][tid];
       in.pd1 = yb[2][tid], in.pd0 = yb[3][tid];
       in.po1 = yb[4][tid], in.po0 = yb[5][tid];
@@ -1159,11 +1184,12 @@ __global__ void __launch_bounds__(BX *BY, HOW == kMomWhole ? 5 : 1)
       in.rho0 = CACHED ? yb[9][tid] : f.add(den0[ix(g, rm, I)], den0[ix(g, r, I)]);  // 2 rho^k
       in.dps = CACHED ? yb[10][tid] : f.sub(ps0, psio[ix(g, rm, I)]);
       coefs(in);
-      if (predict_face<true, false>(f, in, hgrav, adt2, bdt2, k, o))
-        predict_face<false, false>(f, load(reread(r), reread(rm)), hgrav, adt2, bdt2, k, o);
-    } else if (predict_face<INT, false>(f, load(r, rm), hgrav, adt2, bdt2, k, o)) {
-      predict_face<false, false>(f, load(reread(r), reread(rm)), hgrav, adt2, bdt2, k, o);
+    } else {
+      in = load(r, rm);
     }
+    bool redo = INT && at_rest;
+    if (!redo && (redo = predict_face<INT, false>(f, in, hgrav, adt2, bdt2, k, o))) in = load(reread(r), reread(rm));
+    if (redo) predict_face<false, false>(f, in, hgrav, adt2, bdt2, k, o);
     sry[ix(g, r, I)] = o.rho1;
     uy_out[ix(g, r, I)] = o.u;
     sya[ix(g, r, I - 1)] = o.a;
@@ -1415,7 +1441,8 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
       const int c = t / q8, j = t - c * q8;
       const double2 *xr = x + c * M + j;
       double2 *yr = y + c * M + 8 * j;
-      if (radix8<INT>(f, xr, yr, q8, c8, inverse)) radix8<false>(f, xr, yr, q8, c8, inverse);
+      const bool none = INT && zeros(xr[0].x, xr[0].y);  // see radix4's call
+      if (none || radix8<INT>(f, xr, yr, q8, c8, inverse)) radix8<false>(f, xr, yr, q8, c8, inverse);
     }
     __syncthreads();
     double2 *tmp = x;
@@ -1441,11 +1468,13 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
       const int kk = j & (Ns - 1);
       const double2 *xr = x + c * M + j;
       double2 *yr = y + c * M + ((j - kk) << 2) + kk;
+      // zeros (fluid at rest), which the integer forms would give up on: the first input tells
+      const bool none = INT && zeros(xr[0].x, xr[0].y);
       if (Ns > 1) {
-        if (radix4<INT, true>(f, xr, yr, q4, Ns, wm, kk * step, two, inverse))
+        if (none || radix4<INT, true>(f, xr, yr, q4, Ns, wm, kk * step, two, inverse))
           radix4<false, true>(f, xr, yr, q4, Ns, wm, kk * step, two, inverse);
       } else {
-        if (radix4<INT, false>(f, xr, yr, q4, Ns, wm, 0, two, inverse))
+        if (none || radix4<INT, false>(f, xr, yr, q4, Ns, wm, 0, two, inverse))
           radix4<false, false>(f, xr, yr, q4, Ns, wm, 0, two, inverse);
       }
     }
@@ -1756,7 +1785,8 @@ __global__ void __launch_bounds__(512)
       double2 xa = make_double2(0., 0.), xb = make_double2(0., 0.);
       if (i < nx) {
         const double2 wa = tw[p], wb = tw[M - p];
-        if (split_pair<INT>(f64, zm[v], zr[v], wa, wb, xa, xb)) split_pair<false>(f64, zm[v], zr[v], wa, wb, xa, xb);
+        const bool none = INT && zeros(zm[v].x, zm[v].y, zr[v].x, zr[v].y);
+        if (none || split_pair<INT>(f64, zm[v], zr[v], wa, wb, xa, xb)) split_pair<false>(f64, zm[v], zr[v], wa, wb, xa, xb);
       }
       double *o = sm + (size_t)(4 * q) * sys_len + (i / L) * S + (i % L);
       o[0] = xa.x;
@@ -1857,7 +1887,8 @@ __global__ void __launch_bounds__(512)
     const double2 Xb = make_double2(sm[(4 * q + 2) * sys_len + at], sm[(4 * q + 3) * sys_len + at]);
     const double2 wa = tw[p], wb = tw[M - p];
     double2 za, zb;
-    if (merge_pair<INT>(f64, Xa, Xb, wa, wb, za, zb)) merge_pair<false>(f64, Xa, Xb, wa, wb, za, zb);
+    const bool none = INT && zeros(Xa.x, Xa.y, Xb.x, Xb.y);
+    if (none || merge_pair<INT>(f64, Xa, Xb, wa, wb, za, zb)) merge_pair<false>(f64, Xa, Xb, wa, wb, za, zb);
     sp[(size_t)i * M1 + p] = za;
     if (p != 0 && 2 * p != M) sp[(size_t)i * M1 + (M - p)] = zb;
   }
@@ -1905,7 +1936,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(128)
       const double2 zm = sp[(size_t)i * M1 + p];
       const double2 zr = sp[(size_t)i * M1 + (p == 0 ? 0 : M - p)];
       const double2 wa = tw[p], wb = tw[M - p];
-      if (split_pair<INT>(f64, zm, zr, wa, wb, xa, xbv)) split_pair<false>(f64, zm, zr, wa, wb, xa, xbv);
+      const bool none = INT && zeros(zm.x, zm.y, zr.x, zr.y);
+      if (none || split_pair<INT>(f64, zm, zr, wa, wb, xa, xbv)) split_pair<false>(f64, zm, zr, wa, wb, xa, xbv);
     }
     smem_cl[0 * sys_len + at] = xa.x;
     smem_cl[1 * sys_len + at] = xa.y;
@@ -1996,7 +2028,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(128)
     const double2 Xb = make_double2(smem_cl[2 * sys_len + at], smem_cl[3 * sys_len + at]);
     const double2 wa = tw[p], wb = tw[M - p];
     double2 za, zb;
-    if (merge_pair<INT>(f64, Xa, Xb, wa, wb, za, zb)) merge_pair<false>(f64, Xa, Xb, wa, wb, za, zb);
+    const bool none = INT && zeros(Xa.x, Xa.y, Xb.x, Xb.y);
+    if (none || merge_pair<INT>(f64, Xa, Xb, wa, wb, za, zb)) merge_pair<false>(f64, Xa, Xb, wa, wb, za, zb);
     sp[(size_t)i * M1 + p] = za;
     if (p != 0 && 2 * p != M) sp[(size_t)i * M1 + (M - p)] = zb;
   }
@@ -2089,7 +2122,7 @@ __global__ void k_pressure(Grid g, const double *__restrict__ psin, double *__re
 // status word.  Scratch per case (nx + 8 words, zero between launches):
 // [2..nx] column max |ux| bits, [nx+2] max |uy| bits, [nx+4] the complement
 // of the least quotient's bits (so that zero means none yet), [nx+5] the
-// finishing blocks' counter.
+// finishing blocks' counter, [nx+6] whether any ux is not zero.
 // ---------------------------------------------------------------------------
 constexpr unsigned long long kAbsMask = 0x7fffffffffffffffULL;
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ULL;
@@ -2148,6 +2181,7 @@ __global__ void __launch_bounds__(kDtFinThreads)
   __shared__ int wbad[kDtFinThreads / 32];
   __shared__ bool last;
   __shared__ double dt_sh;
+  __shared__ int flow_sh;
   const double small = 1.e-8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // dt_adv = coef * min(1, min_i hx_i / (max|ux|_i + small), hy / (max|uy| + small))
@@ -2157,7 +2191,7 @@ __global__ void __launch_bounds__(kDtFinThreads)
   if (i <= g.nx + 1) {
     // the maxima are final (the stream order) and were formed at L2
     const unsigned long long b = __ldcg(acc + (i <= g.nx ? i : g.nx + 2));
-    bad = b >= kInfBits ? 1 : 0;
+    bad = (b >= kInfBits ? 1 : 0) | (b != 0 && i <= g.nx ? 2 : 0);  // bit 1: there is flow along x
     d = (i <= g.nx ? m.hxxf[i] : g.hy) / (__longlong_as_double((long long)b) + small);
   }
 #pragma unroll
@@ -2175,9 +2209,10 @@ __global__ void __launch_bounds__(kDtFinThreads)
       d = fmin(d, wmin[w]);
       bad |= wbad[w];
     }
-    if (bad) atomicOr(status, 1);
+    if (bad & 1) atomicOr(status, 1);
     last = true;
     if (gridDim.x > 1) {
+      if (bad & 2) atomicOr(acc + g.nx + 6, 1ULL);
       // a positive d (or 1): the least bit pattern is the least value
       atomicMax(acc + g.nx + 4, ~(unsigned long long)dbits(d));
       __threadfence();
@@ -2185,6 +2220,7 @@ __global__ void __launch_bounds__(kDtFinThreads)
       last = (done == gridDim.x - 1);
     }
     dt_sh = d;
+    flow_sh = bad & 2;
   }
   __syncthreads();
   if (!last) return;
@@ -2193,8 +2229,10 @@ __global__ void __launch_bounds__(kDtFinThreads)
   // / dtnew (an FP64 instruction takes the warp's slot once for all of them)
   if (warp == 0) {
     double dt = dt_sh;
+    bool flow = flow_sh != 0;
     if (gridDim.x > 1) {
       __threadfence();
+      flow = __ldcg(acc + g.nx + 6) != 0;
       dt = __longlong_as_double((long long)~__ldcg(acc + g.nx + 4));
     }
     // the 1 of the minimum stands here: with nx a multiple of kDtFinThreads
@@ -2217,7 +2255,10 @@ __global__ void __launch_bounds__(kDtFinThreads)
       const double cadd = -ratio * (0.5 / g.ny);
       const double pax = cadd * (g.idx * g.idx), pay = cadd * (g.ihy * g.ihy);
       const double cnew = dtnew * ph.irefden, cold = -dtold * ph.irefden, coldy = cold * g.ihy;
-      if (k == 0) sc[0] = dt;
+      if (k == 0) {
+        sc[0] = dt;
+        sc[kScStill] = flow ? 0. : 1.;
+      }
       sc[sc_adt(k)] = a * dt;
       sc[sc_bdt(k)] = b * dt;
       sc[sc_gdt(k)] = dtnew;
@@ -2242,7 +2283,7 @@ __global__ void __launch_bounds__(kDtFinThreads)
   }
   __syncthreads();
   // reset the scratch for the next launch
-  for (int t = tid; t <= g.nx + 5; t += kDtFinThreads) acc[t] = 0ULL;
+  for (int t = tid; t <= g.nx + 6; t += kDtFinThreads) acc[t] = 0ULL;
 }
 
 // the per-column coefficients of the three substages from the scalars (one
@@ -2765,7 +2806,7 @@ void launch_momflux(cudaStream_t s, const Grid &g, const Metrics &m, const Phys 
       k = stress == 1 ? k_momflux<1, true, kMomSplit> : k_momflux<0, true, kMomSplit>;
     if (how != kMomWhole) gr.y *= 2;
   }
-  launch_pdl(k, gr, bl, 0, s, g, m, ph, ux, uy, b.visux, b.visuy, b.mfluxx, b.mfluxy, b.pxx, b.pyy, b.pxy, b.pyx,
+  launch_pdl(k, gr, bl, 0, s, g, m, ph, (const double *)b.scalars, ux, uy, b.visux, b.visuy, b.mfluxx, b.mfluxy, b.pxx, b.pyy, b.pxy, b.pyx,
              b.txx, b.txy, b.tyy);
 }
 

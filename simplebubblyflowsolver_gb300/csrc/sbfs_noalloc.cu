@@ -36,8 +36,8 @@ using namespace sbfs;
 
 namespace {
 
-// per-column maxima (nx + 2 words), the |uy| maximum, the least quotient
-// and the block counter (words nx + 2 .. nx + 5)
+// per-column maxima (nx + 2 words), the |uy| maximum, the least quotient, the
+// block counter and the flow flag (words nx + 2 .. nx + 6)
 constexpr int kScratchWords = SBFS_NOALLOC_MAX_NX + 8;
 static __device__ __align__(256) unsigned long long g_dt_scratch[kScratchWords];
 
@@ -76,7 +76,7 @@ extern "C" int sbfs_decide_dt_noalloc(int nx, int ny, double lx, double ly, cons
   unsigned long long *scratch = static_cast<unsigned long long *>(p);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // the kernel needs zeroed accumulators; the array keeps the last call's words
-  e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long) * (nx + 6), s);
+  e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long) * (nx + 7), s);
   if (e != cudaSuccess) return report("sbfs_decide_dt_noalloc: clearing the scratch", e);
   Grid g{};
   g.nc = 1;
