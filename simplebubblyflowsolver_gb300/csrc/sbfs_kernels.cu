@@ -1303,7 +1303,7 @@ __device__ __forceinline__ bool radix4(const Fp64 &f, const double2 *xr, double2
     const double2 w1 = wm[e], w2 = wm[2 * e], w3 = wm[3 * e];
     const double2 a0 = make_double2(fma(w2.x, v2.x, fma(-w2.y, v2.y, v0.x)), fma(w2.x, v2.y, fma(w2.y, v2.x, v0.y)));
     const double2 a1 = make_double2(fma(two, v0.x, -a0.x), fma(two, v0.y, -a0.y));
-    const double2 t1 = make_double2(fma(v1.x, w1.x, (1 ? n.mulz(-v1.y, w1.y) : f.mul(-v1.y, w1.y))), fma(v1.x, w1.y, (1 ? n.mulz(v1.y, w1.x) : f.mul(v1.y, w1.x))));
+    const double2 t1 = make_double2(fma(v1.x, w1.x, n.mulz(-v1.y, w1.y)), fma(v1.x, w1.y, n.mulz(v1.y, w1.x)));
     const double2 a2 = make_double2(fma(w3.x, v3.x, fma(-w3.y, v3.y, t1.x)), fma(w3.x, v3.y, fma(w3.y, v3.x, t1.y)));
     const double2 a3 = make_double2(fma(two, t1.x, -a2.x), fma(two, t1.y, -a2.y));
     const double2 r3 = rot(a3, inverse);
