@@ -117,11 +117,12 @@ int sbfs_set_compaction(int mode);
  * counterpart in the reference.) */
 int sbfs_set_stream_priorities(int on);
 
-/* where a grid solves its tridiagonal systems with four warps each, run the
- * four systems of a wavenumber pair as a cluster of four CTAs, one quarter
- * of the rows each, exchanging the chunk maps through distributed shared
- * memory (default 1); 0 keeps one block per pair or two.  Same results
- * either way, bit for bit.  (No counterpart in the reference.) */
+/* where a grid solves its tridiagonal systems with four warps each (or with
+ * two, while the pairs leave SMs idle), run the four systems of a wavenumber
+ * pair as a cluster of four (two) CTAs, an equal share of the rows each,
+ * exchanging the chunk maps through distributed shared memory (default 1);
+ * 0 keeps one block per pair or two.  Same results either way, bit for bit.
+ * (No counterpart in the reference.) */
 int sbfs_set_tdm_cluster(int on);
 
 /* run each substage's interface geometry ahead of its velocity (default 1):
@@ -274,7 +275,8 @@ int sbfs_set_autotune(int on);
 /* shapes in use (group -1: the single-case context): bx[7], by[7] for
  * props, curvature list, flux/force, vof advance, stress, predict,
  * correct; the Poisson transform width, wavenumbers per tridiagonal block
- * (0: one pair per cluster of four CTAs) and warps per tridiagonal system;
+ * (0: one pair per cluster of as many CTAs as a system has warps, 2 or 4)
+ * and warps per tridiagonal system;
  * compact (may be NULL): 1 when the corner-gradient and curvature work is
  * compacted within blocks */
 int sbfs_tiles(int group, int *bx, int *by, int *fft_w, int *tdm_mb, int *tdm_warps, int *compact);

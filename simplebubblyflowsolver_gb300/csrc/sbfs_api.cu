@@ -1218,7 +1218,7 @@ int autotune(Ctx &c) {
   {
     Tiles cl = c.b.tiles;
     cl.tdm_cl = 1;
-    if (tdm_uses_cluster(cl, c.nx)) tdms.push_back({0, G});  // 0: a cluster of four CTAs per pair
+    if (tdm_uses_cluster(cl, c.nx)) tdms.push_back({0, G});  // 0: a cluster of G CTAs per pair
   }
   for (int mb : {1, 2, 4})
     if (G * mb <= 4 && poisson_tdm_smem(c.nx, mb, G) <= 200 * 1024) tdms.push_back({mb, G});

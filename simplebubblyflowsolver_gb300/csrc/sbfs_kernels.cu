@@ -1894,16 +1894,16 @@ __global__ void __launch_bounds__(512)
   }
 }
 
-// The same solves with four warps per system, spread over a cluster of four
-// CTAs: CTA r of a cluster owns rows 32 L r .. 32 L (r + 1) - 1 of the four
-// systems of one wavenumber pair (warp s: system s), so a launch has four
-// CTAs per pair where k_poisson_tdm has one block per pair or two, and the
-// 4 (ny/4 + 1) CTAs of a case even out over the SMs (in a launch of blocks
-// of one or two pairs, ny/4 + 1 pairs leave SMs idle while the last blocks
-// run, one in six for ny = 1024).  The chunk-map totals of
-// the other CTAs come through distributed shared memory and are combined in
-// the order k_poisson_tdm<false> combines its warps' at G = 4, so both give
-// the same bits.  L = tdm_chunk(nx, 4), S = L | 1; fac is the G = 4 table.
+// The same solves with CL = 2 or 4 warps per system, spread over a cluster of
+// CL CTAs: CTA r of a cluster owns rows 32 L r .. 32 L (r + 1) - 1 of the four
+// systems of one wavenumber pair (warp s: system s), so a launch has CL CTAs
+// per pair where k_poisson_tdm has one block per pair or two, and the CL
+// (ny/4 + 1) CTAs of a case even out over the SMs (in a launch of blocks of
+// one or two pairs, ny/4 + 1 pairs leave SMs idle while the last blocks run,
+// one in six for ny = 1024).  The chunk-map totals of the other CTAs come
+// through distributed shared memory and are combined in the order
+// k_poisson_tdm<false> combines its warps' at G = CL, so both give the same
+// bits.  L = tdm_chunk(nx, CL), S = L | 1; fac is the G = CL table.
 template <bool INT, int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(128)
     k_poisson_tdm_cl(Grid g, int L, int S, const double4_32a *__restrict__ fac, const double2 *__restrict__ tw,
@@ -2584,8 +2584,9 @@ int tdm_group_index(int G) { return G == 4 ? 2 : (G == 2 ? 1 : 0); }
 // 256 x 128 to 1024 x 512; on the 2048 x 1024 swarm 4 warps a system in
 // clusters balance the SMs better but add 6% to the solve's FP64 work, and
 // the step gains nothing: the side stream fills the SMs a block-per-pair
-// launch leaves idle).  At 4 warps a system the solves of a pair run as a
-// cluster of four CTAs (k_poisson_tdm_cl).  A rule of the grid, not a tuned choice: it sets how
+// launch leaves idle).  At 4 warps a system, and at 2 while the pairs leave
+// SMs idle, the solves of a pair run as a cluster of as many CTAs
+// (k_poisson_tdm_cl).  A rule of the grid, not a tuned choice: it sets how
 // the chunk maps are combined, and so the rounding of the solve.
 int tdm_modes_per_block(const Tiles &t, int nx) {
   const int G = t.tdm_g > 0 ? t.tdm_g : 1;
