@@ -1490,7 +1490,7 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
 // grad psi_old (ux, uy are qx, qy; egx, egy unused): 3 FP64 operations per
 // cell instead of 7
 template <int W, bool Q, int HOW>
-__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : 1)
+__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : (HOW == kFftPlain ? 5 : 1))
     k_poisson_fwd(Grid g, const double *__restrict__ sc, int k, const double *__restrict__ ux,
                   const double *__restrict__ uy, const double *__restrict__ egx, const double *__restrict__ egy,
                   const double2 *__restrict__ tw, double2 *__restrict__ spec) {
@@ -1540,7 +1540,7 @@ __global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : 1)
 }
 
 template <int W, int HOW>
-__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : 1)
+__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : (HOW == kFftPlain ? 5 : 1))
     k_poisson_inv(Grid g, const double2 *__restrict__ tw, const double2 *__restrict__ spec, double *__restrict__ psi) {
   pdl_entry();
   spec += (size_t)blockIdx.z * (g.css);
@@ -1606,11 +1606,13 @@ __device__ __forceinline__ bool merge_pair(const Fp64 &f, double2 Xa, double2 Xb
 // One lane's chunk of a system, rows x[0 .. L), factors f[k lanes].  AHEAD:
 // the factors of the next kAhead rows are loaded while those of the present
 // ones are used, since a block's shared memory leaves room for one to three
-// warps a scheduler on large grids, which otherwise wait for them; on short
-// chunks (64 x 64: two rows) its tests cost more than the wait.  One launch
-// of k_poisson_tdm, with the split's sums on the integer pipes: 2048 x 1024
-// 61.7 -> 52.1 us, 4096 x 2048 472 -> 370 us (one warp a scheduler; 326 us
-// with four rows of the split's loads in flight as well).
+// warps a scheduler on large grids, which otherwise wait for them; what is
+// left after the last whole group goes row by row (a test per row in every
+// group, as a first version had it, takes an FP64 slot for each row past the
+// end: 1300 x 1024, 21 rows a lane, 50 -> 42 us).  One launch of
+// k_poisson_tdm, with the split's sums on the integer pipes: 2048 x 1024
+// 61.7 -> 52 us, 4096 x 2048 472 -> 312 us (one warp a scheduler; four rows of
+// the split's loads in flight as well).
 constexpr int kAhead = 8;
 template <bool AHEAD, int STEP, class Load, class Use>
 __device__ __forceinline__ void sweep(int L, Load load, Use use) {
@@ -1621,39 +1623,47 @@ __device__ __forceinline__ void sweep(int L, Load load, Use use) {
     return;
   }
   decltype(load(0)) c[kAhead], n[kAhead];
+  int k0 = 0;
+  if (L >= kAhead) {
 #pragma unroll
-  for (int u = 0; u < kAhead; ++u)
-    if (u < L) c[u] = load(row(u));
-  for (int k0 = 0; k0 < L; k0 += kAhead) {
+    for (int u = 0; u < kAhead; ++u) c[u] = load(row(u));
+    for (; k0 + 2 * kAhead <= L; k0 += kAhead) {
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u)
-      if (k0 + kAhead + u < L) n[u] = load(row(k0 + kAhead + u));
+      for (int u = 0; u < kAhead; ++u) n[u] = load(row(k0 + kAhead + u));
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u)
-      if (k0 + u < L) use(row(k0 + u), c[u]);
+      for (int u = 0; u < kAhead; ++u) use(row(k0 + u), c[u]);
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) c[u] = n[u];
+      for (int u = 0; u < kAhead; ++u) c[u] = n[u];
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) use(row(k0 + u), c[u]);
+    k0 += kAhead;
   }
+#pragma unroll 1
+  for (; k0 < L; ++k0) use(row(k0), load(row(k0)));
 }
-// Chunk<INT> holds a lane's rows and factors between the sweeps.  Small
-// launches (not INT) with chunks of up to kReg rows keep both in registers,
-// the factors loaded before the split's rows arrive: three trips to L2 and
+// HOW a launch solves its chunks (chosen in tdm_how): plainly; chunks of up to
+// kTdmReg rows in registers; shared with the integer pipes, factors ahead.
+// Chunk<HOW> holds a lane's rows and factors between the sweeps.  In registers
+// the factors load before the split's rows arrive: three trips to L2 and
 // back, and the rows' to shared memory, leave the chain (k_poisson_tdm on
 // 256 x 128 11.8 -> 9.0 us with the pairs' clusters at two
 // warps a system, on 509 x 256 14.0 -> 11.4 us).
-template <bool INT>
+enum TdmHow { kTdmPlain, kTdmReg, kTdmInt };
+constexpr int kTdmRegRows = 4;
+template <int HOW>
 struct Chunk {
-  static constexpr int kReg = INT ? 1 : 4;
+  static constexpr bool INT = HOW == kTdmInt, reg = HOW == kTdmReg;
+  static constexpr int kReg = reg ? kTdmRegRows : 1;
   const Fp64 &f64;
   const double4_32a *__restrict__ f;
   size_t lanes;
   int L;
   double *x;
-  bool reg;
   double4_32a c[kReg];
   double r[kReg];
   __device__ __forceinline__ Chunk(const Fp64 &f_, const double4_32a *fac, size_t lanes_, int L_, double *x_, bool act)
-      : f64(f_), f(fac), lanes(lanes_), L(L_), x(x_), reg(!INT && L_ <= kReg) {
+      : f64(f_), f(fac), lanes(lanes_), L(L_), x(x_) {
     if (reg && act) {
 #pragma unroll
       for (int k = 0; k < kReg; ++k)
@@ -1735,7 +1745,7 @@ struct Chunk {
 // Staging: per system a planar array with an odd lane stride S, in shared
 // memory; when four systems of nx rows exceed it (nx above about 6900), in
 // this block's slab of the global buffer stage (L2-resident, same arithmetic).
-template <bool kGlobalStage, bool INT>
+template <bool kGlobalStage, int HOW>
 __global__ void __launch_bounds__(512)
     k_poisson_tdm(Grid g, int PB, int G, int L, int S, const double4_32a *__restrict__ fac,
                   const double2 *__restrict__ tw, double2 *__restrict__ spec, double *__restrict__ stage) {
@@ -1760,7 +1770,8 @@ __global__ void __launch_bounds__(512)
   const int m = (sys & 2) ? M - pq : pq;  // the wavenumber of this system
   double *x = sm + sys * sys_len + j * S;
   const double4_32a *f = fac + (size_t)m * L * lanes + j;
-  Chunk<INT> ch(f64, f, lanes, L, x, act);
+  constexpr bool INT = HOW == kTdmInt;
+  Chunk<HOW> ch(f64, f, lanes, L, x, act);
   // ---- load the packed transform of both wavenumbers of each pair, split
   // it (real-to-complex, times 2: X_m = (z_m + conj z_{M-m}) + w^m (-i)(z_m -
   // conj z_{M-m})) into four planar systems: X_p re, im, X_{M-p} re, im
@@ -1904,7 +1915,7 @@ __global__ void __launch_bounds__(512)
 // through distributed shared memory and are combined in the order
 // k_poisson_tdm<false> combines its warps' at G = CL, so both give the same
 // bits.  L = tdm_chunk(nx, CL), S = L | 1; fac is the G = CL table.
-template <bool INT, int CL>
+template <int HOW, int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(128)
     k_poisson_tdm_cl(Grid g, int L, int S, const double4_32a *__restrict__ fac, const double2 *__restrict__ tw,
                      double2 *__restrict__ spec) {
@@ -1926,7 +1937,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(128)
   const int m = (sys & 2) ? M - p : p;
   double *x = smem_cl + sys * sys_len + lane * S;
   const double4_32a *f = fac + (size_t)m * L * lanes + j;
-  Chunk<INT> ch(f64, f, lanes, L, x, true);
+  constexpr bool INT = HOW == kTdmInt;
+  Chunk<HOW> ch(f64, f, lanes, L, x, true);
   // ---- load and split (as in k_poisson_tdm), this CTA's rows
   for (int t = threadIdx.x; t < rows; t += blockDim.x) {
     const int i = r0 + t;
@@ -2593,8 +2605,8 @@ int tdm_modes_per_block(const Tiles &t, int nx) {
   const int mb = t.tdm_mb > 0 ? t.tdm_mb : poisson_tdm_modes(nx);
   return mb * G > 4 ? 4 / G : mb;  // at most 512 threads a block
 }
-// Whether the stencils, and the transforms, of a launch over these cells share
-// their arithmetic with the integer pipes: only where enough warps are in
+// Whether the stencils of a launch over these cells share their arithmetic
+// with the integer pipes: only where enough warps are in
 // flight to keep the FP64 unit busy; below that an integer form's longer
 // chain of instructions sets a warp's time.  Measured, us a launch, one part
 // a thread on the FP64 unit, shared, and both parts shared: k_momflux 256 x
@@ -2603,25 +2615,55 @@ int tdm_modes_per_block(const Tiles &t, int nx) {
 // 13.3; 20.6, 21.0, 19.2.  The lines follow the whole step, whose side stream
 // runs beside the predictor: us with one part on the FP64 unit and shared, 256
 // x 128 113.7, 115.9; 500 x 128 160.0, 153.6; 509 x 256 244.6, 237.3, and
-// 220.3 with both shared.  k_poisson_fwd in a thread, FP64 alone and shared:
-// 509 x 256 9.2, 10.7; 512 x 512 13.3, 13.7 (k_poisson_inv 12.3, 11.6); 1000 x 512 20.5,
-// 18.4.
+// 220.3 with both shared.
 long cells(const Grid &g) { return (long)g.nx * g.ny * g.nc; }
 bool integer_stencils(const Grid &g) { return cells(g) >= 3L << 15; }
 MomHow stencil_how(const Grid &g) {
   return integer_stencils(g) ? kMomWhole : (cells(g) >= 3L << 14 ? kMomSplitInt : kMomSplit);
 }
-bool integer_transforms(const Grid &g) { return cells(g) >= 1L << 18; }
+// the transforms and tridiagonal solves of smaller launches stay on the FP64 unit
+bool integer_launch(const Grid &g) { return cells(g) >= 1L << 18; }
+// complex rows of a transform launch with w columns a block on the SM with most
+long rows_per_sm(const Grid &g, int w) {
+  const long blocks = (long)((g.nx + w - 1) / w) * g.nc;
+  return w * (g.ny / 2) * ((blocks + 151) / 152);
+}
+// A block of w columns has w M / 4 butterflies a stage (M = ny / 2): short
+// blocks have one to two warps of them, whose chain of instructions the
+// integer forms lengthen, and keep the FP64 unit busy from more blocks an SM
+// instead (five; the forms' registers leave four).  k_poisson_fwd and _inv,
+// us, shared and alone: 250 cases of 64 x 64 73.6, 65.6 and 59.2, 51.8; 32 of
+// 256 x 128 42.0, 34.8 and 35.4, 31.5; 8 of 512 x 256 38.7, 32.7 and 33.7,
+// 28.7; 20 of 100 x 512 32.9, 26.2 and 34.7, 28.7; 4 of 300 x 1024 37.9, 30.5
+// and 44.4, 35.3.  With few blocks an SM both wait for loads and barriers, and
+// what counts is the FP64 unit's time left to the side stream: the step of 512
+// x 512 (two blocks an SM) 287 and 272 us, of 800 x 512 (three) 362 and 372.
+bool integer_transforms(const Grid &g, int w) {
+  return integer_launch(g) && w * (g.ny / 2) >= 512 && rows_per_sm(g, w) >= 1536;
+}
+// Chunks of L rows: the integer forms' registers (94, plainly 60) and groups of
+// kAhead rows pay for long ones.  k_poisson_tdm, us, shared and plainly: 1000
+// cases of 32 x 32 (1 row) 203 and 88, 250 of 64 x 64 (2) 102 and 56, 128 of
+// 128 x 64 (4) 63 and 47, 64 of 224 x 128 (7) 64 and 60; the step of 32 cases
+// of 256 x 128 (8) 846 and 861 us.  Where few pairs are spread over warps (G >
+// 1) the loads ahead count from 5 rows on: 600 x 512 21.6 and 22.4 us, 600 x
+// 1024 (10) 26.3 and 27.6, its step 487 and 524.  Registers pay for a launch
+// of less than two blocks an SM: 256 x 128 (33 pairs, 4 rows) 12.3 us and
+// plainly 14.3, 13 cases of 128 x 64 (221) 12.1 and 12.5; 30 of 64 x 64 (510, 2
+// rows) 14.2 and 13.0; the step of 100 cases of 16 x 8 (300, 1 row) 122 and 112.
+TdmHow tdm_how(const Grid &g, int G) {
+  const int L = tdm_chunk(g.nx, G);
+  if (integer_launch(g) && L >= (G > 1 ? 5 : 8)) return kTdmInt;
+  const long pairs = (g.ny / 4 + 1L) * g.nc;
+  return L <= kTdmRegRows && pairs < (L >= 3 ? 304 : 152) ? kTdmReg : kTdmPlain;
+}
 // Whether a launch spreads its butterflies over lanes: its warps issue twice
 // the FP64 instructions, in a quarter of the turns, so it pays while they are
 // few enough a scheduler, W M complex rows a block and that many blocks an SM
 // making at most 256.  Measured, us a launch of k_poisson_fwd: 64 x 64 (64)
 // 6.7 -> 4.8, 256 x 128 (128) 7.2 -> 5.8, 256 x 256 (256) 8.9 -> 8.7, 509 x
 // 256 (512) 9.3 -> 10.4, 128 x 1024 (1024) 17.1 -> 27.6.
-bool lane_transforms(const Grid &g, int w) {
-  const long blocks = (long)((g.nx + w - 1) / w) * g.nc;
-  return w * (g.ny / 2) * ((blocks + 151) / 152) <= 256;
-}
+bool lane_transforms(const Grid &g, int w) { return rows_per_sm(g, w) <= 256; }
 // default pairs per block: as many as shared memory and 512 threads take, but
 // one block a pair while the pairs are too few to give every SM that many
 // (its warps share one FP64 unit a scheduler: 64 x 64 k_poisson_tdm 10.8 ->
@@ -2662,8 +2704,10 @@ cudaError_t configure_kernels() {
   const int big = 227 * 1024;
   e = configure_fft<1, 2, 4, 8>(big);
   if (e != cudaSuccess) return e;
-  return allow_smem((int)kTdmSmemMax, k_poisson_tdm<false, false>, k_poisson_tdm<false, true>, k_poisson_tdm_cl<false, 4>,
-                    k_poisson_tdm_cl<true, 4>, k_poisson_tdm_cl<false, 2>, k_poisson_tdm_cl<true, 2>);
+  return allow_smem((int)kTdmSmemMax, k_poisson_tdm<false, kTdmPlain>, k_poisson_tdm<false, kTdmReg>,
+                    k_poisson_tdm<false, kTdmInt>, k_poisson_tdm_cl<kTdmPlain, 2>, k_poisson_tdm_cl<kTdmReg, 2>,
+                    k_poisson_tdm_cl<kTdmInt, 2>, k_poisson_tdm_cl<kTdmPlain, 4>, k_poisson_tdm_cl<kTdmReg, 4>,
+                    k_poisson_tdm_cl<kTdmInt, 4>);
 }
 
 void launch_props(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const Bufs &b, bool den, bool vis,
@@ -2841,7 +2885,7 @@ template <int W, bool Q>
 void poisson_fwd_w(cudaStream_t s, const Grid &g, const Bufs &b, const double *sc, int k, const double *ux,
                    const double *uy) {
   const int nb = (g.nx + W - 1) / W;
-  auto kern = integer_transforms(g) ? k_poisson_fwd<W, Q, kFftInt> : k_poisson_fwd<W, Q, kFftPlain>;
+  auto kern = integer_transforms(g, W) ? k_poisson_fwd<W, Q, kFftInt> : k_poisson_fwd<W, Q, kFftPlain>;
   if (W <= 2 && lane_transforms(g, W)) kern = k_poisson_fwd<(W <= 2 ? W : 2), Q, kFftLanes>;
   launch_pdl(kern, dim3(nb, 1, g.nc), 256, poisson_fft_smem(g.ny, W), s, g, sc, k, ux, uy, b.egx, b.egy, b.twiddle, b.spec);
 }
@@ -2875,32 +2919,38 @@ bool tdm_uses_cluster(const Tiles &t, int nx) {
          4 * 32 * (size_t)tdm_stride(nx, t.tdm_g) * sizeof(double) <= kTdmSmemMax;
 }
 
+template <int CL>
+auto tdm_cluster_kernel(TdmHow how) {
+  return how == kTdmInt ? k_poisson_tdm_cl<kTdmInt, CL>
+                        : (how == kTdmReg ? k_poisson_tdm_cl<kTdmReg, CL> : k_poisson_tdm_cl<kTdmPlain, CL>);
+}
+
 void launch_poisson_tdm(cudaStream_t s, const Grid &g, const Bufs &b) {
   const int G = b.tiles.tdm_g > 0 ? b.tiles.tdm_g : 1;
-  const int pairs = g.ny / 4 + 1;
+  const int pairs = g.ny / 4 + 1, L = tdm_chunk(g.nx, G), S = tdm_stride(g.nx, G);
   const double4_32a *fac = reinterpret_cast<const double4_32a *>(b.tdm_fac[tdm_group_index(G)]);
+  const TdmHow how = tdm_how(g, G);
   if (tdm_uses_cluster(b.tiles, g.nx)) {  // G CTAs per pair, four warps each
-    const int L = tdm_chunk(g.nx, G), S = tdm_stride(g.nx, G);
-    auto kern = G == 4 ? k_poisson_tdm_cl<false, 4> : k_poisson_tdm_cl<false, 2>;
-    if (integer_transforms(g)) kern = G == 4 ? k_poisson_tdm_cl<true, 4> : k_poisson_tdm_cl<true, 2>;
-    launch_pdl(kern, dim3(G * pairs, 1, g.nc), 128, 4 * 32 * (size_t)S * sizeof(double), s, g, L, S, fac, b.twiddle,
-               b.spec);
+    launch_pdl(G == 4 ? tdm_cluster_kernel<4>(how) : tdm_cluster_kernel<2>(how), dim3(G * pairs, 1, g.nc), 128,
+               4 * 32 * (size_t)S * sizeof(double), s, g, L, S, fac, b.twiddle, b.spec);
     return;
   }
   if (tdm_global_stage(g.nx, G)) {  // one pair per block, staged in b.tdm_stage
-    launch_pdl(integer_transforms(g) ? k_poisson_tdm<true, true> : k_poisson_tdm<true, false>, dim3(pairs, 1, g.nc), 128 * G, 0, s, g, 1, G, tdm_chunk(g.nx, G), tdm_stride(g.nx, G),
-                                                                 fac, b.twiddle, b.spec, b.tdm_stage);
+    launch_pdl(how == kTdmInt ? k_poisson_tdm<true, kTdmInt> : k_poisson_tdm<true, kTdmPlain>, dim3(pairs, 1, g.nc),
+               128 * G, 0, s, g, 1, G, L, S, fac, b.twiddle, b.spec, b.tdm_stage);
     return;
   }
   const int mb = tdm_modes_per_block(b.tiles, g.nx);  // wavenumber pairs per block
-  launch_pdl(integer_transforms(g) ? k_poisson_tdm<false, true> : k_poisson_tdm<false, false>, dim3((pairs + mb - 1) / mb, 1, g.nc), 128 * mb * G, poisson_tdm_smem(g.nx, mb, G), s,
-      g, mb, G, tdm_chunk(g.nx, G), tdm_stride(g.nx, G), fac, b.twiddle, b.spec, nullptr);
+  auto kern = how == kTdmInt ? k_poisson_tdm<false, kTdmInt>
+                             : (how == kTdmReg ? k_poisson_tdm<false, kTdmReg> : k_poisson_tdm<false, kTdmPlain>);
+  launch_pdl(kern, dim3((pairs + mb - 1) / mb, 1, g.nc), 128 * mb * G, poisson_tdm_smem(g.nx, mb, G), s, g, mb, G, L, S, fac,
+             b.twiddle, b.spec, (double *)nullptr);
 }
 
 template <int W>
 void poisson_inv_w(cudaStream_t s, const Grid &g, const Bufs &b, double *psi_new) {
   const int nb = (g.nx + W - 1) / W;
-  auto kern = integer_transforms(g) ? k_poisson_inv<W, kFftInt> : k_poisson_inv<W, kFftPlain>;
+  auto kern = integer_transforms(g, W) ? k_poisson_inv<W, kFftInt> : k_poisson_inv<W, kFftPlain>;
   if (W <= 2 && lane_transforms(g, W)) kern = k_poisson_inv<(W <= 2 ? W : 2), kFftLanes>;
   launch_pdl(kern, dim3(nb, 1, g.nc), 256, poisson_fft_smem(g.ny, W), s, g, b.twiddle, b.spec, psi_new);
 }

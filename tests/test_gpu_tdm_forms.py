@@ -91,9 +91,12 @@ def test_autotuned_as_default(libs, nx, ny, ahead):
 
 
 # clusters of two in either; of four, shared only in the batch; blocks of two in the batch, shared; one warp a system;
-# 8192 rows staged in global memory, shared only in the batch (the clusters off)
+# 8192 rows staged in global memory, shared only in the batch (the clusters off); transforms shared only in the batch,
+# chunks of 4 rows in registers and plainly, of 5 plainly and shared; of 10 and 22 rows, groups of eight and the rest
 @pytest.mark.parametrize("nx,ny,cases,cluster", [(256, 128, 3, True), (512, 256, 2, True), (256, 128, 8, True),
-                                                 (125, 64, 33, True), (8192, 16, 2, True), (8192, 16, 2, False)])
+                                                 (125, 64, 33, True), (8192, 16, 2, True), (8192, 16, 2, False),
+                                                 (100, 512, 8, True), (300, 512, 3, True), (1200, 64, 4, True),
+                                                 (2700, 64, 2, True)])
 def test_different_cases_in_a_batch_as_alone(libs, nx, ny, cases, cluster):
     gpu = libs[0]
     start = [_start(libs, nx, ny, k % 5) for k in range(cases)]
