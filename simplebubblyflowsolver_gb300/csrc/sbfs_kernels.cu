@@ -2783,10 +2783,22 @@ void launch_interface_stage(cudaStream_t s, const Grid &g, const Metrics &m, con
   }
 }
 
+// An SM takes blocks of another kernel only under the split of its memory that
+// it has: the geometry's blocks beside a short transform's, whose split is
+// smaller, all went to the few SMs without one of those (40 blocks to five
+// SMs, eight on each: 30 us instead of 6).
+// On grids that short, while there is an SM for every block, they ask for the
+// smallest split that holds one (in percent): ten cases of 32 x 32, a step 161
+// -> 92 us, of 64 x 32 147 -> 99 us, of 48 x 32 137 -> 96 us.  Elsewhere the
+// smaller split costs more than the crowding (24 cases of 64 x 32 145 and 160
+// us, 4 of 128 x 64 108 and 115, 509 x 256 183 and 201).
+constexpr int kFewBlocksSmem = 3;
 void launch_geometry(cudaStream_t s, const Grid &g, const Metrics &m, const Bufs &b) {
-  launch_pdl(k_curv_list<false>, tile_grid(b.tiles, TK_CURV_LIST, g.nx, g.ny, g.nc), tile_block(b.tiles, TK_CURV_LIST),
-             0, s, g, m, b.vof, b.dvof, (const double *)nullptr, (const double *)nullptr, b.curv, b.ilist, b.icount,
-             b.flist, b.fcount, b.tf, compaction(b.tiles));
+  const dim3 gr = tile_grid(b.tiles, TK_CURV_LIST, g.nx, g.ny, g.nc);
+  const bool few = g.ny <= 32 && (long)gr.x * gr.y * gr.z <= 152;
+  launch_pdl_smem(few ? kFewBlocksSmem : -1, k_curv_list<false>, gr, tile_block(b.tiles, TK_CURV_LIST), 0, s, g, m, b.vof,
+                  b.dvof, (const double *)nullptr, (const double *)nullptr, b.curv, b.ilist, b.icount, b.flist, b.fcount,
+                  b.tf, compaction(b.tiles));
 }
 
 void launch_bulk_flux(cudaStream_t s, const Grid &g, const Metrics &m, const Phys &ph, const Bufs &b,

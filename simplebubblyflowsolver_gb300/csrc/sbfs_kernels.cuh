@@ -193,23 +193,31 @@ extern int g_compact;  // -1: per context (Tiles::compact), else 0 / 1 for all
 // SMs with the main stream's blocks first and the side stream's in the gaps;
 // 0: every launch at the default priority.  Scheduling only: the same results
 extern int g_stream_prio;
+// carveout: the share of an SM's memory asked for as shared memory, in percent
+// (-1: the driver's choice for the kernel)
 template <typename... P, typename... A>
-void launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...a) {
-  cudaLaunchAttribute at[2];
+void launch_pdl_smem(int carveout, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...a) {
+  cudaLaunchAttribute at[3];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = g_pdl ? 1 : 0;
   int prio = 0;
   if (g_stream_prio) cudaStreamGetPriority(s, &prio);
   at[1].id = cudaLaunchAttributePriority;
   at[1].val.priority = prio;
+  at[2].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at[2].val.sharedMemCarveout = carveout;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = at;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = carveout >= 0 ? 3 : 2;
   cudaLaunchKernelEx(&cfg, k, static_cast<A &&>(a)...);
+}
+template <typename... P, typename... A>
+void launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...a) {
+  launch_pdl_smem(-1, k, grid, block, smem, s, static_cast<A &&>(a)...);
 }
 
 // smem budget checks (host side)
