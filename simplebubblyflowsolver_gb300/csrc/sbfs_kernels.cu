@@ -902,7 +902,8 @@ __device__ __forceinline__ bool still(const double *__restrict__ sc) { return __
 // velocities and four of the products run on the integer pipes.  2048 x 1024
 // swarm, one launch: 110.6 us all in FP64 (FP64 unit 85% busy); 69.1 us with
 // a fifth product on the integer side (integer pipes 90%, FP64 73%), 73.6 us
-// with one sum more; 65.9 us as it stands (89%, 82%).
+// with one sum more; 65.9 us as it stands at five blocks an SM (89%, 82%), 64.1
+// us at four (94%, 85%).
 template <bool INT, bool SCALED, int PART = 0>
 __device__ __forceinline__ bool momflux_cell(const Fp64 &f, const MomIn &in, const Phys &ph, MomOut &o) {
   Fp64Int<INT> q(f);
@@ -1049,8 +1050,8 @@ struct PredOut {
 // launch: 137.4 us all in FP64; with the integer forms 119.8 us, the loads of
 // the second face then exposed (warps waiting on global memory 6.5 of 9.6
 // cycles an issue); 106 us with those loads in flight during the first face
-// (yb); 99.7 us at five blocks an SM and the pressure difference in FP64 (four
-// since: still()).
+// (yb); 99.7 us at five blocks an SM and the pressure difference in FP64, 97.4
+// us at four with still()'s branch.
 template <bool INT, bool GRAV>
 __device__ __forceinline__ bool predict_face(const Fp64 &f, const PredIn &in, double hgrav, double adt2, double bdt2,
                                              int k, PredOut &o) {
@@ -1611,7 +1612,7 @@ __device__ __forceinline__ bool merge_pair(const Fp64 &f, double2 Xa, double2 Xb
 // group, as a first version had it, takes an FP64 slot for each row past the
 // end: 1300 x 1024, 21 rows a lane, 50 -> 42 us).  One launch of
 // k_poisson_tdm, with the split's sums on the integer pipes: 2048 x 1024
-// 61.7 -> 52 us, 4096 x 2048 472 -> 312 us (one warp a scheduler; four rows of
+// 61.7 -> 53 us, 4096 x 2048 472 -> 320 us (one warp a scheduler; four rows of
 // the split's loads in flight as well).
 constexpr int kAhead = 8;
 template <bool AHEAD, int STEP, class Load, class Use>
