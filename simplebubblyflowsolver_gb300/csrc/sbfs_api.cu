@@ -213,11 +213,13 @@ size_t case_off(const Ctx &c, const Layout &l) {
 // instead of 5.78.  Below 4 MB even the look would show.  Pages that are
 // present and all the same fault when the GPU comes to them (the 4096 x 2048
 // state between two segments, at times) are not helped by this.
-// write: the call writes the array, so its pages must not be the shared page
-// of zeros that a read maps.  Contents do not change, and a failure only
+// Arrays in get pages of their own as well: populated for reading they would
+// all map one page of zeros, which the GPU reads more slowly at every copy
+// (fluid_predict_field on 4096 x 2048, its untouched arrays so, 15 ms instead
+// of 9.3).  Contents do not change, and a failure (a read-only mapping) only
 // leaves the faults to the copy.
-void make_present(const void *p, size_t bytes, bool write) {
-#if defined(MADV_POPULATE_READ) && defined(MADV_POPULATE_WRITE)
+void make_present(const void *p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
   static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
   if (bytes < (size_t)4 << 20) return;
   const uintptr_t lo = (uintptr_t)p & ~(uintptr_t)(page - 1);
@@ -234,22 +236,21 @@ void make_present(const void *p, size_t bytes, bool write) {
     for (size_t a = 0, b = 0; a < n; a = b) {
       while (b < n && (in[b] & 1) == (in[a] & 1)) ++b;
       if (!(in[a] & 1))
-        madvise(reinterpret_cast<void *>(at + a * page), (b - a) * page, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ);
+        madvise(reinterpret_cast<void *>(at + a * page), (b - a) * page, MADV_POPULATE_WRITE);
     }
   }
 #else
   (void)p;
   (void)bytes;
-  (void)write;
 #endif
 }
 
-// host array (reference layout, rows J = 1 - ay0 .. ny + ay1) -> device rows J = 1..ny; back: it is written later
-int h2d(Ctx &c, const array_t &a, const Layout &l, double *dev, bool back = false) {
+// host array (reference layout, rows J = 1 - ay0 .. ny + ay1) -> device rows J = 1..ny
+int h2d(Ctx &c, const array_t &a, const Layout &l, double *dev) {
   if (!layout_ok(a, l)) return fail("array layout does not match the reference's (nadds/size)");
   const size_t row = (size_t)(c.nx + l.ax0 + l.ax1) * l.nc;
   const double *src = static_cast<const double *>(a.data) + (size_t)l.ay0 * row;
-  make_present(src, sizeof(double) * row * (size_t)c.ny, back);
+  make_present(src, sizeof(double) * row * (size_t)c.ny);
   dev += case_off(c, l);
   CK(cudaMemcpy2DAsync(dev, sizeof(double) * pitch_of(c, l), src, sizeof(double) * row, sizeof(double) * row, c.ny,
                        cudaMemcpyHostToDevice, c.s));
@@ -262,7 +263,7 @@ int d2h(Ctx &c, array_t &a, const Layout &l, const double *dev) {
   const size_t row = (size_t)(c.nx + l.ax0 + l.ax1) * l.nc;
   const size_t pitch = sizeof(double) * pitch_of(c, l);
   double *dst = static_cast<double *>(a.data);
-  make_present(dst, sizeof(double) * row * (size_t)(c.ny + l.ay0 + l.ay1), true);
+  make_present(dst, sizeof(double) * row * (size_t)(c.ny + l.ay0 + l.ay1));
   dev += case_off(c, l);
   CK(cudaMemcpy2DAsync(dst + (size_t)l.ay0 * row, sizeof(double) * row, dev, pitch, sizeof(double) * row, c.ny,
                        cudaMemcpyDeviceToHost, c.s));
@@ -318,7 +319,6 @@ struct Xfer {
   const array_t *a;
   const Layout *l;
   double *dev;
-  bool back = false;  // of an array in: the call writes it as well
 };
 int transfer(Ctx &c, std::initializer_list<Xfer> list, bool in, bool scalars = false) {
   HostFields fs;
@@ -340,11 +340,11 @@ int transfer(Ctx &c, std::initializer_list<Xfer> list, bool in, bool scalars = f
     f.pitch = pitch_of(c, *x.l);
     f.ay0 = x.l->ay0;
     f.ay1 = x.l->ay1;
-    make_present(x.a->data, sizeof(double) * f.row * (size_t)(f.rows + f.ay0 + f.ay1), !in || x.back);
+    make_present(x.a->data, sizeof(double) * f.row * (size_t)(f.rows + f.ay0 + f.ay1));
   }
   if (!link) {
     for (const Xfer &x : list)
-      if (in ? h2d(c, *x.a, *x.l, x.dev, x.back) : d2h(c, const_cast<array_t &>(*x.a), *x.l, x.dev)) return 1;
+      if (in ? h2d(c, *x.a, *x.l, x.dev) : d2h(c, const_cast<array_t &>(*x.a), *x.l, x.dev)) return 1;
   }
   if (scalars) {
     double *const ct = c.b.coltab + (size_t)ct_cnewx(0) * c.g.ct, *const h = c.small_host;
@@ -1447,10 +1447,8 @@ int launch_step(Ctx &c) {
 
 int upload_fields(Ctx &c, const fluid_t *f, const interface_t *itf) {
   state_touched(c);
-  const bool back = g_sync_mode != SBFS_SYNC_NONE;
-  return h2d(c, f->ux, L_UX, c.U[c.iu], back) || h2d(c, f->uy, L_UY, c.V[c.iu], back) ||
-         h2d(c, f->p, L_P, c.b.p, back) || h2d(c, f->psi[0], L_P, c.PSI[c.ipsi], back) ||
-         h2d(c, itf->vof, L_VOF, c.b.vof, back);
+  return h2d(c, f->ux, L_UX, c.U[c.iu]) || h2d(c, f->uy, L_UY, c.V[c.iu]) || h2d(c, f->p, L_P, c.b.p) ||
+         h2d(c, f->psi[0], L_P, c.PSI[c.ipsi]) || h2d(c, itf->vof, L_VOF, c.b.vof);
 }
 
 int upload_state(Ctx &c, const fluid_t *f, const interface_t *itf) {
@@ -1986,7 +1984,7 @@ bool link_tab_fill(Ctx &c, int k, fluid_t *f, interface_t *itf) {
     if (c.nc == 1) c.link_host[q] = arr[q]->data;
     if (q >= HL_UX_OUT)  // the arrays in are among them
       make_present(arr[q]->data, sizeof(double) * (c.nx + lay[q]->ax0 + lay[q]->ax1) *
-                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1), true);
+                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1));
   }
   if (c.nc == 1 && (c.link_host != c.link_prev || c.link_epoch != g_reg_epoch)) {
     // page-locked or pageable: the copy engines move them differently, and a
@@ -2024,8 +2022,7 @@ bool link_download(Ctx &c, int n, fluid_t *const *f, interface_t *const *itf, co
           !host_addressable(arr[q]->data, &c.link_tab[(size_t)k * kLinkSlots + slot[q]]))
         return false;
       make_present(arr[q]->data, sizeof(double) * (c.nx + lay[q]->ax0 + lay[q]->ax1) *
-                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1),
-                   true);
+                                     (size_t)(c.ny + lay[q]->ay0 + lay[q]->ay1));
     }
   }
   for (int q = 0; q < kOut; q += 3)
@@ -2277,7 +2274,7 @@ int interface_compute_curvature_tensor(const domain_t *d, interface_t *itf) {
   c->resident = false;
   state_touched(*c);
   // cells outside the interface band keep their previous normal, as in the reference
-  if (transfer(*c, {{&itf->vof, &L_VOF, c->b.vof}, {&itf->normal, &L_NORMAL, c->b.normal, true}}, true)) return 1;
+  if (transfer(*c, {{&itf->vof, &L_VOF, c->b.vof}, {&itf->normal, &L_NORMAL, c->b.normal}}, true)) return 1;
   launch_props(c->s, c->g, c->m, c->ph, c->b, false, false, true, nullptr);
   launch_normal_curv(c->s, c->g, c->m, c->b, true, true, false);
   if (transfer(*c, {{&itf->dvof, &L_DVOF, c->b.dvof}, {&itf->normal, &L_NORMAL, c->b.normal},
@@ -2309,7 +2306,7 @@ int interface_update_vof(const domain_t *d, const size_t rkstep, const double dt
   if (rkstep != 0) swap_data(itf->src[0], itf->src[1]);
   Bufs &b = c->b;
   put_scalars(*c, dt, (int)rkstep, 0., 0.);
-  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->vof, &L_VOF, b.vof, true},
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->vof, &L_VOF, b.vof},
                     {&itf->normal, &L_NORMAL, b.normal}, {&itf->src[1], &L_SRC, b.srcvof[1]}}, true, true)) return 1;
   launch_flux_force(c->s, c->g, c->m, c->ph, b, b.ux, b.uy, b.den0, true, false, false);
   launch_vof_advance(c->s, c->g, c->m, c->ph, b, b.scalars, (int)rkstep, b.srcvof[0], b.srcvof[1], false, b.ux,
@@ -2326,8 +2323,8 @@ int interface_compute_mass_flux(const domain_t *d, const fluid_t *f, interface_t
   c->resident = false;
   state_touched(*c);
   Bufs &b = c->b;
-  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->fluxx, &L_FLUXX, b.fluxx, true},
-                    {&itf->fluxy, &L_FLUXY, b.fluxy, true}}, true)) return 1;
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&itf->fluxx, &L_FLUXX, b.fluxx},
+                    {&itf->fluxy, &L_FLUXY, b.fluxy}}, true)) return 1;
   launch_mass_flux_inplace(c->s, c->g, c->ph, b, b.ux, b.uy);
   if (transfer(*c, {{&itf->fluxx, &L_FLUXX, b.fluxx}, {&itf->fluxy, &L_FLUXY, b.fluxy}}, false)) return 1;
   return sync(*c);
@@ -2347,7 +2344,7 @@ int fluid_predict_field(const domain_t *d, const size_t rkstep, const double dt,
   }
   Bufs &b = c->b;
   put_scalars(*c, dt, (int)rkstep, 0., 0.);
-  if (transfer(*c, {{&f->ux, &L_UX, b.ux, true}, {&f->uy, &L_UY, b.uy, true}, {&f->visux, &L_VISUX, b.visux},
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&f->visux, &L_VISUX, b.visux},
                     {&f->visuy, &L_VISUY, b.visuy}, {&itf->fluxx, &L_FLUXX, b.mfluxx},
                     {&itf->fluxy, &L_FLUXY, b.mfluxy}, {&f->p, &L_P, b.p}, {&itf->ifrcx, &L_IFRCX, b.ifrcx},
                     {&itf->ifrcy, &L_IFRCY, b.ifrcy}, {&f->den[0], &L_DEN, b.den0},
@@ -2387,7 +2384,7 @@ int fluid_correct_velocity(const domain_t *d, const double dt_old, const double 
   state_touched(*c);
   Bufs &b = c->b;
   put_scalars(*c, 0., -1, dt_old, dt_new);
-  if (transfer(*c, {{&f->ux, &L_UX, b.ux, true}, {&f->uy, &L_UY, b.uy, true}, {&f->psi[0], &L_P, b.psi0},
+  if (transfer(*c, {{&f->ux, &L_UX, b.ux}, {&f->uy, &L_UY, b.uy}, {&f->psi[0], &L_P, b.psi0},
                     {&f->psi[1], &L_P, b.psi1}, {&f->den[1], &L_DEN, b.den1}}, true, true)) return 1;
   launch_face_factor(c->s, c->g, c->ph, b, b.den1, b.psi0);
   launch_correct(c->s, c->g, c->m, b, b.scalars, 0, b.ux, b.uy, b.psi1, false, false);
@@ -2401,7 +2398,7 @@ int fluid_update_pressure(const domain_t *d, fluid_t *f) {
   if (!c) return 1;
   c->resident = false;
   state_touched(*c);
-  if (transfer(*c, {{&f->p, &L_P, c->b.p, true}, {&f->psi[1], &L_P, c->b.psi1}}, true)) return 1;
+  if (transfer(*c, {{&f->p, &L_P, c->b.p}, {&f->psi[1], &L_P, c->b.psi1}}, true)) return 1;
   launch_pressure(c->s, c->g, c->b, c->b.psi1);
   if (transfer(*c, {{&f->p, &L_P, c->b.p}}, false)) return 1;
   if (sync(*c)) return 1;
@@ -2415,7 +2412,7 @@ static int bc_call(const domain_t *d, array_t *a, const Layout &l, int kind) {
   c->resident = false;
   state_touched(*c);
   double *buf = c->b.txy;  // scratch
-  if (h2d(*c, *a, l, buf, true)) return 1;
+  if (h2d(*c, *a, l, buf)) return 1;
   if (kind == 0) launch_bc_ux(c->s, c->g, buf);
   else if (kind == 1) launch_bc_uy(c->s, c->g, buf);
   else if (kind == 2) launch_bc_neumann(c->s, c->g, buf);
