@@ -194,7 +194,7 @@ extern int g_compact;  // -1: per context (Tiles::compact), else 0 / 1 for all
 // 0: every launch at the default priority.  Scheduling only: the same results
 extern int g_stream_prio;
 // carveout: the share of an SM's memory asked for as shared memory, in percent
-// (-1: the driver's choice for the kernel)
+// (-1: CUDA's choice for the kernel)
 template <typename... P, typename... A>
 void launch_pdl_smem(int carveout, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...a) {
   cudaLaunchAttribute at[3];

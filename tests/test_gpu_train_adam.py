@@ -25,10 +25,13 @@ def data():
 
 
 def _fma(a, b, c):
-    """a b + c rounded once (extended precision holds the exact value on this machine)"""
-    wide = np.longdouble
-    assert np.finfo(wide).nmant >= 112
-    return (wide(a) * wide(b) + wide(c)).astype(F)
+    """a b + c rounded once: the product is exact in FP64, the sum rounded there to odd, which FP32's rounding undoes"""
+    p, c = np.float64(a) * np.asarray(b, np.float64), np.asarray(c, np.float64)
+    s = p + c
+    t = s - p
+    lost = (p - (s - t)) + (c - t)
+    to_odd = (lost != 0) & (s.view(np.int64) % 2 == 0)
+    return np.where(to_odd, np.nextafter(s, np.where(lost > 0, np.inf, -np.inf)), s).astype(F)
 
 
 def _powf():
