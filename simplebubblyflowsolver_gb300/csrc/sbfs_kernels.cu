@@ -2249,8 +2249,9 @@ __global__ void __launch_bounds__(kDtFinThreads)
       dt = __longlong_as_double((long long)~__ldcg(acc + g.nx + 4));
     }
     // the 1 of the minimum stands here: with nx a multiple of kDtFinThreads
-    // every thread above has a quotient in its place (a NaN's minimum is 1 too)
-    dt = fmin(dt, 1.);
+    // every thread above has a quotient in its place
+    // (by words: any positive value above 1, and any NaN)
+    if ((unsigned long long)dbits(dt) > (unsigned long long)dbits(1.)) dt = 1.;
     dt *= coef_adv;
     dt = fmin(dt, dt_fixed);
     const int k = lane % 3, ko = (k + 2) % 3;
