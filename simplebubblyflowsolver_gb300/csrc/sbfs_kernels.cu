@@ -1419,9 +1419,10 @@ __device__ __forceinline__ void radix4_lanes(const Fp64 &f, const double2 *xr, d
 // holding the result.
 // tw: the twiddle buffer, exp(-2 pi i m / 2M) for m = 0..M, then W_M^e for
 // e < M, then their conjugates (the inverse's): one load per twiddle.
-// HOW: a thread's butterflies on the FP64 unit (kFftPlain), shared with the
-// integer pipes (kFftInt), or spread over lanes (kFftLanes).
-enum FftHow { kFftPlain, kFftInt, kFftLanes };
+// HOW: a thread's butterflies on the FP64 unit (kFftPlain; kFftShort with the
+// registers of five blocks an SM, for launches that have them), shared with
+// the integer pipes (kFftInt), or spread over lanes (kFftLanes).
+enum FftHow { kFftPlain, kFftInt, kFftLanes, kFftShort };
 template <int W, int HOW>
 __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__restrict__ tw, bool inverse, const Fp64 &f,
                              int cols) {
@@ -1491,7 +1492,7 @@ __device__ double2 *fft_rows(double2 *x, double2 *y, int M, const double2 *__res
 // grad psi_old (ux, uy are qx, qy; egx, egy unused): 3 FP64 operations per
 // cell instead of 7
 template <int W, bool Q, int HOW>
-__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : (HOW == kFftPlain ? 5 : 1))
+__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : (HOW == kFftShort ? 5 : 1))
     k_poisson_fwd(Grid g, const double *__restrict__ sc, int k, const double *__restrict__ ux,
                   const double *__restrict__ uy, const double *__restrict__ egx, const double *__restrict__ egy,
                   const double2 *__restrict__ tw, double2 *__restrict__ spec) {
@@ -1541,7 +1542,7 @@ __global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : (HOW == kFftPlain ? 
 }
 
 template <int W, int HOW>
-__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : (HOW == kFftPlain ? 5 : 1))
+__global__ void __launch_bounds__(256, HOW == kFftInt ? 4 : (HOW == kFftShort ? 5 : 1))
     k_poisson_inv(Grid g, const double2 *__restrict__ tw, const double2 *__restrict__ spec, double *__restrict__ psi) {
   pdl_entry();
   spec += (size_t)blockIdx.z * (g.css);
@@ -2625,11 +2626,13 @@ MomHow stencil_how(const Grid &g) {
 }
 // the transforms and tridiagonal solves of smaller launches stay on the FP64 unit
 bool integer_launch(const Grid &g) { return cells(g) >= 1L << 18; }
-// complex rows of a transform launch with w columns a block on the SM with most
-long rows_per_sm(const Grid &g, int w) {
-  const long blocks = (long)((g.nx + w - 1) / w) * g.nc;
-  return w * (g.ny / 2) * ((blocks + 151) / 152);
-}
+// of a transform launch with w columns a block: blocks, and complex rows, on the SM with most
+long blocks_per_sm(const Grid &g, int w) { return ((long)((g.nx + w - 1) / w) * g.nc + 151) / 152; }
+long rows_per_sm(const Grid &g, int w) { return w * (g.ny / 2) * blocks_per_sm(g, w); }
+// The FP64 form's registers (60 to 64) leave four blocks an SM; at 48 five are resident, and up to 24 bytes spilled
+// make a block itself slower: forward, 250 cases of 64 x 64 (53 blocks an SM) 59 us and with four resident 67, but
+// 210 x 1024 (a block an SM or none) 20.8 us and at 60 registers 19.8
+bool five_blocks(const Grid &g, int w) { return blocks_per_sm(g, w) > 4; }
 // A block of w columns has w M / 4 butterflies a stage (M = ny / 2): short
 // blocks have one to two warps of them, whose chain of instructions the
 // integer forms lengthen, and keep the FP64 unit busy from more blocks an SM
@@ -2698,7 +2701,8 @@ cudaError_t configure_fft(int bytes) {
   if (e != cudaSuccess) return e;
   return allow_smem(bytes, k_poisson_fwd<W, false, kFftPlain>..., k_poisson_fwd<W, true, kFftPlain>...,
                     k_poisson_fwd<W, false, kFftInt>..., k_poisson_fwd<W, true, kFftInt>...,
-                    k_poisson_inv<W, kFftPlain>..., k_poisson_inv<W, kFftInt>...);
+                    k_poisson_fwd<W, false, kFftShort>..., k_poisson_fwd<W, true, kFftShort>...,
+                    k_poisson_inv<W, kFftPlain>..., k_poisson_inv<W, kFftInt>..., k_poisson_inv<W, kFftShort>...);
 }
 
 cudaError_t configure_kernels() {
@@ -2899,7 +2903,8 @@ template <int W, bool Q>
 void poisson_fwd_w(cudaStream_t s, const Grid &g, const Bufs &b, const double *sc, int k, const double *ux,
                    const double *uy) {
   const int nb = (g.nx + W - 1) / W;
-  auto kern = integer_transforms(g, W) ? k_poisson_fwd<W, Q, kFftInt> : k_poisson_fwd<W, Q, kFftPlain>;
+  auto kern = five_blocks(g, W) ? k_poisson_fwd<W, Q, kFftShort> : k_poisson_fwd<W, Q, kFftPlain>;
+  if (integer_transforms(g, W)) kern = k_poisson_fwd<W, Q, kFftInt>;
   if (W <= 2 && lane_transforms(g, W)) kern = k_poisson_fwd<(W <= 2 ? W : 2), Q, kFftLanes>;
   launch_pdl(kern, dim3(nb, 1, g.nc), 256, poisson_fft_smem(g.ny, W), s, g, sc, k, ux, uy, b.egx, b.egy, b.twiddle, b.spec);
 }
@@ -2964,7 +2969,8 @@ void launch_poisson_tdm(cudaStream_t s, const Grid &g, const Bufs &b) {
 template <int W>
 void poisson_inv_w(cudaStream_t s, const Grid &g, const Bufs &b, double *psi_new) {
   const int nb = (g.nx + W - 1) / W;
-  auto kern = integer_transforms(g, W) ? k_poisson_inv<W, kFftInt> : k_poisson_inv<W, kFftPlain>;
+  auto kern = five_blocks(g, W) ? k_poisson_inv<W, kFftShort> : k_poisson_inv<W, kFftPlain>;
+  if (integer_transforms(g, W)) kern = k_poisson_inv<W, kFftInt>;
   if (W <= 2 && lane_transforms(g, W)) kern = k_poisson_inv<(W <= 2 ? W : 2), kFftLanes>;
   launch_pdl(kern, dim3(nb, 1, g.nc), 256, poisson_fft_smem(g.ny, W), s, g, b.twiddle, b.spec, psi_new);
 }
